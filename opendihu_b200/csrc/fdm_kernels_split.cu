@@ -101,8 +101,8 @@ cudaError_t launch_schedule(const StimArgs& a, const SplitStep* steps, int n_ste
 {
   if (a.n_fibers == 0)
     return cudaSuccess;
-  const int T = 128;
-  stimulation_schedule_kernel<<<(a.n_fibers + T - 1) / T, T, 0, s>>>(a, steps, n_steps);
+  const int fibers = SCHEDULE_T / 32;   // a warp per fiber
+  stimulation_schedule_kernel<<<(a.n_fibers + fibers - 1) / fibers, SCHEDULE_T, 0, s>>>(a, steps, n_steps);
   return cudaGetLastError();
 }
 
