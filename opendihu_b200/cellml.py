@@ -882,6 +882,186 @@ class _FastEmitter(_Emitter):
         return out
 
 
+def _exp_shares(lines, consts):
+    """Exponentials of the FP64 form that follow from others: {repr(exp node): (base, square, constant)} with
+    exp node = base * constant, or base^2 * constant, and the list of the bases (exp nodes, evaluated as written).
+    Members of one slope (exp(a.x + b_k)) take the first member as their base, so that the argument's rounding
+    error is that of a member's own argument; a slope that doubles another one takes that one's base squared."""
+    found = {}
+
+    def walk(e):
+        t = e[0]
+        if t == "call":
+            if e[1] == "exp":
+                af = _affine(e[2][0], consts)
+                if af is not None and af[0]:
+                    key = tuple(sorted((k, round(v, 15)) for k, v in af[0].items()))
+                    found.setdefault(key, {}).setdefault(repr(e), (e, af[1]))
+            for a in e[2]:
+                walk(a)
+        elif t in ("neg", "pos", "not"):
+            walk(e[1])
+        elif t == "bin":
+            walk(e[2])
+            walk(e[3])
+        elif t == "tern":
+            for x in e[1:4]:
+                walk(x)
+    for _, _, e in lines:
+        walk(e)
+    shares, bases, base_of = {}, [], {}
+
+    def half_of(key):
+        for other in found:
+            if other != key and len(other) == len(key) and all(
+                    k == k2 and abs(v - 2 * v2) <= 4e-15 * abs(v) for (k, v), (k2, v2) in zip(key, other)):
+                return other
+        return None
+
+    def base(key):
+        """(index of the base, its constant term) of a slope whose first member is evaluated"""
+        if key not in base_of:
+            e, b = next(iter(found[key].values()))
+            bases.append(e)
+            base_of[key] = (len(bases) - 1, b)
+            shares[repr(e)] = (len(bases) - 1, False, 1.0)
+        return base_of[key]
+
+    for key, members in found.items():
+        half = half_of(key)
+        # one squaring only: the error of the base doubles with it
+        if half is not None and half_of(half) is None:
+            k, b0 = base(half)
+            for r, (_, b) in members.items():
+                shares[r] = (k, True, math.exp(b - 2 * b0))
+        elif len(members) > 1:
+            k, b0 = base(key)
+            for r, (_, b) in members.items():
+                if r not in shares:
+                    shares[r] = (k, False, math.exp(b - b0))
+    return shares, bases
+
+
+class _Fast64Emitter(_Emitter):
+    """FP64 form of the right-hand side.  In FP64 an exponential takes about 20 instructions and a division about
+    10, also one by a constant, so: products and quotients collect their constants into one factor (a division by
+    a constant becomes a multiplication) and exponentials follow from each other (_exp_shares; None: every
+    exponential evaluated, for approximations of it that do not turn sums into products).  Sums, gate terms and
+    divisions by variables stay as the model writes them."""
+
+    def __init__(self, real, consts, shares=None):
+        super().__init__(real, consts, "cuda")
+        self.shares = shares or {}
+
+    def factors(self, e, inverse=False):
+        """(constant, numerators, denominators) of a product / quotient / negation"""
+        af = _affine(e, self.consts)
+        if af is not None and not af[0] and af[1] != 0.0:
+            return (1.0 / af[1] if inverse else af[1]), [], []
+        if e[0] in ("neg", "pos"):
+            c, n, d = self.factors(e[1], inverse)
+            return (-c if e[0] == "neg" else c), n, d
+        if e[0] == "bin" and e[1] in "*/":
+            c1, n1, d1 = self.factors(e[2], inverse)
+            c2, n2, d2 = self.factors(e[3], inverse != (e[1] == "/"))
+            return c1 * c2, n1 + n2, d1 + d2
+        return (1.0, [], [e]) if inverse else (1.0, [e], [])
+
+    def expr(self, e):
+        t = e[0]
+        af = _affine(e, self.consts)
+        if af is not None and not af[0]:
+            return self.lit(af[1])
+        if t in ("neg", "pos") or (t == "bin" and e[1] in "*/"):
+            c, num, den = self.factors(e)
+            if not num:
+                text, c = self.lit(c), 1.0
+            else:
+                text = self.expr(num[0])
+                if c not in (1.0, -1.0):
+                    text = f"({self.lit(c)} * {text})"
+                for x in num[1:]:
+                    text = f"({text} * {self.expr(x)})"
+            for x in den:
+                text = f"({text} / {self.expr(x)})"
+            return f"(-{text})" if c == -1.0 else text
+        if t == "bin" and e[1] == "-":
+            # 1 - exp(u), exp(u) - 1 with a derived exponential: exactly 0 where u is, as with the exponential itself
+            om = _one_minus_exp(e, self.consts)
+            if om is not None and repr(om[1]) in self.shares and self.shares[repr(om[1])][1:] != (False, 1.0):
+                d = f"({self.expr(om[1])} - (({self.real})1.0))" if om[0] < 0 else \
+                    f"((({self.real})1.0) - {self.expr(om[1])})"
+                return f"({self.expr(om[1][2][0])} == (({self.real})0.0) ? (({self.real})0.0) : {d})"
+        if t == "call" and e[1] == "exp" and repr(e) in self.shares:
+            k, square, c = self.shares[repr(e)]
+            x = f"fdm_q{k}" if square else f"fdm_x{k}"
+            return x if c == 1.0 else f"({x} * {self.lit(c)})"
+        return super().expr(e)
+
+    def base_lines(self, bases, used, indent="    "):
+        """Declarations of the bases and squares that the shares in `used` (exp nodes' reprs) need"""
+        out = []
+        need = {self.shares[r][0] for r in used}
+        squares = {self.shares[r][0] for r in used if self.shares[r][1]}
+        for k, e in enumerate(bases):
+            if k in need:
+                out.append(f"{indent}const R fdm_x{k} = FDM_EXP({self.expr(e[2][0])});")
+                if k in squares:
+                    out.append(f"{indent}const R fdm_q{k} = fdm_x{k} * fdm_x{k};")
+        return out
+
+
+def _shares_used(exprs, shares) -> set:
+    """The reprs of the shared exponentials that occur in the expressions"""
+    used = set()
+
+    def walk(e):
+        t = e[0]
+        if t == "call":
+            if repr(e) in shares:
+                used.add(repr(e))
+            for a in e[2]:
+                walk(a)
+        elif t in ("neg", "pos", "not"):
+            walk(e[1])
+        elif t == "bin":
+            walk(e[2])
+            walk(e[3])
+        elif t == "tern":
+            for x in e[1:4]:
+                walk(x)
+    for e in exprs:
+        walk(e)
+    return used
+
+
+_MATH_MACROS = ["#define FDM_EXP(x) M::exp(x)", "#define FDM_LOG(x) M::log(x)", "#define FDM_POWF(x, y) M::pow(x, y)",
+                "#define FDM_ABS(x) fabs(x)", "#define FDM_SQRT(x) sqrt(x)"]
+
+
+def emit_rates_f64(lines, consts, pows) -> List[str]:
+    """``rates_f64`` (shared exponentials) and ``rates_f64_plain`` (every exponential evaluated): the FP64 forms."""
+    out = []
+    for name, shared in (("rates_f64", True), ("rates_f64_plain", False)):
+        shares, bases = _exp_shares(lines, consts) if shared else ({}, [])
+        em = _Fast64Emitter("R", consts, shares)
+        out.append("  template<class R, class M>")
+        out.append(f"  __device__ __forceinline__ static void {name}(const R VOI, const R* __restrict__ STATES,"
+                   " const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)")
+        out.append("  {")
+        out.append("    (void)VOI; (void)PARAMS;")
+        out.extend(_MATH_MACROS)
+        out.extend("#define " + x.split("#define ", 1)[1] for x in _pow_macro_defs(pows))
+        out.extend(em.base_lines(bases, _shares_used([e for _, _, e in lines], shares)))
+        for kind, idx, expr in lines:
+            tgt = f"ALGEBRAIC[{idx}]" if kind == "A" else f"RATES[{idx}]"
+            out.append(f"    {tgt} = {em.expr(expr)};")
+        out.extend(f"#undef FDM_POW{n}" for n in pows)
+        out.append("#undef FDM_EXP\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
+        out.append("  }")
+    return out
+
+
 def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Sequence[int]) -> str:
     """CUDA device right-hand side for one parameter variant.
 
@@ -931,6 +1111,9 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
         out.append(f"#undef FDM_POW{n}")
     out.append("#undef FDM_EXP\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
     out.append("  }")
+    out.append("  // FP64 forms: constants collected into one factor per product, divisions by constants as")
+    out.append("  // multiplications; rates_f64 with exponentials that follow from others (exact exponentials only)")
+    out.extend(emit_rates_f64(lines, model.constants, pows))
     # FP32 variant with shared exponentials
     repl, groups = _exp_groups(lines, model.constants)
     rgroups = _batched_denominators(lines, model.constants, repl=repl)
@@ -984,7 +1167,7 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
     out.append("#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
     out.append("  }")
     # the right-hand side split by state (few-node reaction kernel)
-    out.append("  // the right-hand side of one state at a time: rates_group<R, M, G> = RATES[G]")
+    out.append("  // the right-hand side of one state at a time: rates_group<R, M, G, SHARED> = RATES[G]")
     out.extend(emit_group_rates(model, params_alg, params_const))
     # reverse mode (adjoint)
     out.append("  // vector-Jacobian product: LAM_STATES += J^T LAM_RATES, LAM_PARAMS += (dRATES/dPARAMS)^T LAM_RATES")
@@ -1035,40 +1218,42 @@ MAX_GROUP_STATES = 8
 
 
 def emit_group_rates(model: Model, params_alg: Sequence[int], params_const: Sequence[int]) -> List[str]:
-    """The right-hand side split by state: ``rates_group<R, M, G>`` computes RATES[G] only, from the lines its
-    cone needs, so that the warps of a node group can each evaluate one state's rate (the reaction kernel for
+    """The right-hand side split by state: ``rates_group<R, M, G, SHARED>`` computes RATES[G] only, from the lines
+    its cone needs, so that the warps of a node group can each evaluate one state's rate (the reaction kernel for
     few nodes, where one thread per node leaves the SMs short of independent work).  Same expressions as
-    ``rates``, so the same values."""
+    ``rates_f64`` (SHARED) / ``rates_f64_plain``, so the same values."""
     lines = substitute_parameters(model, params_alg, params_const)
-    em = _Emitter("R", model.constants, "cuda")
     pows = _collect_int_pows(lines)
     out = [f"  static constexpr int nGroups = {model.n_states if model.n_states <= MAX_GROUP_STATES else 0};"]
     if model.n_states > MAX_GROUP_STATES:
         return out
-    out.append("  template<class R, class M, int G>")
+    out.append("  template<class R, class M, int G, bool SHARED>")
     out.append("  __device__ __forceinline__ static R rates_group(const R VOI, const R* __restrict__ STATES,"
                " const R* __restrict__ PARAMS)")
     out.append("  {")
     out.append("    (void)VOI; (void)PARAMS;")
     out.append(f"    R ALGEBRAIC[{max(model.n_algebraics, 1)}];")
     out.append("    (void)ALGEBRAIC;")
-    out.append("#define FDM_EXP(x) M::exp(x)")
-    out.append("#define FDM_LOG(x) M::log(x)")
-    out.append("#define FDM_POWF(x, y) M::pow(x, y)")
-    out.append("#define FDM_ABS(x) fabs(x)")
-    out.append("#define FDM_SQRT(x) sqrt(x)")
+    out.extend(_MATH_MACROS)
     out.extend("#define " + s2.split("#define ", 1)[1] for s2 in _pow_macro_defs(pows))
-    for g in range(model.n_states):
-        out.append(f"    {'if' if g == 0 else 'else if'} constexpr (G == {g}) {{")
-        rate = None
-        for n in rate_cone(lines, [g]):
-            kind, idx, expr = lines[n]
-            if kind == "A":
-                out.append(f"      ALGEBRAIC[{idx}] = {em.expr(expr)};")
-            else:
-                rate = em.expr(expr)
-        out.append(f"      return {rate if rate is not None else '(R)0'};")
-        out.append("    }")
+    first = True
+    for shared in (True, False):
+        shares, bases = _exp_shares(lines, model.constants) if shared else ({}, [])
+        em = _Fast64Emitter("R", model.constants, shares)
+        for g in range(model.n_states):
+            out.append(f"    {'if' if first else 'else if'} constexpr (G == {g} && {'SHARED' if shared else '!SHARED'}) {{")
+            first = False
+            rate = None
+            cone = rate_cone(lines, [g])
+            out.extend(em.base_lines(bases, _shares_used([lines[n][2] for n in cone], shares), "      "))
+            for n in cone:
+                kind, idx, expr = lines[n]
+                if kind == "A":
+                    out.append(f"      ALGEBRAIC[{idx}] = {em.expr(expr)};")
+                else:
+                    rate = em.expr(expr)
+            out.append(f"      return {rate if rate is not None else '(R)0'};")
+            out.append("    }")
     out.append("    else {")
     out.append("      return (R)0;")
     out.append("    }")

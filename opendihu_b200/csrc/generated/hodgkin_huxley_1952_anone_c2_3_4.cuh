@@ -48,6 +48,78 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_ABS
 #undef FDM_SQRT
   }
+  // FP64 forms: constants collected into one factor per product, divisions by constants as
+  // multiplications; rates_f64 with exponentials that follow from others (exact exponentials only)
+  template<class R, class M>
+  __device__ __forceinline__ static void rates_f64(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)
+  {
+    (void)VOI; (void)PARAMS;
+#define FDM_EXP(x) M::exp(x)
+#define FDM_LOG(x) M::log(x)
+#define FDM_POWF(x, y) M::pow(x, y)
+#define FDM_ABS(x) fabs(x)
+#define FDM_SQRT(x) sqrt(x)
+#define FDM_POW2(x) fdm_pow2(x)
+#define FDM_POW3(x) fdm_pow3(x)
+#define FDM_POW4(x) fdm_pow4(x)
+    const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
+    const R fdm_q0 = fdm_x0 * fdm_x0;
+    ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
+    ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+    RATES[1] = ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
+    ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * fdm_x0);
+    ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
+    RATES[2] = ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
+    ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
+    ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+    RATES[3] = ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
+    ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
+    ALGEBRAIC[4] = ((PARAMS[2] * FDM_POW4(STATES[3])) * (STATES[0] - ((R)-0x1.5c00000000000p+6)));
+    ALGEBRAIC[8] = (((R)0x1.3333333333333p-2) * (STATES[0] - ((R)-0x1.018c49ba5e354p+6)));
+    RATES[0] = (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
+#undef FDM_POW2
+#undef FDM_POW3
+#undef FDM_POW4
+#undef FDM_EXP
+#undef FDM_LOG
+#undef FDM_POWF
+#undef FDM_ABS
+#undef FDM_SQRT
+  }
+  template<class R, class M>
+  __device__ __forceinline__ static void rates_f64_plain(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)
+  {
+    (void)VOI; (void)PARAMS;
+#define FDM_EXP(x) M::exp(x)
+#define FDM_LOG(x) M::log(x)
+#define FDM_POWF(x, y) M::pow(x, y)
+#define FDM_ABS(x) fabs(x)
+#define FDM_SQRT(x) sqrt(x)
+#define FDM_POW2(x) fdm_pow2(x)
+#define FDM_POW3(x) fdm_pow3(x)
+#define FDM_POW4(x) fdm_pow4(x)
+    ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+    RATES[1] = ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
+    ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+    ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
+    RATES[2] = ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
+    ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+    RATES[3] = ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
+    ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
+    ALGEBRAIC[4] = ((PARAMS[2] * FDM_POW4(STATES[3])) * (STATES[0] - ((R)-0x1.5c00000000000p+6)));
+    ALGEBRAIC[8] = (((R)0x1.3333333333333p-2) * (STATES[0] - ((R)-0x1.018c49ba5e354p+6)));
+    RATES[0] = (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
+#undef FDM_POW2
+#undef FDM_POW3
+#undef FDM_POW4
+#undef FDM_EXP
+#undef FDM_LOG
+#undef FDM_POWF
+#undef FDM_ABS
+#undef FDM_SQRT
+  }
   // FP32 form: exponentials exp(a.x + b_k) that share a.x are evaluated once as exp(a.x) * e^{b_k};
   // exponentials, logarithms and reciprocals as single SFU instructions (fdm_ex2/fdm_lg2/fdm_rcp)
   static constexpr int nSharedExponentials = 1;
@@ -129,9 +201,9 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_ABS
 #undef FDM_SQRT
   }
-  // the right-hand side of one state at a time: rates_group<R, M, G> = RATES[G]
+  // the right-hand side of one state at a time: rates_group<R, M, G, SHARED> = RATES[G]
   static constexpr int nGroups = 4;
-  template<class R, class M, int G>
+  template<class R, class M, int G, bool SHARED>
   __device__ __forceinline__ static R rates_group(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS)
   {
     (void)VOI; (void)PARAMS;
@@ -145,26 +217,53 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_POW2(x) fdm_pow2(x)
 #define FDM_POW3(x) fdm_pow3(x)
 #define FDM_POW4(x) fdm_pow4(x)
-    if constexpr (G == 0) {
+    if constexpr (G == 0 && SHARED) {
       ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
       ALGEBRAIC[4] = ((PARAMS[2] * FDM_POW4(STATES[3])) * (STATES[0] - ((R)-0x1.5c00000000000p+6)));
       ALGEBRAIC[8] = (((R)0x1.3333333333333p-2) * (STATES[0] - ((R)-0x1.018c49ba5e354p+6)));
-      return ((-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8])) / ((R)0x1.0000000000000p+0));
+      return (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
     }
-    else if constexpr (G == 1) {
-      ALGEBRAIC[1] = (((-((R)0.100000)) * (STATES[0] + ((R)50.0000))) / (FDM_EXP(((-(STATES[0] + ((R)50.0000))) / ((R)10.0000))) - ((R)1.00000)));
-      ALGEBRAIC[5] = (((R)4.00000) * FDM_EXP(((-(STATES[0] + ((R)75.0000))) / ((R)18.0000))));
-      return ((ALGEBRAIC[1] * (((R)1.00000) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
+    else if constexpr (G == 1 && SHARED) {
+      const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
+      const R fdm_q0 = fdm_x0 * fdm_x0;
+      ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
+      ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+      return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     }
-    else if constexpr (G == 2) {
-      ALGEBRAIC[2] = (((R)0.0700000) * FDM_EXP(((-(STATES[0] + ((R)75.0000))) / ((R)20.0000))));
-      ALGEBRAIC[6] = (((R)1.00000) / (FDM_EXP(((-(STATES[0] + ((R)45.0000))) / ((R)10.0000))) + ((R)1.00000)));
-      return ((ALGEBRAIC[2] * (((R)1.00000) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
+    else if constexpr (G == 2 && SHARED) {
+      const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
+      const R fdm_q0 = fdm_x0 * fdm_x0;
+      ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * fdm_x0);
+      ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
+      return ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
     }
-    else if constexpr (G == 3) {
-      ALGEBRAIC[3] = (((-((R)0.0100000)) * (STATES[0] + ((R)65.0000))) / (FDM_EXP(((-(STATES[0] + ((R)65.0000))) / ((R)10.0000))) - ((R)1.00000)));
-      ALGEBRAIC[7] = (((R)0.125000) * FDM_EXP(((STATES[0] + ((R)75.0000)) / ((R)80.0000))));
-      return ((ALGEBRAIC[3] * (((R)1.00000) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
+    else if constexpr (G == 3 && SHARED) {
+      const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
+      const R fdm_q0 = fdm_x0 * fdm_x0;
+      ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
+      ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+      return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
+    }
+    else if constexpr (G == 0 && !SHARED) {
+      ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
+      ALGEBRAIC[4] = ((PARAMS[2] * FDM_POW4(STATES[3])) * (STATES[0] - ((R)-0x1.5c00000000000p+6)));
+      ALGEBRAIC[8] = (((R)0x1.3333333333333p-2) * (STATES[0] - ((R)-0x1.018c49ba5e354p+6)));
+      return (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
+    }
+    else if constexpr (G == 1 && !SHARED) {
+      ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+      return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
+    }
+    else if constexpr (G == 2 && !SHARED) {
+      ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+      ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
+      return ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
+    }
+    else if constexpr (G == 3 && !SHARED) {
+      ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
+      return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     }
     else {
       return (R)0;
