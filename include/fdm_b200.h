@@ -254,7 +254,7 @@ int fdm_checkpoint_restore(fdm_solver *s);
  * standalone operator on DEVICE arrays of the current CUDA device: d_fiber_offsets[n_fibers+1] (node offsets),
  * d_element_lengths (each fiber's n_f-1 lengths, concatenated), d_prefactor[n_fibers], d_vm[n_nodes] (in: u,
  * out: u+).  diffusion_scheme is FDM_IMPLICIT_EULER or FDM_CRANK_NICOLSON, dt the diffusion step width.
- * Scratch memory (7 doubles per node) is allocated by the library with cudaMalloc and kept for later calls.
+ * Scratch memory (2 doubles per node) is allocated by the library with cudaMalloc and kept for later calls.
  * stream is a cudaStream_t (NULL: the legacy default stream); the call returns after the solve. */
 int fdm_diffusion_solve(int n_fibers, int64_t n_nodes, const int64_t *d_fiber_offsets, const double *d_element_lengths,
                         const double *d_prefactor, double dt, int diffusion_scheme, double *d_vm, void *stream);
@@ -263,7 +263,7 @@ int fdm_diffusion_solve(int n_fibers, int64_t n_nodes, const int64_t *d_fiber_of
  * cannot allocate device memory while they run (an application whose memory pool owns the whole GPU, a
  * coupled code that has reserved HBM for its own mesh, a stepping loop that must not synchronize on
  * cudaMalloc/cudaFree).  The scratch is one array compiled into the library, sized for at most
- * FDM_NOALLOC_MAX_NODES nodes (14.7 MB held on every GPU that loads the library until the process exits);
+ * FDM_NOALLOC_MAX_NODES nodes (4.2 MB held on every GPU that loads the library until the process exits);
  * larger n_nodes fail with FDM_ERR_ARG.  The fiber offsets index that array: they must not decrease and must
  * lie in [0, n_nodes] (d_fiber_offsets[n_fibers] <= n_nodes); the call reads their first and last entry back
  * and fails with FDM_ERR_ARG when either end is outside.  The first call on a device looks the array's

@@ -1977,7 +1977,8 @@ static int ensure_coefficients(fdm_solver* s, double dt1)
   if (s->coef_valid && std::fabs(dt1 - s->coef_dt) <= 1e-12 * std::fabs(s->coef_dt))
     return FDM_OK;
   FDM_CUDA(launch_coefficients(s->n_fibers, s->off_d.p, s->elem_d.p, s->prefactor_d.p, dt1,
-                               s->cfg.diffusion_scheme == FDM_IMPLICIT_EULER, s->coef.p, s->n_nodes, s->stream));
+                               s->cfg.diffusion_scheme == FDM_IMPLICIT_EULER, s->coef.p, s->n_nodes, s->max_fiber_len,
+                               s->stream));
   s->launches++;
   s->coef_dt = dt1;
   s->coef_valid = true;
@@ -2237,7 +2238,7 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
         cur ^= 1;
         if (half == 0) {
           FDM_CUDA(launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                         s->stream, E.counter.p, E.nbuf.p, s->cfg.n_ranks));
+                                         s->max_fiber_len, s->stream, E.counter.p, E.nbuf.p, s->cfg.n_ranks));
           s->launches++;
         }
       }
@@ -2261,7 +2262,7 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
           ce = launch_reaction(s->cfg.model, rk, mk, ra, s->stream);
           if (ce == cudaSuccess && half == 0)
             ce = launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                       s->stream);
+                                       s->max_fiber_len, s->stream);
         }
       }
       cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
@@ -2295,7 +2296,7 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
         FDM_CUDA(cudaEventRecord(e1, s->stream));
       if (half == 0) {
         FDM_CUDA(launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                       s->stream));
+                                       s->max_fiber_len, s->stream));
         s->launches++;
       }
     }
@@ -2834,8 +2835,8 @@ extern "C" int fdm_diffusion_solve(int n_fibers, int64_t n_nodes, const int64_t*
     return fail(s, FDM_ERR_ARG, "fdm_diffusion_solve: device ordinal beyond 63");
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_scratch.mu);
-  // scratch: 6 factorization doubles + 1 forward-sweep double per node, allocated by the library
-  const size_t need = (size_t)7 * (size_t)n_nodes;
+  // scratch: two doubles per node (the sweeps of fibers longer than a tile), allocated by the library
+  const size_t need = (size_t)2 * (size_t)n_nodes;
   if (g_scratch.n[dev] < need) {
     if (g_scratch.p[dev])
       FDM_CUDA(cudaFree(g_scratch.p[dev]));
@@ -2844,11 +2845,8 @@ extern "C" int fdm_diffusion_solve(int n_fibers, int64_t n_nodes, const int64_t*
     FDM_CUDA(cudaMalloc((void**)&g_scratch.p[dev], need * sizeof(double)));
     g_scratch.n[dev] = need;
   }
-  double* coef = g_scratch.p[dev];
-  double* fwd = coef + 6 * (size_t)n_nodes;
-  FDM_CUDA(launch_coefficients(n_fibers, d_fiber_offsets, d_element_lengths, d_prefactor, dt,
-                               diffusion_scheme == FDM_IMPLICIT_EULER, coef, n_nodes, st));
-  FDM_CUDA(launch_diffusion(n_fibers, d_fiber_offsets, coef, n_nodes, d_vm, fwd, st));
+  FDM_CUDA(launch_diffusion_operator(n_fibers, n_nodes, d_fiber_offsets, d_element_lengths, d_prefactor, dt,
+                                     diffusion_scheme == FDM_IMPLICIT_EULER, d_vm, g_scratch.p[dev], st));
   FDM_CUDA(cudaStreamSynchronize(st));
   return FDM_OK;
 }
@@ -3386,7 +3384,7 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
     FDM_CUDA(A.coefs.alloc(edt.size() * 6 * (size_t)N));
     for (size_t e = 0; e < edt.size(); e++) {
       FDM_CUDA(launch_coefficients(nf, s->off_d.p, s->elem_d.p, s->prefactor_d.p, edt[e], ie, A.coefs.p + e * 6 * N, N,
-                                   s->stream));
+                                   s->max_fiber_len, s->stream));
       s->launches++;
     }
   }
@@ -3448,7 +3446,8 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
         FDM_CUDA(launch_reaction(s->cfg.model, REAL_F64, mk, ra, s->stream));
         s->launches++;
         if (half == 0) {
-          FDM_CUDA(launch_diffusion(nf, s->off_d.p, coef_of(b + jj), N, s->vm.p, s->scratch.p, s->stream));
+          FDM_CUDA(launch_diffusion(nf, s->off_d.p, coef_of(b + jj), N, s->vm.p, s->scratch.p,
+                                    s->max_fiber_len, s->stream));
           s->launches++;
         }
       }

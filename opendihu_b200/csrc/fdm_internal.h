@@ -64,12 +64,16 @@ cudaError_t launch_schedule(const StimArgs& a, const SplitStep* steps, int n_ste
 cudaError_t launch_states_to_pairs(const double* x, float* hi, float* lo, int64_t n, cudaStream_t s);
 cudaError_t launch_pairs_to_states(const float* hi, const float* lo, double* x, int64_t n, cudaStream_t s);
 cudaError_t launch_coefficients(int n_fibers, const int64_t* fiber_offsets, const double* element_lengths, const double* prefactor, double dt, int implicit_euler,
-                                double* coef, int64_t stride, cudaStream_t s);
-// one diffusion solve of every fiber in place on vm (scratch: one double per node): a warp per fiber, or a
-// CTA per fiber when the fibers are few
+                                double* coef, int64_t stride, int64_t max_fiber_len, cudaStream_t s);
+// factorization and solve in one pass, in place on vm (scratch: two doubles per node)
+cudaError_t launch_diffusion_operator(int n_fibers, int64_t n_nodes, const int64_t* fiber_offsets,
+                                      const double* element_lengths, const double* prefactor, double dt,
+                                      int implicit_euler, double* vm, double* scratch, cudaStream_t s);
+// one diffusion solve of every fiber in place on vm (scratch: one double per node): a CTA per fiber, or a warp per
+// fiber for many short fibers
 cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const double* coef, int64_t stride,
-                             double* vm, double* scratch, cudaStream_t s, const int* eq_counter = nullptr,
-                             const int* eq_nbuf = nullptr, int n_ranks = 1);
+                             double* vm, double* scratch, int64_t max_fiber_len, cudaStream_t s,
+                             const int* eq_counter = nullptr, const int* eq_nbuf = nullptr, int n_ranks = 1);
 // one half step with the equilibrium skip (fdm_equilibrium.cuh): speculative reaction, equilibrium tests,
 // scan of the buffers, commit (and the trace after half 1)
 cudaError_t launch_equilibrium_half(int model, RealKind rk, MathKind mk, const ReactionArgs& a, const EqLayout& L,

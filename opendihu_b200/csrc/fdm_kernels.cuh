@@ -755,90 +755,6 @@ __global__ void __launch_bounds__(32 * (Model::nGroups > 0 ? Model::nGroups : 1)
   }
 }
 
-// --------------------------------------------------------------------------------------------
-// diffusion: coefficients of the per-fiber tridiagonal system, computed once per (dt1D, prefactor)
-//   IE: (K - M/dt) u+ = -M/dt u            CN: (K/2 - M/dt) u+ = (-K/2 - M/dt) u
-// following the element loops of compute.tpp:336-449, and its LU factors for
-//   d'_i = mulF_i d'_{i-1} + inv_i d_i,     x_i = d'_i - cp_i x_{i+1}
-// Per node the six doubles are stored as coef[k*stride + node], k = 0..5 = mulF, inv, cp, l, m, r
-// with d_i = l_i u_{i-1} + m_i u_i + r_i u_{i+1}.
-// --------------------------------------------------------------------------------------------
-#ifdef FDM_COMMON_KERNELS_TU
-__global__ void diffusion_coefficients_kernel(int n_fibers, const int64_t* __restrict__ fiber_offsets,
-                                              const double* __restrict__ element_lengths,
-                                              const double* __restrict__ prefactor, double dt, int implicit_euler,
-                                              double* __restrict__ coef, int64_t stride)
-{
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= n_fibers)
-    return;
-  const int64_t o = fiber_offsets[f];
-  const int64_t n = fiber_offsets[f + 1] - o;
-  const double* h = element_lengths + (o - f); // fiber f's elements follow the previous fibers' n-1 each
-  const double pf = prefactor[f];
-  double cp_prev = 0.0;
-  for (int64_t v = 0; v < n; v++) {
-    double a = 0, b = 0, c = 0, l = 0, m = 0, r = 0;
-    if (v > 0) {
-      const double h_left = h[v - 1];
-      const double k_left = 1. / h_left * (1) * pf;
-      const double m_left = h_left * 1. / 6;
-      const double k_right = 1. / h_left * (-1) * pf;
-      const double m_right = h_left * 1. / 3;
-      if (implicit_euler) {
-        a = (k_left - 1 / dt * m_left);
-        b += (k_right - 1 / dt * m_right);
-        l = (-1 / dt * m_left);
-        m += (-1 / dt * m_right);
-      } else {
-        a = (k_left / 2. - 1 / dt * m_left);
-        b += (k_right / 2. - 1 / dt * m_right);
-        l = (-k_left / 2. - 1 / dt * m_left);
-        m += (-k_right / 2. - 1 / dt * m_right);
-      }
-    }
-    if (v < n - 1) {
-      const double h_right = h[v];
-      const double k_right = 1. / h_right * (1) * pf;
-      const double m_right = h_right * 1. / 6;
-      const double k_left = 1. / h_right * (-1) * pf;
-      const double m_left = h_right * 1. / 3;
-      if (implicit_euler) {
-        c = (k_right - 1 / dt * m_right);
-        b += (k_left - 1 / dt * m_left);
-        m += (-1 / dt * m_left);
-        r = (-1 / dt * m_right);
-      } else {
-        c = (k_right / 2. - 1 / dt * m_right);
-        b += (k_left / 2. - 1 / dt * m_left);
-        m += (-k_left / 2. - 1 / dt * m_left);
-        r = (-k_right / 2. - 1 / dt * m_right);
-      }
-    }
-    double inv, mulF, cp;
-    if (v == 0) {
-      inv = 1.0 / b;
-      mulF = 0.0;
-      cp = c / b;
-    } else {
-      const double den = b - cp_prev * a;
-      inv = 1.0 / den;
-      mulF = -a * inv;
-      cp = (v != n - 1) ? c / den : 0.0;
-    }
-    cp_prev = cp;
-    const int64_t i = o + v;
-    coef[0 * stride + i] = mulF;
-    coef[1 * stride + i] = inv;
-    coef[2 * stride + i] = cp;
-    coef[3 * stride + i] = l;
-    coef[4 * stride + i] = m;
-    coef[5 * stride + i] = r;
-  }
-}
-
-#endif // FDM_COMMON_KERNELS_TU
-
 // affine map x -> F x + G; compose(first, second) = second o first
 struct Affine {
   double F, G;

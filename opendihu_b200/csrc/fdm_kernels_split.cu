@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "fdm_internal.h"
+#include "fdm_diffusion.cuh"
 #include "fdm_equilibrium.cuh"
 #include "fdm_model_launch.cuh"
 
@@ -106,16 +107,39 @@ cudaError_t launch_schedule(const StimArgs& a, const SplitStep* steps, int n_ste
   return cudaGetLastError();
 }
 
-cudaError_t launch_coefficients(int n_fibers, const int64_t* fiber_offsets, const double* element_lengths,
-                                const double* prefactor, double dt, int implicit_euler, double* coef, int64_t stride,
-                                cudaStream_t s)
+template<int WHAT>
+static cudaError_t factor_launch(int n_fibers, int tile, const int64_t* fiber_offsets, const double* element_lengths,
+                                 const double* prefactor, double dt, int implicit_euler, double* coef, int64_t stride,
+                                 double* vm, double* scratch, cudaStream_t s)
 {
   if (n_fibers == 0)
     return cudaSuccess;
-  const int T = 64;
-  diffusion_coefficients_kernel<<<(n_fibers + T - 1) / T, T, 0, s>>>(n_fibers, fiber_offsets, element_lengths,
-                                                                     prefactor, dt, implicit_euler, coef, stride);
+  const size_t smem = factor_smem_bytes(tile);
+  const cudaError_t e = cudaFuncSetAttribute(diffusion_factor_kernel<WHAT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+  if (e != cudaSuccess)
+    return e;
+  diffusion_factor_kernel<WHAT><<<(unsigned)n_fibers, FACTOR_T, smem, s>>>(
+      fiber_offsets, element_lengths, prefactor, dt, implicit_euler, coef, stride, vm, scratch, tile);
   return cudaGetLastError();
+}
+
+cudaError_t launch_coefficients(int n_fibers, const int64_t* fiber_offsets, const double* element_lengths,
+                                const double* prefactor, double dt, int implicit_euler, double* coef, int64_t stride,
+                                int64_t max_fiber_len, cudaStream_t s)
+{
+  // shared memory for the longest fiber only: more CTAs per SM
+  const int tile = (int)std::min<int64_t>(FACTOR_TILE, std::max<int64_t>(max_fiber_len, 1));
+  return factor_launch<FACTOR>(n_fibers, tile, fiber_offsets, element_lengths, prefactor, dt, implicit_euler, coef,
+                               stride, nullptr, nullptr, s);
+}
+
+cudaError_t launch_diffusion_operator(int n_fibers, int64_t n_nodes, const int64_t* fiber_offsets,
+                                      const double* element_lengths, const double* prefactor, double dt,
+                                      int implicit_euler, double* vm, double* scratch, cudaStream_t s)
+{
+  return factor_launch<FACTOR_SOLVE>(n_fibers, FACTOR_TILE, fiber_offsets, element_lengths, prefactor, dt,
+                                     implicit_euler, nullptr, n_nodes, vm, scratch, s);
 }
 
 __global__ void __launch_bounds__(256) states_to_pairs_kernel(const double* __restrict__ x, float* __restrict__ hi,
@@ -162,23 +186,46 @@ cudaError_t launch_pairs_to_states(const float* hi, const float* lo, double* x, 
 // needed before a warp per fiber fills the GPU)
 constexpr int DIFFUSION_BLOCK_MAX_FIBERS = 4 * 148;
 
+template<int M>
+static cudaError_t diffusion_reg_launch(int n_fibers, const int64_t* fiber_offsets, const double* coef, int64_t stride,
+                                        double* vm, cudaStream_t s, const int* eq_counter, const int* eq_nbuf,
+                                        int n_ranks)
+{
+  diffusion_reg_kernel<M><<<(unsigned)n_fibers, DIFFUSION_T, 0, s>>>(fiber_offsets, coef, stride, vm, eq_counter,
+                                                                     eq_nbuf, n_ranks);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const double* coef, int64_t stride,
-                                  double* vm, double* scratch, cudaStream_t s, const int* eq_counter,
-                                  const int* eq_nbuf, int n_ranks)
+                                  double* vm, double* scratch, int64_t max_fiber_len, cudaStream_t s,
+                                  const int* eq_counter, const int* eq_nbuf, int n_ranks)
 {
   if (n_fibers == 0)
     return cudaSuccess;
-  if (n_fibers < DIFFUSION_BLOCK_MAX_FIBERS) {
-    // few fibers: a CTA per fiber fills more of the GPU than a warp per fiber
+  const int nr = n_ranks > 0 ? n_ranks : 1;
+  // many short fibers: a warp per fiber, as half of a CTA's threads would have no node (4096 fibers: of 100 nodes 12.5 us
+  // against 18.5 us with a CTA each, of 200 nodes 20.6 against 18.5; 592 fibers of 100 nodes: 6.2 us both)
+  const bool many = n_fibers >= DIFFUSION_BLOCK_MAX_FIBERS;
+  if (!(many && max_fiber_len <= DIFFUSION_T / 2)) {
+    switch ((max_fiber_len + 2 * DIFFUSION_T - 1) / (2 * DIFFUSION_T)) {
+    case 1: return diffusion_reg_launch<2>(n_fibers, fiber_offsets, coef, stride, vm, s, eq_counter, eq_nbuf, nr);
+    case 2: return diffusion_reg_launch<4>(n_fibers, fiber_offsets, coef, stride, vm, s, eq_counter, eq_nbuf, nr);
+    case 3: return diffusion_reg_launch<6>(n_fibers, fiber_offsets, coef, stride, vm, s, eq_counter, eq_nbuf, nr);
+    case 4: return diffusion_reg_launch<8>(n_fibers, fiber_offsets, coef, stride, vm, s, eq_counter, eq_nbuf, nr);
+    case 5: return diffusion_reg_launch<10>(n_fibers, fiber_offsets, coef, stride, vm, s, eq_counter, eq_nbuf, nr);
+    default: break;
+    }
+  }
+  if (!many) {
+    // fibers too long for registers
     diffusion_block_kernel<256><<<(unsigned)n_fibers, 256, 0, s>>>(fiber_offsets, coef, stride, vm, scratch,
-                                                                   eq_counter, eq_nbuf, n_ranks > 0 ? n_ranks : 1);
+                                                                   eq_counter, eq_nbuf, nr);
     return cudaGetLastError();
   }
   const int T = 128;
   const int64_t threads = (int64_t)n_fibers * 32;
   diffusion_warp_kernel<<<(unsigned)((threads + T - 1) / T), T, 0, s>>>(n_fibers, fiber_offsets, coef, stride, vm,
-                                                                        scratch, eq_counter, eq_nbuf,
-                                                                        n_ranks > 0 ? n_ranks : 1);
+                                                                        scratch, eq_counter, eq_nbuf, nr);
   return cudaGetLastError();
 }
 

@@ -5,12 +5,12 @@
 // that reserves nearly all of HBM for its 3D mesh), where an extra cudaMalloc fails or fragments the pool;
 // and time-critical stepping loops, where cudaMalloc/cudaFree may synchronize the device and stall other
 // work.  For them this entry point takes its scratch from one array compiled into the library instead of
-// calling cudaMalloc: FDM_NOALLOC_MAX_NODES nodes x 7 doubles (14.7 MB), which every GPU that loads this
+// calling cudaMalloc: FDM_NOALLOC_MAX_NODES nodes x 2 doubles (4.2 MB), which every GPU that loads this
 // library holds until the process exits.
 //
 // The array is shared by all calls and keeps the previous call's contents.  Nothing in it has to start at
-// zero: the factorization kernel writes every coefficient the solve reads, and the forward sweep writes
-// every intermediate value before the backward sweep reads it.  Calls whose work overlaps on the GPU
+// zero: the forward sweep (of fibers longer than a tile) writes every intermediate value before the backward sweep
+// reads it.  Calls whose work overlaps on the GPU
 // (from several host threads, or on several streams without ordering between them) use the same memory and
 // race; order them on one stream or serialize them.
 #include <cuda_runtime.h>
@@ -21,8 +21,8 @@
 #include "../../include/fdm_b200.h"
 #include "fdm_internal.h"
 
-// scratch of the allocation-free solve: 6 factorization doubles + 1 forward-sweep double per node
-static __device__ __align__(256) double fdm_noalloc_scratch[7 * (size_t)FDM_NOALLOC_MAX_NODES];
+// scratch of the allocation-free solve: d' and cp per node
+static __device__ __align__(256) double fdm_noalloc_scratch[2 * (size_t)FDM_NOALLOC_MAX_NODES];
 
 // Device code that names the array, so that it stays in this file's device image (never launched).
 __global__ void fdm_noalloc_keep_kernel(int write)
@@ -93,12 +93,8 @@ extern "C" int fdm_diffusion_solve_noalloc(int n_fibers, int64_t n_nodes, const 
     return fdm_report_error(FDM_ERR_ARG, "fdm_diffusion_solve_noalloc: fiber offsets [" + std::to_string(ends[0]) +
                                              ", " + std::to_string(ends[1]) + "] outside [0, n_nodes = " +
                                              std::to_string(n_nodes) + "]");
-  double* coef = scratch;
-  double* fwd = scratch + 6 * (size_t)n_nodes;
-  e = fdm::launch_coefficients(n_fibers, d_fiber_offsets, d_element_lengths, d_prefactor, dt,
-                               diffusion_scheme == FDM_IMPLICIT_EULER, coef, n_nodes, st);
-  if (e == cudaSuccess)
-    e = fdm::launch_diffusion(n_fibers, d_fiber_offsets, coef, n_nodes, d_vm, fwd, st);
+  e = fdm::launch_diffusion_operator(n_fibers, n_nodes, d_fiber_offsets, d_element_lengths, d_prefactor, dt,
+                                     diffusion_scheme == FDM_IMPLICIT_EULER, d_vm, scratch, st);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(st);
   if (e != cudaSuccess)

@@ -1,10 +1,14 @@
 """The split path's kernels at the sizes where their work partition changes: the stimulation schedule (a warp per
-fiber, 32 substeps at a time)."""
+fiber, 32 substeps at a time), the factorization (chunks started speculatively, tiles) and the diffusion solves."""
+import ctypes as C
+
 import numpy as np
 import pytest
+import torch
 
 import helpers as H
 from oracle import oracle as O
+from opendihu_b200 import _native as N
 from opendihu_b200 import solver as S
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +48,56 @@ def test_schedule_word_edges(frequency, repeat, dt0, steps):
         np.testing.assert_array_equal(log["fiber"], f[order])
         # every clamp decision equal: FP64 Vm within rounding of the oracle's
         assert np.max(np.abs(vm - ref[0])) < 1e-8
+
+
+def _tridiagonal(h, pf, dt, scheme, u):
+    """One diffusion solve by dense elimination: (K - M/dt) x = -M/dt u or its Crank-Nicolson form."""
+    n = len(h) + 1
+    K, M = np.zeros((n, n)), np.zeros((n, n))
+    for e, he in enumerate(h):
+        K[e:e + 2, e:e + 2] += pf / he * np.array([[-1.0, 1.0], [1.0, -1.0]])
+        M[e:e + 2, e:e + 2] += he / 6 * np.array([[2.0, 1.0], [1.0, 2.0]])
+    if scheme == "ImplicitEuler":
+        return np.linalg.solve(K - M / dt, -M / dt @ u)
+    return np.linalg.solve(K / 2 - M / dt, (-K / 2 - M / dt) @ u)
+
+
+# lengths around the chunks (a warm-up of 12 nodes), the 256 threads and the tile of 2560 nodes; dt = 10 couples the
+# nodes so strongly that no chunk's guess is right and the rounds run
+@pytest.mark.parametrize("lengths", [[2, 3, 12, 13, 14, 101], [255, 256, 257, 511, 512, 513], [2559, 2560, 2561],
+                                     [5120, 5200]])
+@pytest.mark.parametrize("scheme", ["ImplicitEuler", "CrankNicolson"])
+@pytest.mark.parametrize("dt", [1e-3, 10.0])
+def test_diffusion_operator(lengths, scheme, dt):
+    rng = np.random.default_rng(5)
+    off = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64)
+    h = 0.01 * rng.uniform(0.8, 1.2, off[-1] - len(lengths))
+    pf = rng.uniform(2.5, 5.0, len(lengths)) / 500
+    u = rng.uniform(-80.0, 40.0, off[-1])
+    ref = np.concatenate([_tridiagonal(h[off[f] - f:off[f + 1] - f - 1], pf[f], dt, scheme, u[off[f]:off[f + 1]])
+                          for f in range(len(lengths))])
+    dev = [torch.from_numpy(x).cuda() for x in (off, h, pf)]
+    for entry in ("fdm_diffusion_solve", "fdm_diffusion_solve_noalloc"):
+        x = torch.from_numpy(u.copy()).cuda()
+        N.check(getattr(N.lib(), entry)(len(lengths), len(u), *[C.c_void_p(d.data_ptr()) for d in dev], dt,
+                                        S.SCHEMES[scheme], C.c_void_p(x.data_ptr()), None))
+        torch.cuda.synchronize()
+        # condition number: at most 4 pf/h dt / (h/3) + 3, about 2e4 at dt = 10; 100 roundings of it
+        assert np.max(np.abs(x.cpu().numpy() - ref)) < 80 * 2.3e-16 * 100 * max(1.0, 2e3 * dt)
+
+
+@pytest.mark.parametrize("lengths", [[41] * 600, [40 + k % 89 for k in range(600)], [40 + k % 217 for k in range(600)], [257 + k % 40 for k in range(595)],
+                                     [2, 511, 512, 513], [1024, 1025, 1537, 2049], [2560], [2561, 40], [2570] * 592])
+def test_split_diffusion_partitions(lengths):
+    s = S.uniform_fibers(H.HH, lengths, 0.01, 3.828 / 500, call_frequency=0.1, repeat_after_first_call=0.1,
+                         call_enable_begin=0.0, end_time=2e-3, dt_0d=5e-4, dt_1d=1e-3, dt_splitting=1e-3,
+                         dt_repeated_call=1e-3, clamp_rule="center", diffusion_scheme="CrankNicolson")
+    rng = np.random.default_rng(1)
+    s = H.complete(s)
+    s.states = s.states.copy()
+    s.states[0] += rng.uniform(0.0, 60.0, s.n_nodes)
+    ref = H.run_oracle(s.copy())[0]
+    with S.FastMonodomainSolver(s.copy(), method="split", precision="fp64") as slv:
+        slv.advanceTimeSpan()
+        got = slv.states()
+    assert np.max(np.abs(got - ref)) < 1e-9
