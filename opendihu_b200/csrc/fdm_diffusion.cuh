@@ -42,8 +42,9 @@ struct ElementTerms {
 // in scratch between the two sweeps).  Threads hold an odd number of consecutive nodes, so that their shared-memory
 // accesses, that many doubles apart, meet no bank twice.
 // Bound by FP64 work (two divisions per element, two to three per node with the warm-up) and latency; a thread per
-// fiber, with six divisions and six uncoalesced stores per node, took 2519 us for the factorization of 4096 fibers of 500 to
-// 2500 nodes and a solve 524 us more; FACTOR_SOLVE does both in 214 us.  (64 fibers of 1481 nodes: 1129 us, now 8.)
+// fiber, with six divisions and six uncoalesced stores per node, took 2519 us for the factorization of 4096 fibers of
+// 500 to 2500 nodes and a solve 524 us more; FACTOR_SOLVE does both in 214 us.  (64 fibers of 1481 nodes: 1129 us,
+// now 8.)
 constexpr int FACTOR_T = 256;
 constexpr int FACTOR_M = 11;          // most nodes per thread (odd)
 constexpr int FACTOR_TILE = 2560;
@@ -228,9 +229,9 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
 // partition follows from the fiber's own length alone: a fiber's result does not depend on the fibers beside it.
 // eq_counter / eq_nbuf (or null): the equilibrium skip's per-rank count of inactive buffers and number of
 // buffers; a fiber of a rank whose buffers are all counted inactive is not solved (compute.tpp:261-265)
-// Bound by the latency of the loads and the two scans for few fibers (16 x 1481: 6.5 us with a loop over the nodes and d'
-// in memory, now 4.4), by memory for many (1024 fibers of 500 to 2500 nodes: 156 us with a warp per fiber and its
-// uncoalesced chunks, now 31.7; 100 MB, 0.5 of the measured copy rate).
+// Bound by the latency of the loads and the two scans for few fibers (16 x 1481: 6.5 us with a loop over the nodes
+// and d' in memory, now 4.4), by memory for many (1024 fibers of 500 to 2500 nodes: 156 us with a warp per fiber and
+// its uncoalesced chunks, now 31.7; 100 MB, 0.5 of the measured copy rate).
 constexpr int DIFFUSION_T = 256;
 
 template<int M>
@@ -261,7 +262,8 @@ __global__ void __launch_bounds__(DIFFUSION_T) diffusion_reg_kernel(const int64_
     if (j < cnt) {
       F[j] = c0[j];
       C[j] = c0[2 * stride + j];
-      G[j] = c0[stride + j] * (c0[3 * stride + j] * u[j] + c0[4 * stride + j] * u[j + 1] + c0[5 * stride + j] * u[j + 2]);
+      G[j] = c0[stride + j] *
+             (c0[3 * stride + j] * u[j] + c0[4 * stride + j] * u[j + 1] + c0[5 * stride + j] * u[j + 2]);
     } else {
       F[j] = 1.0;   // the identity map
       C[j] = -1.0;

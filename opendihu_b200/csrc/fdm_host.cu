@@ -2229,6 +2229,7 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
       ra.step = j;
       for (int half = 0; half < 2; half++) {
         ra.half = half;
+        ra.n_halves = 1;
         ra.store_alg = (store_alg && s->n_alg_out > 0 && half == 1 && j == n_steps - 1) ? 1 : 0;
         L.st_in = E.st[cur].p;
         L.st_out = E.st[cur ^ 1].p;
@@ -2245,6 +2246,29 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
     }
     return FDM_OK;
   }
+  // Launches of the window: the first half step, the diffusion solve, then per following split step one launch of the
+  // second half step and the next one's first (nothing lies between them: one launch and one pass over the states
+  // instead of two), the diffusion solve; the second half step of the last one.  (16 x 1481 fibers FP64, 400 steps:
+  // 8.26 -> 7.47 ms; 1024 uneven fibers, 50 steps: 19.3 -> 18.8.)
+  auto launches = [&](auto&& reaction, auto&& diffusion) -> cudaError_t {
+    cudaError_t e = cudaSuccess;
+    for (int j = 0; j <= n_steps && e == cudaSuccess; j++) {
+      ra.step = j == 0 ? 0 : j - 1;
+      ra.half = j == 0 ? 0 : 1;
+      ra.n_halves = j > 0 && j < n_steps ? 2 : 1;
+      ra.store_alg = store_alg && s->n_alg_out > 0 && j == n_steps ? 1 : 0;
+      e = reaction();
+      if (e == cudaSuccess && j < n_steps)
+        e = diffusion();
+    }
+    return e;
+  };
+  auto reaction = [&]() { return launch_reaction(s->cfg.model, rk, mk, ra, s->stream); };
+  auto diffusion = [&]() {
+    return launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p, s->max_fiber_len,
+                            s->stream);
+  };
+  s->launches += 2 * (int64_t)n_steps + 1;
   // without profiling, a window that stores no algebraics replays a captured CUDA graph of its launches
   const bool graph_ok = s->cfg.use_graph && !prof && !(store_alg && s->n_alg_out > 0);
   if (graph_ok) {
@@ -2253,18 +2277,7 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
     if (it == s->graphs.end()) {
       cudaGraph_t g = nullptr;
       FDM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t ce = cudaSuccess;
-      for (int j = 0; j < n_steps && ce == cudaSuccess; j++) {
-        ra.step = j;
-        for (int half = 0; half < 2 && ce == cudaSuccess; half++) {
-          ra.half = half;
-          ra.store_alg = 0;
-          ce = launch_reaction(s->cfg.model, rk, mk, ra, s->stream);
-          if (ce == cudaSuccess && half == 0)
-            ce = launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                       s->max_fiber_len, s->stream);
-        }
-      }
+      const cudaError_t ce = launches(reaction, diffusion);
       cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
       if (ce != cudaSuccess)
         return cuda_fail(s, ce, "capture of the window launches");
@@ -2276,31 +2289,18 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
       it = s->graphs.emplace(key, ex).first;
     }
     FDM_CUDA(cudaGraphLaunch(it->second, s->stream));
-    s->launches += 3 * (int64_t)n_steps;
     return FDM_OK;
   }
-  for (int j = 0; j < n_steps; j++) {
-    ra.step = j;
-    for (int half = 0; half < 2; half++) {
-      ra.half = half;
-      ra.store_alg = (store_alg && s->n_alg_out > 0 && half == 1 && j == n_steps - 1) ? 1 : 0;
-      cudaEvent_t e0 = nullptr, e1 = nullptr;
-      if (prof) {
-        e0 = next_event(s);
-        e1 = next_event(s);
-        FDM_CUDA(cudaEventRecord(e0, s->stream));
-      }
-      FDM_CUDA(launch_reaction(s->cfg.model, rk, mk, ra, s->stream));
-      s->launches++;
-      if (prof)
-        FDM_CUDA(cudaEventRecord(e1, s->stream));
-      if (half == 0) {
-        FDM_CUDA(launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                       s->max_fiber_len, s->stream));
-        s->launches++;
-      }
-    }
-  }
+  auto timed_reaction = [&]() -> cudaError_t {
+    if (!prof)
+      return reaction();
+    const cudaEvent_t e0 = next_event(s), e1 = next_event(s);
+    cudaError_t e = cudaEventRecord(e0, s->stream);
+    if (e == cudaSuccess)
+      e = reaction();
+    return e == cudaSuccess ? cudaEventRecord(e1, s->stream) : e;
+  };
+  FDM_CUDA(launches(timed_reaction, diffusion));
   return FDM_OK;
 }
 
@@ -3430,26 +3430,27 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
     ra.stimulus_parameter = s->cfg.stimulus_parameter;
     ra.stimulus_value = s->cfg.stimulus_value;
     ra.steps = s->steps_d.p;
-    for (int jj = 0; jj < len; jj++) {
-      if (!pipelined) {
-        rc = ensure_coefficients(s, A.dt1s[b + jj]);
-        if (rc)
-          return rc;
-      }
-      ra.step = jj;
-      for (int half = 0; half < 2; half++) {
-        ra.half = half;
-        ra.store_states = A.H[k].p + ((size_t)jj * 2 + half) * hstride;
-        // Vm before the diffusion solve (U) comes out of the first half step; Vm after it is the stored input
-        // of the second half step's first substep
-        ra.store_vm_out = half == 0 ? A.U[k].p + (size_t)jj * N : nullptr;
-        FDM_CUDA(launch_reaction(s->cfg.model, REAL_F64, mk, ra, s->stream));
-        s->launches++;
-        if (half == 0) {
-          FDM_CUDA(launch_diffusion(nf, s->off_d.p, coef_of(b + jj), N, s->vm.p, s->scratch.p,
-                                    s->max_fiber_len, s->stream));
-          s->launches++;
+    // launches as in run_window: the second half step of a split step and the first of the next one together
+    ra.store_half_stride = (int64_t)hstride;
+    for (int jj = 0; jj <= len; jj++) {
+      ra.step = jj == 0 ? 0 : jj - 1;
+      ra.half = jj == 0 ? 0 : 1;
+      ra.n_halves = jj > 0 && jj < len ? 2 : 1;
+      ra.store_states = A.H[k].p + ((size_t)ra.step * 2 + ra.half) * hstride;
+      // Vm before the diffusion solve (U) comes out of the first half step; Vm after it is the stored input
+      // of the second half step's first substep
+      ra.store_vm_out = jj < len ? A.U[k].p + (size_t)jj * N : nullptr;
+      FDM_CUDA(launch_reaction(s->cfg.model, REAL_F64, mk, ra, s->stream));
+      s->launches++;
+      if (jj < len) {
+        if (!pipelined) {
+          rc = ensure_coefficients(s, A.dt1s[b + jj]);
+          if (rc)
+            return rc;
         }
+        FDM_CUDA(launch_diffusion(nf, s->off_d.p, coef_of(b + jj), N, s->vm.p, s->scratch.p,
+                                    s->max_fiber_len, s->stream));
+        s->launches++;
       }
     }
     FDM_CUDA(cudaEventRecord(A.replayed[k], s->stream));

@@ -581,6 +581,8 @@ struct ReactionArgs {
   const SplitStep* steps;
   int step;                       // index in window
   int half;                       // 0: first half step, 1: second
+  int n_halves;                   // 2 (half == 1): the first half step of the next split step follows in the same
+                                  // launch (nothing lies between the two)
   int store_alg;                  // store the requested algebraics after the last substep
   int n_alg_out;
   const int* alg_indices;         // device
@@ -591,8 +593,9 @@ struct ReactionArgs {
   int64_t trace_capacity;
   ActivationRec act;
   double* store_states;           // adjoint replay (FP64 only): input state of substep k at
-                                  // store_states[(k*nStates + s)*stride + node], or null
-  double* store_vm_out;           // adjoint replay: Vm after the half step also written here, or null
+                                  // store_states[(k*nStates + s)*stride + node], or null; a second half step's
+  int64_t store_half_stride;      // store_half_stride doubles further
+  double* store_vm_out;           // adjoint replay: Vm after the launch's half step 0 also written here, or null
   int per_node;                   // 1: one thread per node whatever the size (the adjoint's checkpointed
                                   // forward, which its replay reproduces bit for bit)
   const int* gate;                // onlyComputeIfHasBeenStimulated: per node gate code, or null
@@ -625,47 +628,53 @@ __global__ void __launch_bounds__(128) reaction_kernel(ReactionArgs a)
     Pstim[q] = (a.stimulus_mode == 1 && q == a.stimulus_parameter) ? (RR)a.stimulus_value : P[q];
   }
   const int cf = a.clamp_fiber[i];
-  const SplitStep s = a.steps[a.step];
-  const double t0 = a.half ? s.mid : s.t;
-  const int base = (a.step * 2 + a.half) * a.nsub_stride;
-  const int first = a.gate ? gate_first(a.gate_start, a.gate_stride, a.gate[i], a.step * 2 + a.half) : 0;
-  for (int k = 0; k < s.n0; k++) {
-    const double t = xadd(t0, xmul((double)k, s.dt0));
-    const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
-    const bool vclamp = stim && a.stimulus_mode == 0;
-    if (a.store_states) {
-      a.store_states[(int64_t)(k * NS) * a.stride + i] = V;
+#pragma unroll 1
+  for (int hh = 0; hh < a.n_halves; hh++) {
+    const int hs = a.step * 2 + a.half + hh; // half step of the window
+    const SplitStep s = a.steps[hs >> 1];
+    const double t0 = (hs & 1) ? s.mid : s.t;
+    const int base = hs * a.nsub_stride;
+    const int first = a.gate ? gate_first(a.gate_start, a.gate_stride, a.gate[i], hs) : 0;
+#pragma unroll 1
+    for (int k = 0; k < s.n0; k++) {
+      const double t = xadd(t0, xmul((double)k, s.dt0));
+      const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
+      const bool vclamp = stim && a.stimulus_mode == 0;
+      if (a.store_states) {
+        double* out = a.store_states + hh * a.store_half_stride;
+        out[(int64_t)(k * NS) * a.stride + i] = V;
 #pragma unroll
-      for (int s2 = 1; s2 < NS; s2++)
-        a.store_states[(int64_t)(k * NS + s2) * a.stride + i] = (double)S[s2 - 1];
-    }
-    if (k < first)
-      continue; // not computed before the attributed fiber was stimulated
-    RR Pk[NP];
+        for (int s2 = 1; s2 < NS; s2++)
+          out[(int64_t)(k * NS + s2) * a.stride + i] = (double)S[s2 - 1];
+      }
+      if (k < first)
+        continue; // not computed before the attributed fiber was stimulated
+      RR Pk[NP];
 #pragma unroll
-    for (int q = 0; q < NP; q++)
-      Pk[q] = (stim && a.stimulus_mode == 1) ? Pstim[q] : P[q];
-    if (a.store_alg && k == s.n0 - 1) {
-      RR alg[Model::nAlgebraics];
-      heun_step<Model, RR, Math, true>(V, S, L, Pk, t, s.dt0, vclamp, a.vstim, alg);
-      store_algebraics<Model>(alg, a.n_alg_out, a.alg_indices, a.alg_out, a.n_nodes, i);
-    } else {
-      heun_step<Model, RR, Math, false>(V, S, L, Pk, t, s.dt0, vclamp, a.vstim, nullptr);
+      for (int q = 0; q < NP; q++)
+        Pk[q] = (stim && a.stimulus_mode == 1) ? Pstim[q] : P[q];
+      if (a.store_alg && k == s.n0 - 1) {
+        RR alg[Model::nAlgebraics];
+        heun_step<Model, RR, Math, true>(V, S, L, Pk, t, s.dt0, vclamp, a.vstim, alg);
+        store_algebraics<Model>(alg, a.n_alg_out, a.alg_indices, a.alg_out, a.n_nodes, i);
+      } else {
+        heun_step<Model, RR, Math, false>(V, S, L, Pk, t, s.dt0, vclamp, a.vstim, nullptr);
+      }
     }
+    if ((hs & 1) && a.trace_slot) {
+      const int slot = a.trace_slot[i];
+      if (slot >= 0)
+        record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, V);
+    }
+    if (!(hs & 1) && a.store_vm_out)
+      a.store_vm_out[i] = V;
   }
   a.vm[i] = V;
-  if (a.store_vm_out)
-    a.store_vm_out[i] = V;
 #pragma unroll
   for (int s2 = 1; s2 < NS; s2++) {
     st[(s2 - 1) * a.stride + i] = S[s2 - 1];
     if (Compensated<RR>::value)
       stl[(s2 - 1) * a.stride + i] = L[s2 - 1];
-  }
-  if (a.half == 1 && a.trace_slot) {
-    const int slot = a.trace_slot[i];
-    if (slot >= 0)
-      record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, V);
   }
 }
 
@@ -709,50 +718,52 @@ __global__ void __launch_bounds__(32 * (Model::nGroups > 0 ? Model::nGroups : 1)
     Pstim[q] = (a.stimulus_mode == 1 && q == a.stimulus_parameter) ? a.stimulus_value : P[q];
   }
   const int cf = ok ? a.clamp_fiber[i] : -1;
-  const SplitStep s = a.steps[a.step];
-  const double t0 = a.half ? s.mid : s.t;
-  const int base = (a.step * 2 + a.half) * a.nsub_stride;
+  const int slot = (ok && g == 0 && a.trace_slot) ? a.trace_slot[i] : -1;
   __syncthreads();
-  for (int k = 0; k < s.n0; k++) {
-    const double t = xadd(t0, xmul((double)k, s.dt0));
-    const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
-    const bool vclamp = stim && a.stimulus_mode == 0;
-    double Pk[NP];
+#pragma unroll 1
+  for (int hh = 0; hh < a.n_halves; hh++) {
+    const int hs = a.step * 2 + a.half + hh; // half step of the window
+    const SplitStep s = a.steps[hs >> 1];
+    const double t0 = (hs & 1) ? s.mid : s.t;
+    const int base = hs * a.nsub_stride;
+#pragma unroll 1
+    for (int k = 0; k < s.n0; k++) {
+      const double t = xadd(t0, xmul((double)k, s.dt0));
+      const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
+      const bool vclamp = stim && a.stimulus_mode == 0;
+      double Pk[NP];
 #pragma unroll
-    for (int q = 0; q < NP; q++)
-      Pk[q] = (stim && a.stimulus_mode == 1) ? Pstim[q] : P[q];
-    double y[NS];
+      for (int q = 0; q < NP; q++)
+        Pk[q] = (stim && a.stimulus_mode == 1) ? Pstim[q] : P[q];
+      double y[NS];
 #pragma unroll
-    for (int q = 0; q < NS; q++)
-      y[q] = sy[q][lane];
-    const double r = group_rate<Model, Math, 0>(g, t, y, Pk);
-    double ys = own + s.dt0 * r;
-    if (g == 0 && vclamp)
-      ys = a.vstim;
-    sys[g][lane] = ys;
-    __syncthreads();
+      for (int q = 0; q < NS; q++)
+        y[q] = sy[q][lane];
+      const double r = group_rate<Model, Math, 0>(g, t, y, Pk);
+      double ys = own + s.dt0 * r;
+      if (g == 0 && vclamp)
+        ys = a.vstim;
+      sys[g][lane] = ys;
+      __syncthreads();
 #pragma unroll
-    for (int q = 0; q < NS; q++)
-      y[q] = sys[q][lane];
-    const double r2 = group_rate<Model, Math, 0>(g, t, y, Pk);
-    own += 0.5 * s.dt0 * (r + r2);
-    if (g == 0 && vclamp)
-      own = a.vstim;
-    sy[g][lane] = own;
-    __syncthreads();
+      for (int q = 0; q < NS; q++)
+        y[q] = sys[q][lane];
+      const double r2 = group_rate<Model, Math, 0>(g, t, y, Pk);
+      own += 0.5 * s.dt0 * (r + r2);
+      if (g == 0 && vclamp)
+        own = a.vstim;
+      sy[g][lane] = own;
+      __syncthreads();
+    }
+    if ((hs & 1) && slot >= 0)
+      record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, own);
   }
   if (!ok)
     return;
-  if (g == 0) {
+  if (g == 0)
     a.vm[i] = own;
-    if (a.half == 1 && a.trace_slot) {
-      const int slot = a.trace_slot[i];
-      if (slot >= 0)
-        record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, own);
-    }
-  } else {
+  else
     ((double*)a.states)[(g - 1) * a.stride + i] = own;
-  }
 }
 
 // affine map x -> F x + G; compose(first, second) = second o first

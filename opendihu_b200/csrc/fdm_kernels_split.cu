@@ -203,8 +203,8 @@ cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const d
   if (n_fibers == 0)
     return cudaSuccess;
   const int nr = n_ranks > 0 ? n_ranks : 1;
-  // many short fibers: a warp per fiber, as half of a CTA's threads would have no node (4096 fibers: of 100 nodes 12.5 us
-  // against 18.5 us with a CTA each, of 200 nodes 20.6 against 18.5; 592 fibers of 100 nodes: 6.2 us both)
+  // many short fibers: a warp per fiber, as half of a CTA's threads would have no node (4096 fibers: of 100 nodes
+  // 12.5 us against 18.5 us with a CTA each, of 200 nodes 20.6 against 18.5; 592 fibers of 100 nodes: 6.2 us both)
   const bool many = n_fibers >= DIFFUSION_BLOCK_MAX_FIBERS;
   if (!(many && max_fiber_len <= DIFFUSION_T / 2)) {
     switch ((max_fiber_len + 2 * DIFFUSION_T - 1) / (2 * DIFFUSION_T)) {

@@ -86,8 +86,8 @@ def test_diffusion_operator(lengths, scheme, dt):
         assert np.max(np.abs(x.cpu().numpy() - ref)) < 80 * 2.3e-16 * 100 * max(1.0, 2e3 * dt)
 
 
-@pytest.mark.parametrize("lengths", [[41] * 600, [40 + k % 89 for k in range(600)], [40 + k % 217 for k in range(600)], [257 + k % 40 for k in range(595)],
-                                     [2, 511, 512, 513], [1024, 1025, 1537, 2049], [2560], [2561, 40], [2570] * 592])
+@pytest.mark.parametrize("lengths", [[41] * 600, [40 + k % 89 for k in range(600)], [40 + k % 217 for k in range(600)],
+                                     [257 + k % 40 for k in range(595)], [2, 511, 512, 513], [1024, 1025, 1537, 2049], [2560], [2561, 40], [2570] * 592])
 def test_split_diffusion_partitions(lengths):
     s = S.uniform_fibers(H.HH, lengths, 0.01, 3.828 / 500, call_frequency=0.1, repeat_after_first_call=0.1,
                          call_enable_begin=0.0, end_time=2e-3, dt_0d=5e-4, dt_1d=1e-3, dt_splitting=1e-3,
