@@ -282,8 +282,8 @@ struct fdm_solver {
   std::vector<cudaEvent_t> xfer_ev;
   DevBuf<double> xfer64; // direct transfers from fdm_host_alloc memory: the other states in FP64 (FP32 mode)
 
-  // split-path window graphs: (steps, words, nsub, flags pointer) -> executable graph
-  std::map<std::tuple<int, int, int, const void*>, cudaGraphExec_t> graphs;
+  // split-path window graphs: (steps, words, nsub, flags pointer) -> executable graph and its number of launches
+  std::map<std::tuple<int, int, int, const void*>, std::pair<cudaGraphExec_t, int64_t>> graphs;
 
   // timing
   std::vector<cudaEvent_t> ev_pool;
@@ -339,7 +339,7 @@ static void invalidate_graphs(fdm_solver* s)
   s->xfer_ev.clear();
   s->xfer64.release();
   for (auto& kv : s->graphs)
-    cudaGraphExecDestroy(kv.second);
+    cudaGraphExecDestroy(kv.second.first);
   s->graphs.clear();
 }
 
@@ -604,7 +604,7 @@ extern "C" int fdm_destroy(fdm_solver* s)
   s->steps_d.release();
   s->adj.release();
   for (auto& kv : s->graphs)
-    cudaGraphExecDestroy(kv.second);
+    cudaGraphExecDestroy(kv.second.first);
   s->graphs.clear();
   if (s->stage)
     cudaFreeHost(s->stage);
@@ -1580,7 +1580,7 @@ static int eq_build(fdm_solver* s, const std::vector<int>& center)
     FDM_CUDA(E.st[k].alloc(std::max<int64_t>(E.n_buffers, 1)));
   FDM_CUDA(E.info.alloc(std::max<int64_t>(E.n_buffers, 1)));
   FDM_CUDA(E.prefix.alloc(std::max<int64_t>(E.n_buffers, 1)));
-  FDM_CUDA(E.block_agg.alloc(std::max<int64_t>((E.n_buffers + EQ_SCAN_T - 1) / EQ_SCAN_T, 1)));
+  FDM_CUDA(E.block_agg.alloc(std::max<int64_t>((E.n_buffers * W + EQ_T - 1) / EQ_T + E.n_buffers / EQ_SCAN_T + 1, 1)));
   FDM_CUDA(E.ran_b.alloc(std::max<int64_t>(nt, 1)));
   FDM_CUDA(E.vm_pad.alloc(std::max(n_pad, 1)));
   FDM_CUDA(E.states_pad.alloc(nsm * std::max(n_pad, 1) * rb));
@@ -2188,6 +2188,37 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
   ra.trace_capacity = s->trace_capacity;
   ra.act = activation_rec(s);
   ra.per_node = s->adj_forward ? 1 : 0;
+  // without profiling, a window that stores no algebraics replays a captured CUDA graph of its launches; *n_launches
+  // is their number once they were issued
+  auto replay_or_launch = [&](auto&& launches, const int* n_launches) -> int {
+    if (!s->cfg.use_graph || prof || (store_alg && s->n_alg_out > 0)) {
+      FDM_CUDA(launches());
+      s->launches += *n_launches;
+      return FDM_OK;
+    }
+    const auto key = std::make_tuple(n_steps, words, nsub, (const void*)s->flags.p);
+    auto it = s->graphs.find(key);
+    if (it == s->graphs.end()) {
+      cudaGraph_t g = nullptr;
+      FDM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+      const cudaError_t ce = launches();
+      cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
+      if (ce != cudaSuccess) {
+        if (g)
+          cudaGraphDestroy(g);
+        return cuda_fail(s, ce, "capture of the window launches");
+      }
+      FDM_CUDA(ee);
+      cudaGraphExec_t ex = nullptr;
+      cudaError_t ie = cudaGraphInstantiate(&ex, g, 0);
+      cudaGraphDestroy(g);
+      FDM_CUDA(ie);
+      it = s->graphs.emplace(key, std::make_pair(ex, (int64_t)*n_launches)).first;
+    }
+    FDM_CUDA(cudaGraphLaunch(it->second.first, s->stream));
+    s->launches += it->second.second;
+    return FDM_OK;
+  };
   if (s->eq.on) {
     // equilibrium skip: every half step is a speculative reaction, the buffer scan and a commit; the statuses
     // alternate between the two status arrays, and a window has an even number of half steps
@@ -2207,6 +2238,10 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
     L.buf_rank = E.buf_rank.p;
     L.rank_first = E.rank_first.p;
     L.counter = E.counter.p;
+    L.info = E.info.p;
+    L.prefix = E.prefix.p;
+    L.block_agg = E.block_agg.p;
+    L.in_warp = 32 % L.W == 0;
     EqSpec e{};
     e.nt = nt;
     e.vm_pad = E.vm_pad.p;
@@ -2224,27 +2259,32 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
     e.stl_b = E.stl_b.p;
     e.alg_b = E.alg_b.p;
     e.ran_b = E.ran_b.p;
-    int cur = 0;
-    for (int j = 0; j < n_steps; j++) {
-      ra.step = j;
-      for (int half = 0; half < 2; half++) {
-        ra.half = half;
-        ra.n_halves = 1;
-        ra.store_alg = (store_alg && s->n_alg_out > 0 && half == 1 && j == n_steps - 1) ? 1 : 0;
-        L.st_in = E.st[cur].p;
-        L.st_out = E.st[cur ^ 1].p;
-        FDM_CUDA(launch_equilibrium_half(s->cfg.model, rk, mk, ra, L, e, E.info.p, E.prefix.p, E.block_agg.p,
-                                         s->model->n_states, half == 1, s->stream));
-        s->launches += 6;
-        cur ^= 1;
-        if (half == 0) {
-          FDM_CUDA(launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
-                                         s->max_fiber_len, s->stream, E.counter.p, E.nbuf.p, s->cfg.n_ranks));
-          s->launches++;
+    int n_launches = 0;
+    auto eq_launches = [&]() -> cudaError_t {
+      int cur = 0;
+      for (int j = 0; j < n_steps; j++) {
+        ra.step = j;
+        for (int half = 0; half < 2; half++) {
+          ra.half = half;
+          ra.n_halves = 1;
+          ra.store_alg = (store_alg && s->n_alg_out > 0 && half == 1 && j == n_steps - 1) ? 1 : 0;
+          L.st_in = E.st[cur].p;
+          L.st_out = E.st[cur ^ 1].p;
+          cudaError_t ce = launch_equilibrium_half(s->cfg.model, rk, mk, ra, L, e, s->model->n_states, &n_launches,
+                                                   s->stream);
+          cur ^= 1;
+          if (ce == cudaSuccess && half == 0) {
+            ce = launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p,
+                                  s->max_fiber_len, s->stream, E.counter.p, E.nbuf.p, s->cfg.n_ranks);
+            n_launches++;
+          }
+          if (ce != cudaSuccess)
+            return ce;
         }
       }
-    }
-    return FDM_OK;
+      return cudaSuccess;
+    };
+    return replay_or_launch(eq_launches, &n_launches);
   }
   // Launches of the window: the first half step, the diffusion solve, then per following split step one launch of the
   // second half step and the next one's first (nothing lies between them: one launch and one pass over the states
@@ -2268,29 +2308,6 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
     return launch_diffusion(s->n_fibers, s->off_d.p, s->coef.p, s->n_nodes, s->vm.p, s->scratch.p, s->max_fiber_len,
                             s->stream);
   };
-  s->launches += 2 * (int64_t)n_steps + 1;
-  // without profiling, a window that stores no algebraics replays a captured CUDA graph of its launches
-  const bool graph_ok = s->cfg.use_graph && !prof && !(store_alg && s->n_alg_out > 0);
-  if (graph_ok) {
-    const auto key = std::make_tuple(n_steps, words, nsub, (const void*)s->flags.p);
-    auto it = s->graphs.find(key);
-    if (it == s->graphs.end()) {
-      cudaGraph_t g = nullptr;
-      FDM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-      const cudaError_t ce = launches(reaction, diffusion);
-      cudaError_t ee = cudaStreamEndCapture(s->stream, &g);
-      if (ce != cudaSuccess)
-        return cuda_fail(s, ce, "capture of the window launches");
-      FDM_CUDA(ee);
-      cudaGraphExec_t ex = nullptr;
-      cudaError_t ie = cudaGraphInstantiate(&ex, g, 0);
-      cudaGraphDestroy(g);
-      FDM_CUDA(ie);
-      it = s->graphs.emplace(key, ex).first;
-    }
-    FDM_CUDA(cudaGraphLaunch(it->second, s->stream));
-    return FDM_OK;
-  }
   auto timed_reaction = [&]() -> cudaError_t {
     if (!prof)
       return reaction();
@@ -2300,8 +2317,8 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
       e = reaction();
     return e == cudaSuccess ? cudaEventRecord(e1, s->stream) : e;
   };
-  FDM_CUDA(launches(timed_reaction, diffusion));
-  return FDM_OK;
+  int n_launches = 2 * n_steps + 1;
+  return replay_or_launch([&]() { return launches(timed_reaction, diffusion); }, &n_launches);
 }
 
 // The split steps of RepeatedCall<FastMonodomainSolver>::advanceTimeSpan over [t_start, t_end]

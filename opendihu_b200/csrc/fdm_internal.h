@@ -75,10 +75,9 @@ cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const d
                              double* vm, double* scratch, int64_t max_fiber_len, cudaStream_t s,
                              const int* eq_counter = nullptr, const int* eq_nbuf = nullptr, int n_ranks = 1);
 // one half step with the equilibrium skip (fdm_equilibrium.cuh): speculative reaction, equilibrium tests,
-// scan of the buffers, commit (and the trace after half 1)
+// scan of the buffers, commit (and the trace after half 1); adds the number of its launches to *n_launches
 cudaError_t launch_equilibrium_half(int model, RealKind rk, MathKind mk, const ReactionArgs& a, const EqLayout& L,
-                                    const EqSpec& e, uint8_t* info, uint8_t* prefix, uint8_t* block_agg, int n_states,
-                                    bool trace, cudaStream_t s);
+                                    const EqSpec& e, int n_states, int* n_launches, cudaStream_t s);
 // adjoint (FP64)
 cudaError_t launch_adjoint_half(int model, MathKind mk, const AdjointArgs& a, cudaStream_t s);
 cudaError_t launch_adjoint_diffusion(int n_fibers, const int64_t* fiber_offsets, const double* element_lengths,

@@ -231,8 +231,7 @@ cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const d
 
 // ---- equilibrium skip ----
 cudaError_t launch_equilibrium_half(int model, RealKind rk, MathKind mk, const ReactionArgs& a, const EqLayout& L,
-                                    const EqSpec& e, uint8_t* info, uint8_t* prefix, uint8_t* block_agg, int n_states,
-                                    bool trace, cudaStream_t s)
+                                    const EqSpec& e, int n_states, int* n_launches, cudaStream_t s)
 {
   cudaError_t ce = cudaSuccess;
   switch (model) {
@@ -247,21 +246,22 @@ cudaError_t launch_equilibrium_half(int model, RealKind rk, MathKind mk, const R
   }
   if (ce != cudaSuccess || L.n_buffers == 0)
     return ce;
-  const int T = 128;
-  const unsigned bb = (unsigned)((L.n_buffers + T - 1) / T);
+  *n_launches += 2;
+  if (!L.in_warp) {
+    const int T = 128;
+    const unsigned bb = (unsigned)((L.n_buffers + T - 1) / T);
+    if (rk == REAL_F64)
+      eq_changed_kernel<double><<<bb, T, 0, s>>>(a, L, e, n_states);
+    else
+      eq_changed_kernel<float><<<bb, T, 0, s>>>(a, L, e, n_states);
+    eq_scan_block_kernel<<<(unsigned)((L.n_buffers + EQ_SCAN_T - 1) / EQ_SCAN_T), EQ_SCAN_T, 0, s>>>(L);
+    *n_launches += 2;
+  }
+  const unsigned blocks = (unsigned)((L.n_buffers * L.W + EQ_T - 1) / EQ_T);
   if (rk == REAL_F64)
-    eq_changed_kernel<double><<<bb, T, 0, s>>>(a, L, e, n_states, info);
+    eq_commit_kernel<double><<<blocks, EQ_T, 0, s>>>(a, L, e, n_states);
   else
-    eq_changed_kernel<float><<<bb, T, 0, s>>>(a, L, e, n_states, info);
-  const int64_t nblk = (L.n_buffers + EQ_SCAN_T - 1) / EQ_SCAN_T;
-  eq_scan_block_kernel<<<(unsigned)nblk, EQ_SCAN_T, 0, s>>>(L, info, prefix, block_agg);
-  eq_scan_top_kernel<<<1, 1, 0, s>>>(block_agg, nblk);
-  if (rk == REAL_F64)
-    eq_commit_kernel<double><<<bb, T, 0, s>>>(a, L, e, info, prefix, block_agg, n_states);
-  else
-    eq_commit_kernel<float><<<bb, T, 0, s>>>(a, L, e, info, prefix, block_agg, n_states);
-  if (trace && a.trace_slot)
-    eq_trace_kernel<<<(unsigned)((a.n_nodes + T - 1) / T), T, 0, s>>>(a);
+    eq_commit_kernel<float><<<blocks, EQ_T, 0, s>>>(a, L, e, n_states);
   return cudaGetLastError();
 }
 

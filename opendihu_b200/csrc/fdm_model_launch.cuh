@@ -74,11 +74,13 @@ inline cudaError_t equilibrium_search_model(MathKind mk, double* u, const double
 template<class Model, class RR, class Math>
 inline cudaError_t reaction_eq_one(const ReactionArgs& a, const EqLayout& L, const EqSpec& e, cudaStream_t s)
 {
-  const int T = 128;
-  const int64_t blocks = (e.nt + T - 1) / T;
+  const int64_t blocks = (e.nt + EQ_T - 1) / EQ_T;
   if (blocks == 0)
     return cudaSuccess;
-  reaction_eq_kernel<Model, RR, Math><<<(unsigned)blocks, T, 0, s>>>(a, L, e);
+  if (L.in_warp)
+    reaction_eq_kernel<Model, RR, Math, true><<<(unsigned)blocks, EQ_T, 0, s>>>(a, L, e);
+  else
+    reaction_eq_kernel<Model, RR, Math, false><<<(unsigned)blocks, EQ_T, 0, s>>>(a, L, e);
   return cudaGetLastError();
 }
 

@@ -101,3 +101,26 @@ def test_split_diffusion_partitions(lengths):
         slv.advanceTimeSpan()
         got = slv.states()
     assert np.max(np.abs(got - ref)) < 1e-9
+
+
+# lane widths that divide the warp (tested and scanned in the reaction kernel) and that do not (kernels of their own);
+# 5 fibers of 30 to 61 nodes, and enough nodes for several blocks of the scan
+@pytest.mark.parametrize("width,scale", [(1, 1), (2, 1), (3, 1), (5, 1), (16, 1), (4, 12), (3, 12), (8, 12)])
+def test_equilibrium_lane_widths(width, scale):
+    import test_gpu_equilibrium as EQ
+    from opendihu_b200 import workloads as WL
+    s = WL.batched_hh(clamp_rule="vc", n_fibers=5, min_nodes=30 * scale, max_nodes=61 * scale, seed=5, end_time=0.3,
+                      diffusion_scheme="ImplicitEuler", n_ranks=2, vc_width=width)
+    s.firing_events = np.array([[1, 0, 1, 1, 0]], np.uint8)
+    s.motor_unit_no = np.arange(5, dtype=np.int32)
+    H.complete(s)
+    s.states = np.repeat(EQ._rest()[:, None], s.n_nodes, axis=1)
+    s.skip_close_to_equilibrium = True
+    ref, ref_status, ref_counter, _ = EQ._oracle(s)
+    with S.FastMonodomainSolver(s.copy(), method="split", precision="fp64", steps_per_launch=7) as slv:
+        slv.advanceTimeSpan()
+        st = slv.states()
+        status, counter = slv.equilibrium_state()
+    assert np.max(np.abs(st - ref)) < 1e-8
+    np.testing.assert_array_equal(status, ref_status)
+    np.testing.assert_array_equal(counter, ref_counter)
