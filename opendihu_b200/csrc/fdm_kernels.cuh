@@ -603,8 +603,17 @@ struct ReactionArgs {
   int gate_stride;
 };
 
+// CTAs per SM the registers are held to.  A model of many states spills either way in FP64 (Shorten: 110 registers for its
+// states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 53,316 nodes, 25 substeps
+// 980 -> 770 us.  In FP32 its 255 registers hold everything (168: 481 -> 1173 us).
+template<class Model, class RR>
+constexpr int reaction_min_ctas()
+{
+  return sizeof(RR) == 8 && Model::nStates > 16 ? 3 : 1;
+}
+
 template<class Model, class RR, class Math>
-__global__ void __launch_bounds__(128) reaction_kernel(ReactionArgs a)
+__global__ void __launch_bounds__(128, reaction_min_ctas<Model, RR>()) reaction_kernel(ReactionArgs a)
 {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n_nodes)

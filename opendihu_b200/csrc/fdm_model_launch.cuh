@@ -18,9 +18,12 @@ inline cudaError_t reaction_one(const ReactionArgs& a, cudaStream_t s)
   return cudaGetLastError();
 }
 
-// up to this many nodes the FP64 split path advances a node's states on separate warps (reaction_group_kernel):
-// one thread per node would leave fewer than about 16 warps per SM
-constexpr int64_t kGroupKernelMaxNodes = 65536;
+// Up to this many nodes the FP64 split path advances a node's states on separate warps (reaction_group_kernel): six of its
+// CTAs of 32 nodes on each of 148 SMs.  The group form shortens a node's chain but needs a third more FP64 work and two
+// barriers per right-hand side, so it wins while latency counts (two half steps of 5 substeps: up to 12,000 nodes
+// 12.4 us against 14.5 us, 23,696 nodes 15.5 against 16.5) and loses once the FP64 pipe does (40,000 nodes 24.0
+// against 18.6, 94,784 nodes 43.3 against 32.7).
+constexpr int64_t kGroupKernelMaxNodes = 148 * 6 * 32;
 
 template<class Model, class Math>
 inline cudaError_t reaction_group_one(const ReactionArgs& a, cudaStream_t s)
