@@ -943,8 +943,9 @@ def _exp_shares(lines, consts):
 
 
 class _Fast64Emitter(_Emitter):
-    """FP64 form of the right-hand side.  In FP64 an exponential takes about 20 instructions and a division about
-    10, also one by a constant, so: products and quotients collect their constants into one factor (a division by
+    """FP64 form of the right-hand side, with the branch-free exponential and division of fdm_math.cuh (FDM_EXP,
+    FDM_DIV).  In FP64 an exponential takes about 20 instructions and a division about 10, also one by a constant,
+    so: products and quotients collect their constants into one factor (a division by
     a constant becomes a multiplication) and exponentials follow from each other (_exp_shares; None: every
     exponential evaluated, for approximations of it that do not turn sums into products).  Sums, gate terms and
     divisions by variables stay as the model writes them."""
@@ -983,7 +984,7 @@ class _Fast64Emitter(_Emitter):
                 for x in num[1:]:
                     text = f"({text} * {self.expr(x)})"
             for x in den:
-                text = f"({text} / {self.expr(x)})"
+                text = f"FDM_DIV({text}, {self.expr(x)})"
             return f"(-{text})" if c == -1.0 else text
         if t == "bin" and e[1] == "-":
             # 1 - exp(u), exp(u) - 1 with a derived exponential: exactly 0 where u is, as with the exponential itself
@@ -1035,7 +1036,7 @@ def _shares_used(exprs, shares) -> set:
     return used
 
 
-_MATH_MACROS = ["#define FDM_EXP(x) M::exp(x)", "#define FDM_LOG(x) M::log(x)", "#define FDM_POWF(x, y) M::pow(x, y)",
+_MATH_MACROS = ["#define FDM_EXP(x) M::fast_exp(x)", "#define FDM_DIV(x, y) M::fast_div(x, y)", "#define FDM_LOG(x) M::log(x)", "#define FDM_POWF(x, y) M::pow(x, y)",
                 "#define FDM_ABS(x) fabs(x)", "#define FDM_SQRT(x) sqrt(x)"]
 
 
@@ -1057,7 +1058,7 @@ def emit_rates_f64(lines, consts, pows) -> List[str]:
             tgt = f"ALGEBRAIC[{idx}]" if kind == "A" else f"RATES[{idx}]"
             out.append(f"    {tgt} = {em.expr(expr)};")
         out.extend(f"#undef FDM_POW{n}" for n in pows)
-        out.append("#undef FDM_EXP\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
+        out.append("#undef FDM_EXP\n#undef FDM_DIV\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
         out.append("  }")
     return out
 
@@ -1259,7 +1260,7 @@ def emit_group_rates(model: Model, params_alg: Sequence[int], params_const: Sequ
     out.append("    }")
     for n in pows:
         out.append(f"#undef FDM_POW{n}")
-    out.append("#undef FDM_EXP\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
+    out.append("#undef FDM_EXP\n#undef FDM_DIV\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
     out.append("  }")
     return out
 
@@ -1563,7 +1564,7 @@ class _VjpBuilder:
                     c = self.lit(1.0 / den[1])
                     return self.temp("*", [a, c], f"({a[1]} * {c[1]})")
                 b = self.build(e[3])
-                r = self.temp("rcp", [b], f"((({self.real})1) / {b[1]})")
+                r = self.temp("rcp", [b], f"M::fast_rcp({b[1]})")
                 return self.temp("*", [a, r], f"({a[1]} * {r[1]})")
             if op in "+-*/":
                 a = self.build(e[2])
@@ -1596,13 +1597,13 @@ class _VjpBuilder:
                         term = ("bin", "*", ("num", _hexf(coef), coef), ("var", kind, idx))
                         arg = term if arg is None else ("bin", "+", arg, term)
                     x = self.build(arg)
-                    self.group_temp[g] = self.temp("exp", [x], f"M::exp({x[1]})")
+                    self.group_temp[g] = self.temp("exp", [x], f"M::fast_exp({x[1]})")
                 ge = self.group_temp[g]
                 c = self.lit(math.exp(off))
                 return self.temp("*", [ge, c], f"({ge[1]} * {c[1]})")
             a = self.build(e[2][0])
             if f == "exp":
-                return self.temp("exp", [a], f"M::exp({a[1]})")
+                return self.temp("exp", [a], f"M::{'fast_exp' if self.fast else 'exp'}({a[1]})")
             if f == "log":
                 return self.temp("log", [a], f"M::log({a[1]})")
             if f == "fabs":

@@ -603,13 +603,15 @@ struct ReactionArgs {
   int gate_stride;
 };
 
-// CTAs per SM the registers are held to.  A model of many states spills either way in FP64 (Shorten: 110 registers for its
-// states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 53,316 nodes, 25 substeps
-// 980 -> 770 us.  In FP32 its 255 registers hold everything (168: 481 -> 1173 us).
+// CTAs of 128 threads per SM that the registers are held to.  A model of many states spills either way in FP64 (Shorten:
+// 110 registers for its states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 53,316
+// nodes, 25 substeps 980 -> 770 us (four CTAs: 905).  In FP32 its 255 registers hold everything (168: 481 -> 1173 us).
+// Hodgkin-Huxley in FP64 is bound by its dependent FP64 chains: six CTAs, 1,566,410 nodes, 10 substeps: 309 us against 350
+// with four and 318 with five.
 template<class Model, class RR>
 constexpr int reaction_min_ctas()
 {
-  return sizeof(RR) == 8 && Model::nStates > 16 ? 3 : 1;
+  return Model::nStates > 16 ? (sizeof(RR) == 8 ? 3 : 1) : (sizeof(RR) == 8 ? 6 : 8);
 }
 
 template<class Model, class RR, class Math>

@@ -54,7 +54,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
   __device__ __forceinline__ static void rates_f64(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)
   {
     (void)VOI; (void)PARAMS;
-#define FDM_EXP(x) M::exp(x)
+#define FDM_EXP(x) M::fast_exp(x)
+#define FDM_DIV(x, y) M::fast_div(x, y)
 #define FDM_LOG(x) M::log(x)
 #define FDM_POWF(x, y) M::pow(x, y)
 #define FDM_ABS(x) fabs(x)
@@ -64,13 +65,13 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_POW4(x) fdm_pow4(x)
     const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
     const R fdm_q0 = fdm_x0 * fdm_x0;
-    ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
+    ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
     ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
     RATES[1] = ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * fdm_x0);
-    ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
     RATES[2] = ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
-    ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
+    ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
     ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
     RATES[3] = ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
@@ -81,6 +82,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_POW3
 #undef FDM_POW4
 #undef FDM_EXP
+#undef FDM_DIV
 #undef FDM_LOG
 #undef FDM_POWF
 #undef FDM_ABS
@@ -90,7 +92,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
   __device__ __forceinline__ static void rates_f64_plain(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)
   {
     (void)VOI; (void)PARAMS;
-#define FDM_EXP(x) M::exp(x)
+#define FDM_EXP(x) M::fast_exp(x)
+#define FDM_DIV(x, y) M::fast_div(x, y)
 #define FDM_LOG(x) M::log(x)
 #define FDM_POWF(x, y) M::pow(x, y)
 #define FDM_ABS(x) fabs(x)
@@ -98,13 +101,13 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_POW2(x) fdm_pow2(x)
 #define FDM_POW3(x) fdm_pow3(x)
 #define FDM_POW4(x) fdm_pow4(x)
-    ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
     ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
     RATES[1] = ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
-    ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
     RATES[2] = ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
-    ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
+    ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
     ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
     RATES[3] = ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
@@ -115,6 +118,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_POW3
 #undef FDM_POW4
 #undef FDM_EXP
+#undef FDM_DIV
 #undef FDM_LOG
 #undef FDM_POWF
 #undef FDM_ABS
@@ -209,7 +213,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     (void)VOI; (void)PARAMS;
     R ALGEBRAIC[9];
     (void)ALGEBRAIC;
-#define FDM_EXP(x) M::exp(x)
+#define FDM_EXP(x) M::fast_exp(x)
+#define FDM_DIV(x, y) M::fast_div(x, y)
 #define FDM_LOG(x) M::log(x)
 #define FDM_POWF(x, y) M::pow(x, y)
 #define FDM_ABS(x) fabs(x)
@@ -226,7 +231,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     else if constexpr (G == 1 && SHARED) {
       const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
       const R fdm_q0 = fdm_x0 * fdm_x0;
-      ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
+      ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.85d6fd931e0bbp+3)) - ((R)1.0))));
       ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
       return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     }
@@ -234,13 +239,13 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
       const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
       const R fdm_q0 = fdm_x0 * fdm_x0;
       ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * fdm_x0);
-      ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), ((fdm_q0 * ((R)0x1.415e5bf6fb106p+4)) + ((R)0x1.0000000000000p+0)));
       return ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
     }
     else if constexpr (G == 3 && SHARED) {
       const R fdm_x0 = FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6))));
       const R fdm_q0 = fdm_x0 * fdm_x0;
-      ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
+      ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6))) == ((R)0.0) ? ((R)0.0) : ((fdm_q0 * ((R)0x1.5bf0a8b145769p+1)) - ((R)1.0))));
       ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
       return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     }
@@ -251,17 +256,17 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
       return (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
     }
     else if constexpr (G == 1 && !SHARED) {
-      ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5)))) - ((R)0x1.0000000000000p+0)));
       ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((((R)-0x1.c71c71c71c71cp-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
       return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     }
     else if constexpr (G == 2 && !SHARED) {
       ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((((R)-0x1.999999999999ap-5) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
-      ALGEBRAIC[6] = (((R)0x1.0000000000000p+0) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.6800000000000p+5)))) + ((R)0x1.0000000000000p+0)));
       return ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
     }
     else if constexpr (G == 3 && !SHARED) {
-      ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))) / (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
+      ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), (FDM_EXP((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.0400000000000p+6)))) - ((R)0x1.0000000000000p+0)));
       ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((((R)0x1.999999999999ap-7) * (STATES[0] + ((R)0x1.2c00000000000p+6)))));
       return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     }
@@ -272,6 +277,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_POW3
 #undef FDM_POW4
 #undef FDM_EXP
+#undef FDM_DIV
 #undef FDM_LOG
 #undef FDM_POWF
 #undef FDM_ABS
@@ -922,16 +928,16 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     const R t1 = (STATES[0] + ((R)50.0000));
     const R t2 = (t0 * t1);
     const R t3 = (((R)-0x1.999999999999ap-4) * STATES[0]);
-    const R t4 = M::exp(t3);
+    const R t4 = M::fast_exp(t3);
     const R t5 = (t4 * ((R)0x1.b993fe00d5376p-8));
     const R t6 = (t5 - ((R)1.00000));
-    const R t7 = (((R)1) / t6);
+    const R t7 = M::fast_rcp(t6);
     const R t8 = (t2 * t7);
     ALG[1] = t8;
     const R t9 = (STATES[0] + ((R)75.0000));
     const R t10 = (-t9);
     const R t11 = (t10 * ((R)0x1.c71c71c71c71cp-5));
-    const R t12 = M::exp(t11);
+    const R t12 = M::fast_exp(t11);
     const R t13 = (((R)4.00000) * t12);
     ALG[5] = t13;
     const R t14 = (((R)1.00000) - STATES[1]);
@@ -941,12 +947,12 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     const R t18 = (STATES[0] + ((R)75.0000));
     const R t19 = (-t18);
     const R t20 = (t19 * ((R)0x1.999999999999ap-5));
-    const R t21 = M::exp(t20);
+    const R t21 = M::fast_exp(t20);
     const R t22 = (((R)0.0700000) * t21);
     ALG[2] = t22;
     const R t23 = (t4 * ((R)0x1.6c0504695c417p-7));
     const R t24 = (t23 + ((R)1.00000));
-    const R t25 = (((R)1) / t24);
+    const R t25 = M::fast_rcp(t24);
     const R t26 = (((R)1.00000) * t25);
     ALG[6] = t26;
     const R t27 = (((R)1.00000) - STATES[2]);
@@ -958,12 +964,12 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     const R t33 = (t31 * t32);
     const R t34 = (t4 * ((R)0x1.8a1e18a954ffap-10));
     const R t35 = (t34 - ((R)1.00000));
-    const R t36 = (((R)1) / t35);
+    const R t36 = M::fast_rcp(t35);
     const R t37 = (t33 * t36);
     ALG[3] = t37;
     const R t38 = (STATES[0] + ((R)75.0000));
     const R t39 = (t38 * ((R)0x1.999999999999ap-7));
-    const R t40 = M::exp(t39);
+    const R t40 = M::fast_exp(t39);
     const R t41 = (((R)0.125000) * t40);
     ALG[7] = t41;
     const R t42 = (((R)1.00000) - STATES[3]);
@@ -1155,13 +1161,13 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[2] = t2;
     const R t3 = (((R)-0x1.999999999999ap-4) * STATES[0]);
     TAPE[3] = t3;
-    const R t4 = M::exp(t3);
+    const R t4 = M::fast_exp(t3);
     TAPE[4] = t4;
     const R t5 = (t4 * ((R)0x1.b993fe00d5376p-8));
     TAPE[5] = t5;
     const R t6 = (t5 - ((R)1.00000));
     TAPE[6] = t6;
-    const R t7 = (((R)1) / t6);
+    const R t7 = M::fast_rcp(t6);
     TAPE[7] = t7;
     const R t8 = (t2 * t7);
     TAPE[8] = t8;
@@ -1172,7 +1178,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[10] = t10;
     const R t11 = (t10 * ((R)0x1.c71c71c71c71cp-5));
     TAPE[11] = t11;
-    const R t12 = M::exp(t11);
+    const R t12 = M::fast_exp(t11);
     TAPE[12] = t12;
     const R t13 = (((R)4.00000) * t12);
     TAPE[13] = t13;
@@ -1191,7 +1197,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[19] = t19;
     const R t20 = (t19 * ((R)0x1.999999999999ap-5));
     TAPE[20] = t20;
-    const R t21 = M::exp(t20);
+    const R t21 = M::fast_exp(t20);
     TAPE[21] = t21;
     const R t22 = (((R)0.0700000) * t21);
     TAPE[22] = t22;
@@ -1200,7 +1206,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[23] = t23;
     const R t24 = (t23 + ((R)1.00000));
     TAPE[24] = t24;
-    const R t25 = (((R)1) / t24);
+    const R t25 = M::fast_rcp(t24);
     TAPE[25] = t25;
     const R t26 = (((R)1.00000) * t25);
     TAPE[26] = t26;
@@ -1223,7 +1229,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[34] = t34;
     const R t35 = (t34 - ((R)1.00000));
     TAPE[35] = t35;
-    const R t36 = (((R)1) / t35);
+    const R t36 = M::fast_rcp(t35);
     TAPE[36] = t36;
     const R t37 = (t33 * t36);
     TAPE[37] = t37;
@@ -1232,7 +1238,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     TAPE[38] = t38;
     const R t39 = (t38 * ((R)0x1.999999999999ap-7));
     TAPE[39] = t39;
-    const R t40 = M::exp(t39);
+    const R t40 = M::fast_exp(t39);
     TAPE[40] = t40;
     const R t41 = (((R)0.125000) * t40);
     TAPE[41] = t41;
