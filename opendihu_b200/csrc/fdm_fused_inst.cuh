@@ -84,7 +84,7 @@ static cudaError_t fused_shape(int shape, const FusedArgs& a, cudaStream_t s)
 template<class Model, class RR, class Math, int T, int M>
 static cudaError_t fused_cluster_one(const FusedArgs& a, int csize, cudaStream_t s)
 {
-  constexpr size_t smem = fused_smem_bytes<Model, RR, Math, T, M>();
+  constexpr size_t smem = fused_smem_bytes<Model, RR, Math, T, M, true>();
   auto kernel = fused_kernel<Model, RR, Math, T, M, false, true>;
   static std::atomic<uint64_t> attr_done{0};
   cudaError_t e = set_smem_once(kernel, smem, attr_done);
@@ -94,7 +94,7 @@ static cudaError_t fused_cluster_one(const FusedArgs& a, int csize, cudaStream_t
     return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.n_bins * csize), 1, 1);
-  cfg.blockDim = dim3(T, 1, 1);
+  cfg.blockDim = dim3(T + 64, 1, 1);   // with the halo warps
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

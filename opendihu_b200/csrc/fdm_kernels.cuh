@@ -1243,6 +1243,39 @@ __device__ __forceinline__ Affine block_scan_map(Affine acc, double* sF, double*
   return compose(wp, Affine{exF, exG});
 }
 
+// The value entering this thread's first node where the product of the F over any `span` (8, 16 or 32) consecutive threads
+// of a warp is negligible: the thread's own exclusive prefix over at least that many threads, and at the warp's start
+// the total of the warp before it in scan order (pos: this warp's position in that order, 0 the first; the lanes run in
+// the same direction).  sG: one slot per warp; one barrier.
+template<bool REVERSE>
+__device__ __forceinline__ double warp_chain_incoming(Affine acc, double* sG, int pos, int span)
+{
+  const int lane = threadIdx.x & 31;
+  auto level = [&](int off) {
+    const double F = REVERSE ? __shfl_down_sync(0xffffffffu, acc.F, off) : __shfl_up_sync(0xffffffffu, acc.F, off);
+    const double G = REVERSE ? __shfl_down_sync(0xffffffffu, acc.G, off) : __shfl_up_sync(0xffffffffu, acc.G, off);
+    if (REVERSE ? lane + off < 32 : lane >= off)
+      acc = compose(Affine{F, G}, acc);
+  };
+  level(1);
+  level(2);
+  level(4);
+  if (span > 8)
+    level(8);
+  if (span > 16)
+    level(16);
+  if (lane == (REVERSE ? 0 : 31))
+    sG[pos] = acc.G;
+  double F = REVERSE ? __shfl_down_sync(0xffffffffu, acc.F, 1) : __shfl_up_sync(0xffffffffu, acc.F, 1);
+  double G = REVERSE ? __shfl_down_sync(0xffffffffu, acc.G, 1) : __shfl_up_sync(0xffffffffu, acc.G, 1);
+  if (lane == (REVERSE ? 31 : 0)) {
+    F = 1.0;
+    G = 0.0;
+  }
+  __syncthreads();
+  return fma(F, pos > 0 ? sG[pos - 1] : 0.0, G);
+}
+
 // the value entering this thread's first node: the exclusive prefix map applied to the zero entering the
 // first node of the scan
 template<int T, bool REVERSE>
@@ -1408,32 +1441,46 @@ __global__ void __launch_bounds__(T) adjoint_diffusion_block_kernel(
 // GATE: onlyComputeIfHasBeenStimulated is on (a.gate is set); a separate instantiation so that the
 // default path carries none of its per-substep checks.
 // CLUSTER: for few fibers (the GPU would be mostly idle with one CTA per bin), one fiber per thread-block
-// cluster: CTA r of the cluster holds the fiber's nodes [r * T*M, (r+1) * T*M); the CTAs exchange the Vm of
-// their edge nodes and the totals of their scans through distributed shared memory, with three cluster
-// barriers per Strang step (every CTA of a cluster takes every barrier: no CTA returns early).
+// cluster: CTA r of the cluster holds the fiber's nodes [r * T*M, (r+1) * T*M) and, in two more warps that take no
+// part in the reaction, copies of the 32 M nodes left and right of them.  The solve's sweeps lose the value that
+// enters them by |mulF|, |cp| per node (about 0.1 for the usual steps), so sweeps started from 0 at the outer ends of
+// the halos are exact to rounding in the CTA's own nodes once the products over any warp's nodes are below
+// CHAIN_NEGLIGIBLE (a span is found at the start, over the whole cluster); then the CTAs exchange Vm through distributed shared
+// memory with one cluster barrier per Strang step, and within the CTA a warp needs the total of the warp before it
+// only.  Otherwise (large steps on fine meshes) the halos stay out of the scans, and the CTAs' scan totals
+// go through two more cluster barriers.  Every CTA of a cluster takes every barrier: no CTA returns early.
+// Bound by the latency of one node's Heun chain and of the exchange.  16 fibers of 1481 nodes, FP32, 8 CTAs of 192
+// nodes each: 6.93 us per Strang step with three cluster barriers and complete scans, 5.32 us so.
+constexpr double CHAIN_NEGLIGIBLE = 0x1p-70;   // times |Vm| <= 1e3 mV: below 1e-18 mV
+
 template<class Model, class RR, class Math, int T, int M, bool GATE, bool CLUSTER>
-__global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
+__global__ void __launch_bounds__(CLUSTER ? T + 64 : T, 1) fused_kernel(FusedArgs a)
 {
   constexpr int NS = Model::nStates;
   constexpr int NP = Model::nParameters > 0 ? Model::nParameters : 1;
-  constexpr int CAP = T * M;
+  constexpr int CAP = T * M;             // nodes of the CTA
+  constexpr int TT = CLUSTER ? T + 64 : T; // threads: with the halo warps
+  constexpr int SLOTS = TT * M;
+  constexpr int NWT = TT / 32;           // warps
   extern __shared__ double smem[];
-  // 5 x CAP coefficients: mulF, cp, and the right-hand side stencil l, m, r premultiplied by inv
+  // 5 x SLOTS coefficients: mulF, cp, and the right-hand side stencil l, m, r premultiplied by inv
   double* sc = smem;
-  double* vfirst = sc + 5 * CAP;     // T
-  double* vlast = vfirst + T;        // T
-  double* sF = vlast + T;            // 2 * (T/32) + 1
-  double* sG = sF + 2 * (T / 32) + 1; // 2 * (T/32) + 1
-  int* s_cf = (int*)(sG + 2 * (T / 32) + 1); // CAP: clamp fiber of each node (-1: not a junction node)
-  int* s_ts = s_cf + CAP;                // CAP: trace slot of each node (-1: not traced)
-  int* s_gate = s_ts + CAP;              // CAP: gate code of each node (onlyComputeIfHasBeenStimulated)
-  // paired FP32 path: the parameters of node pair p of thread tid, parameter k, at (p * NP + k) * T + tid
-  fdm_f2* sP2 = (fdm_f2*)(s_gate + CAP);
+  // Vm exchange: the first and last node of every thread (T each), or (cluster mode) all nodes, two sets in turn
+  double* vfirst = sc + 5 * SLOTS;
+  double* vlast = vfirst + (CLUSTER ? CAP : T);
+  double* sF = vlast + (CLUSTER ? CAP : T); // 2 * NWT + 1
+  double* sG = sF + 2 * NWT + 1;         // 2 * NWT + 1
+  int* s_cf = (int*)(sG + 2 * NWT + 1);  // SLOTS: clamp fiber of each node (-1: not a junction node)
+  int* s_ts = s_cf + SLOTS;              // SLOTS: trace slot of each node (-1: not traced)
+  int* s_gate = s_ts + SLOTS;            // SLOTS: gate code of each node (onlyComputeIfHasBeenStimulated)
+  // paired FP32 path: the parameters of node pair p of thread tid, parameter k, at (p * NP + k) * TT + tid
+  fdm_f2* sP2 = (fdm_f2*)(s_gate + SLOTS);
   __shared__ int64_t fib_global[FUSED_MAX_FIBERS_PER_BIN];
   __shared__ int fib_local[FUSED_MAX_FIBERS_PER_BIN + 1];
 
   __shared__ double ctot[4];      // cluster mode: this CTA's forward and backward scan totals (F, G)
   __shared__ double cpre[2 * 16]; // cluster mode: the other CTAs' totals this CTA composes
+  __shared__ int weak[2];         // the span the scans need (this CTA; cluster mode: the cluster)
   const int tid = threadIdx.x;
   int bin = blockIdx.x, crank = 0, csize = 1;
   if constexpr (CLUSTER) {
@@ -1449,6 +1496,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
   const int f0 = a.bin_fiber_start[bin];
   const int nf = CLUSTER ? 1 : a.bin_fiber_start[bin + 1] - f0;
   if (tid == 0) {
+    weak[0] = 0;
     if (CLUSTER) {
       const int fib = a.bin_fibers[f0];
       const int64_t len = a.fiber_offsets[fib + 1] - a.fiber_offsets[fib];
@@ -1516,20 +1564,35 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
     return fib_global[k] + (q - fib_local[k]);
   };
 
+  // cluster mode: halo warp of this thread (-1: none, 0: left, 1: right); its nodes' positions relative to the CTA's
+  // first node, and the fiber's extent in those positions
+  const int halo = CLUSTER && tid >= T ? (tid - T) >> 5 : -1;
+  auto position = [&](int t, int j) -> int {
+    if (!CLUSTER || t < T)
+      return t * M + j;
+    return t < T + 32 ? (t - T - 32) * M + j : CAP + (t - T - 32) * M + j;
+  };
+  int fiber_lo = 0, fiber_hi = nb;
+  if constexpr (CLUSTER) {
+    const int fib = a.bin_fibers[f0];
+    fiber_lo = -crank * CAP;
+    fiber_hi = fiber_lo + (int)(a.fiber_offsets[fib + 1] - a.fiber_offsets[fib]);
+  }
+
   // coefficients into shared memory (zero beyond the bin: those nodes carry x = 0); the forward sweep's
   // inv * d is formed as (inv l) u_{i-1} + (inv m) u_i + (inv r) u_{i+1}.  The per-node shared arrays hold
-  // node j of thread t (bin node t * M + j) at slot j * T + t: a warp's accesses to one j are consecutive
+  // node j of thread t (bin node t * M + j) at slot j * TT + t: a warp's accesses to one j are consecutive
   // words, free of bank conflicts
-  for (int sl = tid; sl < CAP; sl += T) {
-    const int q = (sl % T) * M + sl / T;
-    const bool ok = q < nb;
-    const int64_t g = ok ? global_node(q) : 0;
+  for (int sl = tid; sl < SLOTS; sl += TT) {
+    const int q = position(sl % TT, sl / TT);
+    const bool ok = CLUSTER ? q >= fiber_lo && q < fiber_hi : q < nb;
+    const int64_t g = ok ? (CLUSTER ? fib_global[0] + q : global_node(q)) : 0;
     const double inv = ok ? a.coef[1 * a.stride + g] : 0.0;
-    sc[0 * CAP + sl] = ok ? a.coef[0 * a.stride + g] : 0.0;
-    sc[1 * CAP + sl] = ok ? a.coef[2 * a.stride + g] : 0.0;
+    sc[0 * SLOTS + sl] = ok ? a.coef[0 * a.stride + g] : 0.0;
+    sc[1 * SLOTS + sl] = ok ? a.coef[2 * a.stride + g] : 0.0;
 #pragma unroll
     for (int k = 3; k < 6; k++)
-      sc[(k - 1) * CAP + sl] = ok ? inv * a.coef[k * a.stride + g] : 0.0;
+      sc[(k - 1) * SLOTS + sl] = ok ? inv * a.coef[k * a.stride + g] : 0.0;
   }
 
   const RR* pr = (const RR*)a.params;
@@ -1555,10 +1618,10 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
     for (int p = 0; p < Model::nParameters; p++)
       P[j][p] = ok ? pr[p * a.stride + i] : (RR)0;
     const int cfj = ok ? a.clamp_fiber[i] : -1;
-    s_cf[j * T + tid] = cfj;
+    s_cf[j * TT + tid] = cfj;
     cmask |= (cfj >= 0 ? 1u : 0u) << j;
-    s_ts[j * T + tid] = (ok && a.trace_slot) ? a.trace_slot[i] : -1;
-    s_gate[j * T + tid] = (ok && a.gate) ? a.gate[i] : 0;
+    s_ts[j * TT + tid] = (ok && a.trace_slot) ? a.trace_slot[i] : -1;
+    s_gate[j * TT + tid] = (ok && a.gate) ? a.gate[i] : 0;
   }
   // the clamp fiber of the thread's junction nodes when they all belong to one fiber (the usual case: a
   // junction is a few consecutive nodes of one fiber): one flag read per substep instead of one per node
@@ -1567,14 +1630,14 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
 #pragma unroll
   for (int j = 0; j < M; j++) {
     if ((cmask >> j) & 1u) {
-      const int c = s_cf[j * T + tid];
+      const int c = s_cf[j * TT + tid];
       cf_one = cf_one && (cf_first < 0 || c == cf_first);
       cf_first = cf_first < 0 ? c : cf_first;
     }
   }
   // stimulation bit of node j at substep bit `bit` (junction nodes only read their fiber's bit)
   auto node_stim = [&](int j, int bit) -> bool {
-    return ((cmask >> j) & 1u) && stim_bit(a.flags, a.words_per_fiber, s_cf[j * T + tid], bit);
+    return ((cmask >> j) & 1u) && stim_bit(a.flags, a.words_per_fiber, s_cf[j * TT + tid], bit);
   };
   // FP32 exact-exponential reaction: nodes (2p, 2p+1) advance together in packed FP32 (heun_step2);
   // an odd last node runs alone
@@ -1593,7 +1656,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
       }
 #pragma unroll
       for (int q = 0; q < NP; q++)
-        sP2[(p * NP + q) * T + tid] = fdm_f2((float)P[2 * p][q], (float)P[2 * p + 1][q]);
+        sP2[(p * NP + q) * TT + tid] = fdm_f2((float)P[2 * p][q], (float)P[2 * p + 1][q]);
     }
   }
   // the scalar state of node j (from the pair arrays where node j is paired)
@@ -1615,7 +1678,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
         }
 #pragma unroll
         for (int q = 0; q < NP; q++)
-          Pj[q] = (RR)((j & 1) ? sP2[((j >> 1) * NP + q) * T + tid].v.y : sP2[((j >> 1) * NP + q) * T + tid].v.x);
+          Pj[q] = (RR)((j & 1) ? sP2[((j >> 1) * NP + q) * TT + tid].v.y : sP2[((j >> 1) * NP + q) * TT + tid].v.x);
       }
     }
   };
@@ -1655,6 +1718,45 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
     }
   };
   __syncthreads();
+  // The sweeps' scans need no more than `span` threads of a warp (and its neighbour's total) once the products of |mulF|
+  // and of |cp| over that many consecutive threads are negligible: the smallest of 8, 16, 32 for which they are in every
+  // warp (of the cluster); 0 if not even a whole warp's are, then the scans are complete.  (4096 uneven fibers, FP32, bins,
+  // 150 steps: 39.4 -> 38.6 ms with a span of 8.)
+  int span = 0;
+  {
+    double F = 1.0, B = 1.0;
+#pragma unroll
+    for (int j = 0; j < M; j++) {
+      F *= fabs(sc[0 * SLOTS + j * TT + tid]);
+      B *= fabs(sc[1 * SLOTS + j * TT + tid]);
+    }
+    double w = fmax(F, B);   // over the 2 off threads that end at this lane (fewer at the warp's start, where a prefix
+    int need = 0;            // is complete); need: 8, 16, 32, or 64 (not even 32)
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const double before = __shfl_up_sync(0xffffffffu, w, off);
+      if ((tid & 31) >= off)
+        w *= before;
+      if (off >= 4 && need == 0 && __all_sync(0xffffffffu, (tid & 31) < 2 * off - 1 || w <= CHAIN_NEGLIGIBLE))
+        need = 2 * off;
+    }
+    if (need == 0)
+      need = 64;
+    if ((tid & 31) == 0)
+      atomicMax(&weak[0], need);
+    cluster_sync();
+    if constexpr (CLUSTER) {
+      if (tid == 0) {
+        int all = 0;
+        for (int k = 0; k < csize; k++)
+          all = max(all, cg::this_cluster().map_shared_rank(weak, k)[0]);
+        weak[1] = all;
+      }
+      __syncthreads();
+    }
+    span = weak[CLUSTER ? 1 : 0];
+    span = span > 32 ? 0 : span;
+  }
 
   for (int step = 0; step < a.n_steps; step++) {
     const SplitStep s = a.steps[step];
@@ -1674,7 +1776,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
       if constexpr (gate_on) {
 #pragma unroll
         for (int j = 0; j < M; j++)
-          gfirst[j >> 2] |= (unsigned)gate_first(a.gate_start, a.gate_stride, s_gate[j * T + tid], step * 2 + half)
+          gfirst[j >> 2] |= (unsigned)gate_first(a.gate_start, a.gate_stride, s_gate[j * TT + tid], step * 2 + half)
                             << (8 * (j & 3));
       }
       auto node_on = [&](int j, int k) -> bool { return k >= (int)((gfirst[j >> 2] >> (8 * (j & 3))) & 0xffu); };
@@ -1688,7 +1790,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
         }
       }
 #pragma unroll 1
-      for (int k = 0; k < k_end; k++) {
+      for (int k = 0; k < (halo < 0 ? k_end : 0); k++) {
         const double t = xadd(t0, xmul((double)k, s.dt0));
         if constexpr (gate_on) {
           // a substep that no node of the warp computes is skipped by the whole warp
@@ -1720,7 +1822,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
           for (int p = 0; p < MP; p++)
 #pragma unroll
             for (int q = 0; q < NP; q++)
-              Pk[p][q] = sP2[(p * NP + q) * T + tid];
+              Pk[p][q] = sP2[(p * NP + q) * TT + tid];
           if (__any_sync(0xffffffffu, (clamp & pair_mask) != 0u)) {
             const bool m1 = a.stimulus_mode == 1;
             const float sv = (float)a.stimulus_value;
@@ -1764,7 +1866,7 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
             fdm_f2 Pp[NP];
 #pragma unroll
             for (int q = 0; q < NP; q++)
-              Pp[q] = sP2[(p * NP + q) * T + tid];
+              Pp[q] = sP2[(p * NP + q) * TT + tid];
             if ((stim0 || stim1) && a.stimulus_mode == 1) {
               fdm_f2 Pk[NP];
               const float sv = (float)a.stimulus_value;
@@ -1841,68 +1943,106 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
         break;
 
       // ---- diffusion: block-wide tridiagonal solve in FP64 ----
-      vfirst[tid] = V[0];
-      vlast[tid] = V[M - 1];
-      cluster_sync();
-      double vprev = tid > 0 ? vlast[tid - 1] : 0.0;
-      double vnext = tid < T - 1 ? vfirst[tid + 1] : 0.0;
+      double vprev, vnext;
       if constexpr (CLUSTER) {
+        // publish the CTA's Vm; the set written two steps ago is read by no one after the last step's barrier
+        double* pub = step & 1 ? vlast : vfirst;
+        if (halo < 0) {
+#pragma unroll
+          for (int j = 0; j < M; j++)
+            pub[tid * M + j] = V[j];
+        }
+        cluster_sync();
         cg::cluster_group cl = cg::this_cluster();
-        if (tid == 0 && crank > 0)
-          vprev = cl.map_shared_rank(vlast, crank - 1)[T - 1];
-        if (tid == T - 1 && crank < csize - 1)
-          vnext = cl.map_shared_rank(vfirst, crank + 1)[0];
+        const double* left = crank > 0 ? cl.map_shared_rank(pub, crank - 1) : nullptr;
+        const double* right = crank < csize - 1 ? cl.map_shared_rank(pub, crank + 1) : nullptr;
+        // Vm at position q relative to the CTA's first node (the CTAs beside it: one halo warp's reach)
+        auto at = [&](int q) -> double {
+          if (q < 0)
+            return left && q >= -CAP ? left[CAP + q] : 0.0;
+          if (q >= CAP)
+            return right && q < 2 * CAP ? right[q - CAP] : 0.0;
+          return pub[q];
+        };
+        if (halo >= 0) {
+#pragma unroll
+          for (int j = 0; j < M; j++)
+            V[j] = at(position(tid, j));
+        }
+        vprev = at(position(tid, 0) - 1);
+        vnext = at(position(tid, M - 1) + 1);
+      } else {
+        vfirst[tid] = V[0];
+        vlast[tid] = V[M - 1];
+        __syncthreads();
+        vprev = tid > 0 ? vlast[tid - 1] : 0.0;
+        vnext = tid < T - 1 ? vfirst[tid + 1] : 0.0;
       }
       double d[M];
 #pragma unroll
       for (int j = 0; j < M; j++) {
-        const int q = j * T + tid;
+        const int q = j * TT + tid;
         const double um = j > 0 ? V[j - 1] : vprev;
         const double up = j < M - 1 ? V[j + 1] : vnext;
-        d[j] = sc[2 * CAP + q] * um + sc[3 * CAP + q] * V[j] + sc[4 * CAP + q] * up;
+        d[j] = sc[2 * SLOTS + q] * um + sc[3 * SLOTS + q] * V[j] + sc[4 * SLOTS + q] * up;
       }
+      // without a span the halo warps are the identity in the scans
+      const bool idle = CLUSTER && !span && halo >= 0;
       Affine acc{1.0, 0.0};
 #pragma unroll
       for (int j = 0; j < M; j++) {
-        const int q = j * T + tid;
-        acc = compose(acc, Affine{sc[0 * CAP + q], d[j]});
+        const int q = j * TT + tid;
+        if (!idle)
+          acc = compose(acc, Affine{sc[0 * SLOTS + q], d[j]});
       }
-      Affine tot_f;
-      // one barrier per scan (block_scan_map), the forward and backward warp totals in separate halves of sF/sG
-      const Affine ex_f = block_scan_map<T, false>(acc, sF, sG, &tot_f);
-      double dp = cluster_incoming(ex_f, tot_f, false);
+      double dp;
+      const int warp_pos = CLUSTER ? (halo == 0 ? 0 : (halo == 1 ? NWT - 1 : 1 + (tid >> 5))) : tid >> 5;
+      if (span) {
+        dp = warp_chain_incoming<false>(acc, sG, warp_pos, span);
+      } else {
+        Affine tot_f;
+        // one barrier per scan (block_scan_map), the forward and backward warp totals in separate halves of sF/sG
+        const Affine ex_f = block_scan_map<T, false>(acc, sF, sG, &tot_f);
+        dp = cluster_incoming(ex_f, tot_f, false);
+      }
 #pragma unroll
       for (int j = 0; j < M; j++) {
-        const int q = j * T + tid;
-        dp = sc[0 * CAP + q] * dp + d[j];
+        const int q = j * TT + tid;
+        dp = sc[0 * SLOTS + q] * dp + d[j];
         d[j] = dp;
       }
       Affine bacc{1.0, 0.0};
 #pragma unroll
       for (int j = M - 1; j >= 0; j--) {
-        const int q = j * T + tid;
-        bacc = compose(bacc, Affine{-sc[1 * CAP + q], d[j]});
+        const int q = j * TT + tid;
+        if (!idle)
+          bacc = compose(bacc, Affine{-sc[1 * SLOTS + q], d[j]});
       }
       // No barrier is needed before the backward scan: its warp totals go to the other half of sF/sG (the
       // forward totals may still be read).  In cluster mode the backward scan's CTA totals take other slots of
       // ctot, and cpre is rewritten only after the backward cluster barrier, which every forward read precedes.
-      Affine tot_b;
-      const Affine ex_b = block_scan_map<T, true>(bacc, sF + T / 32, sG + T / 32, &tot_b);
-      double x = cluster_incoming(ex_b, tot_b, true);
+      double x;
+      if (span) {
+        x = warp_chain_incoming<true>(bacc, sG + NWT, NWT - 1 - warp_pos, span);
+      } else {
+        Affine tot_b;
+        const Affine ex_b = block_scan_map<T, true>(bacc, sF + NWT, sG + NWT, &tot_b);
+        x = cluster_incoming(ex_b, tot_b, true);
+      }
 #pragma unroll
       for (int j = M - 1; j >= 0; j--) {
-        const int q = j * T + tid;
-        x = -sc[1 * CAP + q] * x + d[j];
+        const int q = j * TT + tid;
+        x = -sc[1 * SLOTS + q] * x + d[j];
         V[j] = x;
       }
-      // the next writes of vfirst/vlast, sF/sG and ctot come after the next diffusion's first (cluster)
-      // barrier, or after this one's backward cluster barrier, which every read of this one precedes
+      // the next writes of vfirst/vlast (cluster mode: of this step's set), sF/sG and ctot come after the next
+      // diffusion's first (cluster) barrier, or after this one's last barrier, which every read of this one precedes
     }
     if (a.trace_slot) {
 #pragma unroll
       for (int j = 0; j < M; j++)
-        if (s_ts[j * T + tid] >= 0)
-          record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, s_ts[j * T + tid], s.global_no, V[j]);
+        if (s_ts[j * TT + tid] >= 0)
+          record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, s_ts[j * TT + tid], s.global_no, V[j]);
     }
   }
 
@@ -1937,13 +2077,14 @@ __global__ void __launch_bounds__(T, 1) fused_kernel(FusedArgs a)
   }
 }
 
-template<class Model, class RR, class Math, int T, int M>
+template<class Model, class RR, class Math, int T, int M, bool CLUSTER = false>
 constexpr size_t fused_smem_bytes()
 {
   constexpr bool PAIR = std::is_same<RR, float>::value && std::is_same<Math, fdm_math_exact>::value;
   constexpr int NP = Model::nParameters > 0 ? Model::nParameters : 1;
-  return sizeof(double) * (5 * T * M + 2 * T + 4 * (T / 32) + 2) + sizeof(int) * 3 * T * M +
-         (PAIR ? sizeof(fdm_f2) * (M / 2) * NP * T : 0);
+  constexpr int TT = CLUSTER ? T + 64 : T;
+  return sizeof(double) * (5 * TT * M + 2 * (CLUSTER ? T * M : T) + 4 * (TT / 32) + 2) + sizeof(int) * 3 * TT * M +
+         (PAIR ? sizeof(fdm_f2) * (M / 2) * NP * TT : 0);
 }
 
 } // namespace fdm

@@ -124,3 +124,26 @@ def test_equilibrium_lane_widths(width, scale):
     assert np.max(np.abs(st - ref)) < 1e-8
     np.testing.assert_array_equal(status, ref_status)
     np.testing.assert_array_equal(counter, ref_counter)
+
+
+# fused, a fiber over the CTAs of a cluster: with the usual step the halos carry the sweeps across the CTAs, with a step
+# of 0.1 ms (0.75 per node and sweep) they cannot and the scan totals are exchanged; fibers that end inside a CTA, at
+# its end and inside a neighbour's halo
+@pytest.mark.parametrize("dt", [1e-3, 0.1])
+@pytest.mark.parametrize("threads,per_thread", [(128, 2), (192, 1)])
+def test_cluster_halos(dt, threads, per_thread):
+    cap = threads * per_thread
+    s = S.uniform_fibers(H.HH, [cap * 3, cap * 2, cap * 2 + 1, cap + 5, cap - 1, 2], 0.01, 3.828 / 500,
+                         call_frequency=0.1, repeat_after_first_call=0.1, call_enable_begin=0.0, end_time=4 * dt,
+                         dt_0d=dt / 10, dt_1d=dt, dt_splitting=dt, dt_repeated_call=dt, clamp_rule="center",
+                         diffusion_scheme="CrankNicolson")
+    s = H.complete(s)
+    s.states = s.states.copy()
+    s.states[0] += np.random.default_rng(2).uniform(0.0, 40.0, s.n_nodes)
+    ref = H.run_oracle(s.copy())[0]
+    for precision, tol in (("fp64", (1e-8, 1e-8)), ("fp32", (0.1, 1e-3))):   # FP32: the mode's accuracy contract
+        with S.FastMonodomainSolver(s.copy(), method="fused", precision=precision, threads_per_block=threads,
+                                    nodes_per_thread=per_thread, cluster_size=3, steps_per_launch=3) as slv:
+            slv.advanceTimeSpan()
+            got = slv.states()
+        assert np.max(np.abs(got[0] - ref[0])) < tol[0] and np.max(np.abs(got[1:] - ref[1:])) < tol[1]
