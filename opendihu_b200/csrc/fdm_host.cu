@@ -231,6 +231,7 @@ struct fdm_solver {
   struct Adjoint {
     bool ready = false;
     int kc = 0, n_seg = 0, n_sensors = 0, n0max = 1;
+    int64_t n_nodes = 0;
     std::vector<SplitStep> steps;
     std::vector<double> dt1s;
     DevBuf<double> ck_vm, ck_states, ck_last, ck_jit, fin_vm, fin_states, fin_last, fin_jit;
@@ -3257,11 +3258,21 @@ extern "C" int fdm_adjoint_forward(fdm_solver* s, double t_start, double t_end, 
   if (s->n_fibers == 0 || !s->stimulation_set)
     return fail(s, FDM_ERR_ARG, "fdm_adjoint_forward: set fibers and stimulation first");
   auto& A = s->adj;
-  A.release();
+  const std::vector<SplitStep> last_steps = std::move(A.steps);
+  const int last_kc = A.kc;
+  A.ready = false;
   A.steps.clear();
   A.dt1s.clear();
   plan_advance(s, t_start, t_end, A.steps, A.dt1s);
   const int64_t NT = (int64_t)A.steps.size();
+  // A run of the last run's shape (an optimization loop) keeps its checkpoints and tapes: freeing and allocating the
+  // several GB of them took 10 of 26 ms (64 x 1481 fibers, 100 steps).  Any other shape starts from nothing, so no more is held than it needs.
+  bool same = A.kc > 0 && last_kc == checkpoint_every && last_steps.size() == A.steps.size();
+  for (size_t j = 0; same && j < A.steps.size(); j++)
+    same = last_steps[j].n0 == A.steps[j].n0;
+  if (!same || A.n_nodes != s->n_nodes)
+    A.release();
+  A.n_nodes = s->n_nodes;
   for (int64_t j = 0; j < NT; j++)
     A.steps[j].global_no = (int)j; // trace rows of this run
   int rc = fdm_set_trace(s, n_sensors, sensor_nodes, NT);
