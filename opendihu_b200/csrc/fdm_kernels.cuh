@@ -989,6 +989,9 @@ __global__ void __launch_bounds__(128) adjoint_diffusion_warp_kernel(
 struct AdjointArgs {
   int64_t n_nodes;
   const double* states;           // stored substep input states of this half step: [(k*nS + s)*N + node]
+  int n_halves;                   // 2 (half == 0): the second half step of the split step before, `before`, is reversed
+  SplitStep before;               // in the same launch; its stored states lie half_stride doubles before `states`, its
+  int64_t half_stride;            // trace row and index in the window are one less
   const double* params;           // [p][node]
   double* lam;                    // adjoint of the state [s][node], in/out
   double* grad_params;            // [p][node], accumulated
@@ -1079,88 +1082,92 @@ __global__ void __launch_bounds__(128, 3) adjoint_half_kernel(AdjointArgs a)
     P[q] = a.params[q * N + i];
     gP[q] = 0.0;
   }
-  if (a.half == 1 && a.trace_slot && a.trace_row >= 0) {
-    const int slot = a.trace_slot[i];
-    if (slot >= 0)
-      lam[0] += a.trace_grad[a.trace_row * a.n_trace + slot];
-  }
   const int cf = a.clamp_fiber[i];
-  const SplitStep st = a.step;
-  const double t0 = a.half ? st.mid : st.t;
-  const int base = (a.step_in_window * 2 + a.half) * a.nsub_stride;
-  const double dt = st.dt0;
-  const int first = a.gate ? gate_first(a.gate_start, a.gate_stride, a.gate[i], a.step_in_window * 2 + a.half) : 0;
-  double ynext[PREFETCH ? NS : 1];
-  if (PREFETCH && st.n0 > 0) {
-#pragma unroll
-    for (int s = 0; s < NS; s++)
-      ynext[s] = a.states[(int64_t)((st.n0 - 1) * NS + s) * N + i];
-  }
-  for (int k = st.n0 - 1; k >= 0; k--) {
-    const double t = xadd(t0, xmul((double)k, dt));
-    const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
-    const bool clamp = stim && a.stimulus_mode == 0;
-    double Pk[NP];
-#pragma unroll
-    for (int q = 0; q < NP; q++)
-      Pk[q] = (stim && a.stimulus_mode == 1 && q == a.stimulus_parameter) ? a.stimulus_value : P[q];
-    double y[NS], r[NS], ys[NS];
-    if (PREFETCH) {
+  const int slot = a.trace_slot ? a.trace_slot[i] : -1;
+#pragma unroll 1
+  for (int hh = 0; hh < a.n_halves; hh++) {
+    const int hs = a.step_in_window * 2 + a.half - hh; // half step of the window
+    const SplitStep st = hh ? a.before : a.step;
+    const double* __restrict__ states = a.states - hh * a.half_stride;
+    if ((hs & 1) && slot >= 0)
+      lam[0] += a.trace_grad[(a.trace_row - hh) * a.n_trace + slot];
+    const double t0 = (hs & 1) ? st.mid : st.t;
+    const int base = hs * a.nsub_stride;
+    const double dt = st.dt0;
+    const int first = a.gate ? gate_first(a.gate_start, a.gate_stride, a.gate[i], hs) : 0;
+    double ynext[PREFETCH ? NS : 1];
+    if (PREFETCH && st.n0 > 0) {
 #pragma unroll
       for (int s = 0; s < NS; s++)
-        y[s] = ynext[s];
-      if (k > 0) {
+        ynext[s] = states[(int64_t)((st.n0 - 1) * NS + s) * N + i];
+    }
+#pragma unroll 1
+    for (int k = st.n0 - 1; k >= 0; k--) {
+      const double t = xadd(t0, xmul((double)k, dt));
+      const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
+      const bool clamp = stim && a.stimulus_mode == 0;
+      double Pk[NP];
+#pragma unroll
+      for (int q = 0; q < NP; q++)
+        Pk[q] = (stim && a.stimulus_mode == 1 && q == a.stimulus_parameter) ? a.stimulus_value : P[q];
+      double y[NS], r[NS], ys[NS];
+      if (PREFETCH) {
 #pragma unroll
         for (int s = 0; s < NS; s++)
-          ynext[s] = a.states[(int64_t)((k - 1) * NS + s) * N + i];
+          y[s] = ynext[s];
+        if (k > 0) {
+#pragma unroll
+          for (int s = 0; s < NS; s++)
+            ynext[s] = states[(int64_t)((k - 1) * NS + s) * N + i];
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+          y[s] = states[(int64_t)(k * NS + s) * N + i];
       }
-    } else {
+      if (k < first)
+        continue; // the forward substep was skipped: its reverse is the identity
+      constexpr bool TAPE_OK = F::nTape <= 256;
+      double tape[TAPE_OK ? F::nTape : 1];
+      if (TAPE_OK && a.use_tape) {
+        F::tape(t, y, Pk, r, tape);
+      } else {
+        double alg[Model::nAlgebraics];
+        Model::template rates<double, Math>(t, y, Pk, r, alg);
+      }
 #pragma unroll
       for (int s = 0; s < NS; s++)
-        y[s] = a.states[(int64_t)(k * NS + s) * N + i];
-    }
-    if (k < first)
-      continue; // the forward substep was skipped: its reverse is the identity
-    constexpr bool TAPE_OK = F::nTape <= 256;
-    double tape[TAPE_OK ? F::nTape : 1];
-    if (TAPE_OK && a.use_tape) {
-      F::tape(t, y, Pk, r, tape);
-    } else {
-      double alg[Model::nAlgebraics];
-      Model::template rates<double, Math>(t, y, Pk, r, alg);
-    }
+        ys[s] = y[s] + dt * r[s];
+      if (clamp) {
+        ys[0] = a.vstim;
+        lam[0] = 0.0;
+      }
+      double lr2[NS], lys[NS], lr[NS], gPk[NP];
 #pragma unroll
-    for (int s = 0; s < NS; s++)
-      ys[s] = y[s] + dt * r[s];
-    if (clamp) {
-      ys[0] = a.vstim;
-      lam[0] = 0.0;
+      for (int s = 0; s < NS; s++) {
+        lr2[s] = 0.5 * dt * lam[s];
+        lys[s] = 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < NP; q++)
+        gPk[q] = 0.0;
+      F::vjp(t, ys, Pk, lr2, lys, gPk);
+      if (clamp)
+        lys[0] = 0.0;
+#pragma unroll
+      for (int s = 0; s < NS; s++) {
+        lr[s] = 0.5 * dt * lam[s] + dt * lys[s];
+        lam[s] = lam[s] + lys[s];
+      }
+      if (TAPE_OK && a.use_tape)
+        F::vjp_tape(t, y, Pk, tape, lr, lam, gPk);
+      else
+        F::vjp(t, y, Pk, lr, lam, gPk);
+#pragma unroll
+      for (int q = 0; q < Model::nParameters; q++)
+        if (!(stim && a.stimulus_mode == 1 && q == a.stimulus_parameter))
+          gP[q] += gPk[q];
     }
-    double lr2[NS], lys[NS], lr[NS], gPk[NP];
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-      lr2[s] = 0.5 * dt * lam[s];
-      lys[s] = 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < NP; q++)
-      gPk[q] = 0.0;
-    F::vjp(t, ys, Pk, lr2, lys, gPk);
-    if (clamp)
-      lys[0] = 0.0;
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-      lr[s] = 0.5 * dt * lam[s] + dt * lys[s];
-      lam[s] = lam[s] + lys[s];
-    }
-    if (TAPE_OK && a.use_tape)
-      F::vjp_tape(t, y, Pk, tape, lr, lam, gPk);
-    else
-      F::vjp(t, y, Pk, lr, lam, gPk);
-#pragma unroll
-    for (int q = 0; q < Model::nParameters; q++)
-      if (!(stim && a.stimulus_mode == 1 && q == a.stimulus_parameter))
-        gP[q] += gPk[q];
   }
 #pragma unroll
   for (int s = 0; s < NS; s++)
