@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(EMG_T, 4) cg_direction_kernel(Grid g, const do
 // With a node per thread and no tiles (mg_jacobi_kernel and so on) every coefficient comes from L2 twice, once
 // for each end of its edge, 312 B per node, which bounds those; here 195 B, of which 144 B are from HBM.  On 97 x 97 x 297
 // nodes a direction pass takes 115 us against 146 (0.56 of the measured copy rate), a V-cycle's passes over the two
-// finest levels 452 against 600.
+// finest levels 457 against 593.
 constexpr int ST_T = 352;              // threads: (tx + 2) (ty + 2) <= ST_T
 constexpr int64_t ST_MIN_NODES = 100000;
 enum StencilOp { ST_RESIDUAL, ST_JACOBI, ST_DIRECTION };
