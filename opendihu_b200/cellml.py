@@ -638,6 +638,41 @@ def _exp_groups(lines, consts):
     return repl, groups
 
 
+def _squared_groups(lines, consts, groups):
+    """Groups of _exp_groups whose exponential is the square of one exponential outside them, at half their slope:
+    {group: (exp node, its constant term, the positive constant it is multiplied with in the model or 1)}"""
+    found = []
+
+    def walk(e, factor=1.0):
+        t = e[0]
+        if t == "call":
+            if e[1] == "exp":
+                af = _affine(e[2][0], consts)
+                if af is not None and af[0]:
+                    found.append((e, af, factor))
+            for a in e[2]:
+                walk(a)
+        elif t in ("neg", "pos", "not"):
+            walk(e[1])
+        elif t == "bin":
+            for x, other in ((e[2], e[3]), (e[3], e[2])):
+                c = _affine(other, consts) if e[1] == "*" else None
+                walk(x, c[1] if c is not None and not c[0] and c[1] > 0.0 else 1.0)
+        elif t == "tern":
+            for x in e[1:4]:
+                walk(x)
+    for _, _, e in lines:
+        walk(e)
+    out = {}
+    for g, key in enumerate(groups):
+        for e, af, factor in found:
+            half = tuple(sorted(af[0].items()))
+            if len(half) == len(key) and all(k == k2 and abs(v - 2 * v2) <= 4e-15 * abs(v)
+                                             for (k, v), (k2, v2) in zip(key, half)):
+                out.setdefault(g, (e, af[1], factor))
+    return out
+
+
 _LOG2E = 1.4426950408889634
 _LN2 = 0.6931471805599453
 
@@ -726,9 +761,13 @@ class _FastEmitter(_Emitter):
         denominators free of algebraic variables share one SFU reciprocal per group of up to three
         (fdm_rcp_batch: 1/d_k from 1/(d_0 d_1 d_2) and the other factors)."""
 
-    def __init__(self, real, consts, repl, paired: bool = False, recip=None, alg_defs=None):
+    def __init__(self, real, consts, repl, paired: bool = False, recip=None, alg_defs=None, squares=None):
         super().__init__(real, consts, "cuda")
         self.repl = repl
+        # paired form: group -> (exp node of half its slope, that node's constant term, constant factor it has in the
+        # model): fdm_h<group> = factor exp(node), and the group's exponential is its square over factor^2 e^(2 b)
+        self.squares = squares or {}
+
         self.paired = paired        # fdm_f2 operands: conditional expressions become per-component selects
         self.recip = recip or {}    # repr(denominator) -> name of its batched reciprocal
         # paired form: definitions of the algebraic variables (index -> expression), for _folded_subtrahend
@@ -780,8 +819,14 @@ class _FastEmitter(_Emitter):
 
     def exp_text(self, e, factor: float = 1.0):
         """factor * exp(arg) for the exp call node e (factor > 0)"""
+        for g, (node, _, f) in self.squares.items():
+            if repr(e) == repr(node):
+                return f"fdm_h{g}" if factor == f else f"(fdm_h{g} * (({self.real}){_hexf(factor / f)}))"
         if repr(e) in self.repl:
             g, b = self.repl[repr(e)]
+            if g in self.squares:
+                _, b_half, f = self.squares[g]
+                b, factor = b - 2 * b_half, factor / (f * f)
             return f"(fdm_e{g} * (({self.real}){_hexf(math.exp(b) * factor)}))"
         af = _affine(e[2][0], self.consts)
         if af is not None:
@@ -863,6 +908,20 @@ class _FastEmitter(_Emitter):
         if t == "bin" and e[1] == "-":
             return f"({self.neg_text(e[2])} + {self.expr(e[3])})"
         return f"(-{self.expr(e)})"
+
+    def group_lines(self, groups):
+        """Declarations of the shared exponentials"""
+        out = []
+        for g, key in enumerate(groups):
+            if g in self.squares:
+                node, _, f = self.squares[g]
+                af = _affine(node[2][0], self.consts)
+                arg = self.affine_text(sorted(af[0].items()), af[1] + math.log(f), _LOG2E)
+                out.append(f"    const R fdm_h{g} = fdm_ex2({arg});")
+                out.append(f"    const R fdm_e{g} = fdm_h{g} * fdm_h{g};")
+            else:
+                out.append(f"    const R fdm_e{g} = fdm_ex2({self.affine_text(list(key), 0.0, _LOG2E)});")
+        return out
 
     def batch_lines(self, groups):
         """Declarations of the batched reciprocals (after the shared exponentials); fills self.recip."""
@@ -1145,7 +1204,8 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
     out.append("  }")
     # the same FP32 form over node pairs (packed FP32 instructions)
     fem2 = _FastEmitter("R", model.constants, repl, paired=True,
-                        alg_defs={idx: expr for kind, idx, expr in lines if kind == "A"})
+                        alg_defs={idx: expr for kind, idx, expr in lines if kind == "A"},
+                        squares=_squared_groups(lines, model.constants, groups))
     out.append("  // paired FP32 form: the FP32 form over two nodes at once (fdm_f2, packed FP32 instructions)")
     out.append("  template<class M>")
     out.append("  __device__ __forceinline__ static void rates_fast2(const fdm_f2 VOI, const fdm_f2* __restrict__ STATES,"
@@ -1157,8 +1217,7 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
     out.append("#define FDM_ABS(x) fabs(x)")
     out.append("#define FDM_SQRT(x) sqrt(x)")
     out.extend("#define " + s2.split("#define ", 1)[1] for s2 in _pow_macro_defs(pows))
-    for g, key in enumerate(groups):
-        out.append(f"    const R fdm_e{g} = fdm_ex2({fem2.affine_text(list(key), 0.0, _LOG2E)});")
+    out.extend(fem2.group_lines(groups))
     out.extend(fem2.batch_lines(rgroups))
     for kind, idx, expr in lines:
         tgt = f"ALGEBRAIC[{idx}]" if kind == "A" else f"RATES[{idx}]"

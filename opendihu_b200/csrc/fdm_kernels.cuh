@@ -395,8 +395,12 @@ __device__ __forceinline__ void heun_step2(fdm_f2& Vf, fdm_f2& LV, double& V0, d
 
 // heun_step2 over the MP node pairs of one thread, without branches: every pair computes (the caller zeroes
 // the Vm of nodes beyond its bin), clamps are selects (bit 2p / 2p + 1 of `clamp`: node 2p / 2p + 1 clamped;
-// a constant 0 removes them).  Arithmetic per pair identical to heun_step2.  (Issuing the pairs' first
-// right-hand sides before their second ones measured 0.7 % slower than pair after pair.)
+// a constant 0 removes them).  The scheme per pair is heun_step2's; the two rates are added to the half-step
+// residual one after the other, the first before the second right-hand side.  Issue-bound, so instructions count: this
+// and the generated pair form's exp(-V/10) as the square of the half-slope exponential that the model has anyway
+// (a special-function instruction less per node and right-hand side) take 4096 fibers of 500 to 2500 nodes from 46.2 to
+// 45.5 ms per 150 steps, and the error against 64-bit arithmetic from 3.4e-7 to 1.6e-7.  (Issuing the pairs'
+// first right-hand sides before their second ones measured 0.7 % slower than pair after pair.)
 template<class Model, int MP, int NSM, int NP>
 __device__ __forceinline__ void heun_step2_pairs(fdm_f2 (&Vf)[MP], fdm_f2 (&LV)[MP], double* V,
                                                  fdm_f2 (&S)[MP][NSM], fdm_f2 (&L)[MP][NSM],
@@ -417,13 +421,18 @@ __device__ __forceinline__ void heun_step2_pairs(fdm_f2 (&Vf)[MP], fdm_f2 (&LV)[
 #pragma unroll
     for (int s = 0; s < NS; s++)
       ys[s] = dtr * r[s] + y[s];
+    // (the first rates are added at once: they need no registers beside the second right-hand side)
+#pragma unroll
+    for (int s = 1; s < NS; s++)
+      L[p][s - 1] = hdt * r[s] + L[p][s - 1];
+    LV[p] = hdt * r[0] + LV[p];
     ys[0].v.x = ((clamp >> (2 * p)) & 1u) ? vs : ys[0].v.x;
     ys[0].v.y = ((clamp >> (2 * p + 1)) & 1u) ? vs : ys[0].v.y;
     Model::template rates_fast2<fdm_math_exact>(tr, ys, P[p], r2, alg);
 #pragma unroll
     for (int s = 1; s < NS; s++)
-      L[p][s - 1] = hdt * (r[s] + r2[s]) + L[p][s - 1];
-    LV[p] = hdt * (r[0] + r2[0]) + LV[p];
+      L[p][s - 1] = hdt * r2[s] + L[p][s - 1];
+    LV[p] = hdt * r2[0] + LV[p];
     const bool c0 = (clamp >> (2 * p)) & 1u, c1 = (clamp >> (2 * p + 1)) & 1u;
     V[2 * p] = c0 ? vstim : V[2 * p];
     V[2 * p + 1] = c1 ? vstim : V[2 * p + 1];

@@ -179,16 +179,17 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_POW2(x) fdm_pow2(x)
 #define FDM_POW3(x) fdm_pow3(x)
 #define FDM_POW4(x) fdm_pow4(x)
-    const R fdm_e0 = fdm_ex2(((R)-0x1.2776c50ef9bffp-3) * STATES[0]);
-    const R fdm_d0 = ((fdm_e0 * ((R)0x1.b993fe00d5376p-8)) + ((R)-0x1.0000000000000p+0));
-    const R fdm_d1 = ((fdm_e0 * ((R)0x1.6c0504695c417p-7)) + ((R)1.00000));
-    const R fdm_d2 = ((fdm_e0 * ((R)0x1.8a1e18a954ffap-10)) + ((R)-0x1.0000000000000p+0));
+    const R fdm_h0 = fdm_ex2(((R)-0x1.2776c50ef9bffp-4) * STATES[0] + ((R)-0x1.27e435c543615p+3));
+    const R fdm_e0 = fdm_h0 * fdm_h0;
+    const R fdm_d0 = ((fdm_e0 * ((R)0x1.36c724ec76f8fp+11)) + ((R)-0x1.0000000000000p+0));
+    const R fdm_d1 = ((fdm_e0 * ((R)0x1.00316d3b6c10ap+12)) + ((R)1.00000));
+    const R fdm_d2 = ((fdm_e0 * ((R)0x1.15602daa0de7fp+9)) + ((R)-0x1.0000000000000p+0));
     R fdm_r0, fdm_r1, fdm_r2;
     fdm_rcp_batch(fdm_d0, fdm_d1, fdm_d2, fdm_r0, fdm_r1, fdm_r2);
     ALGEBRAIC[1] = ((((R)-0x1.999999999999ap-4) * STATES[0] + ((R)-0x1.4000000000000p+2)) * fdm_r0);
     ALGEBRAIC[5] = fdm_ex2(((R)-0x1.484b13d7c02a9p-4) * STATES[0] + ((R)-0x1.00b7fb40d531ep+2));
     RATES[1] = (ALGEBRAIC[1] - (ALGEBRAIC[1] + ALGEBRAIC[5]) * STATES[1]);
-    ALGEBRAIC[2] = fdm_ex2(((R)-0x1.2776c50ef9bffp-4) * STATES[0] + ((R)-0x1.27e435c543615p+3));
+    ALGEBRAIC[2] = fdm_h0;
     ALGEBRAIC[6] = fdm_r1;
     RATES[2] = (ALGEBRAIC[2] - (ALGEBRAIC[2] + ALGEBRAIC[6]) * STATES[2]);
     ALGEBRAIC[3] = ((((R)-0x1.47ae147ae147bp-7) * STATES[0] + ((R)-0x1.4cccccccccccdp-1)) * fdm_r2);
