@@ -234,6 +234,64 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
 // its uncoalesced chunks, now 31.7; 100 MB, 0.5 of the measured copy rate).
 constexpr int DIFFUSION_T = 256;
 
+// the stored factorization of a thread's chunk of a fiber, and the solve of the CTA's fiber with it
+template<int M>
+struct DiffusionChunk {
+  int n, lo, cnt;               // nodes of the fiber, the thread's first node and number of nodes
+  double F[M], C[M], inv[M], cl[M], cm[M], cr[M];
+  __device__ __forceinline__ void load(const double* __restrict__ coef, int64_t stride, int64_t o, int nodes)
+  {
+    n = nodes;
+    const int L = (n + DIFFUSION_T - 1) / DIFFUSION_T;
+    lo = min((int)threadIdx.x * L, n);
+    cnt = min(L, n - lo);
+    const double* c0 = coef + o + lo;
+#pragma unroll
+    for (int j = 0; j < M; j++) {
+      const bool on = j < cnt;
+      F[j] = on ? c0[j] : 1.0;   // beyond the chunk the identity map
+      C[j] = on ? c0[2 * stride + j] : -1.0;
+      inv[j] = on ? c0[stride + j] : 0.0;
+      cl[j] = on ? c0[3 * stride + j] : 0.0;
+      cm[j] = on ? c0[4 * stride + j] : 0.0;
+      cr[j] = on ? c0[5 * stride + j] : 0.0;
+    }
+  }
+  // v: the fiber's Vm (global or shared memory), solved in place; sF, sG: 2 * DIFFUSION_T / 32 slots
+  __device__ __forceinline__ void solve(double* v, double* sF, double* sG) const
+  {
+    double u[M + 2], G[M];
+#pragma unroll
+    for (int j = 0; j < M + 2; j++)
+      u[j] = (j <= cnt + 1 && lo + j >= 1 && lo + j <= n) ? v[lo + j - 1] : 0.0;
+#pragma unroll
+    for (int j = 0; j < M; j++)
+      G[j] = inv[j] * (cl[j] * u[j] + cm[j] * u[j + 1] + cr[j] * u[j + 2]);
+    Affine acc{1.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < M; j++)
+      acc = compose(acc, Affine{F[j], G[j]});
+    // its barrier follows every read of the old Vm
+    double d = block_scan_incoming<DIFFUSION_T, false>(acc, sF, sG);
+    Affine bacc{1.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < M; j++) {
+      d = F[j] * d + G[j];
+      G[j] = j < cnt ? d : 0.0;
+    }
+#pragma unroll
+    for (int j = M - 1; j >= 0; j--)
+      bacc = compose(bacc, Affine{-C[j], G[j]});
+    double x = block_scan_incoming<DIFFUSION_T, true>(bacc, sF + DIFFUSION_T / 32, sG + DIFFUSION_T / 32);
+#pragma unroll
+    for (int j = M - 1; j >= 0; j--) {
+      x = -C[j] * x + G[j];
+      if (j < cnt)
+        v[lo + j] = x;
+    }
+  }
+};
+
 template<int M>
 __global__ void __launch_bounds__(DIFFUSION_T) diffusion_reg_kernel(const int64_t* __restrict__ fiber_offsets,
                                                                     const double* __restrict__ coef, int64_t stride,
@@ -246,52 +304,107 @@ __global__ void __launch_bounds__(DIFFUSION_T) diffusion_reg_kernel(const int64_
   if (eq_counter && eq_counter[f % n_ranks] == eq_nbuf[f % n_ranks])
     return; // the whole CTA: the rank's buffers are all inactive
   const int64_t o = fiber_offsets[f];
+  DiffusionChunk<M> chunk;
+  chunk.load(coef, stride, o, (int)(fiber_offsets[f + 1] - o));
+  chunk.solve(vm + o, sF, sG);
+}
+
+// A whole window of split steps of few fibers in one launch, FP64: a fiber per thread-block cluster, a thread per node.
+// With a launch per half step and per solve the launches, the passes over the states and the start of every kernel
+// take about half of a step that has some hundred nodes per SM.  Here the states stay in registers for the window; the
+// CTAs send their Vm to the cluster's first one, which solves the fiber's diffusion as diffusion_reg_kernel does, with
+// the factors in registers, and the others fetch theirs back: two cluster barriers per step.  Same functions and
+// partition as the kernels it stands in for, so the same values whichever form the number of fibers leads to.
+// Bound by the latency of a node's Heun chain, 1.6 us of the 1.8 + 1.6 n0 us per step at n0 substeps a half step.  16
+// fibers of 1481 nodes (clusters of 6), 400 steps: 7.06 -> 4.38 ms; one of 101 nodes, 50 steps: 588 -> 412 us; 74 of 500:
+// 13.2 -> 8.8 us per step.
+constexpr int WINDOW_T = DIFFUSION_T;
+
+template<class Model, class Math, int M>
+__global__ void __launch_bounds__(WINDOW_T, 1) window_cluster_kernel(ReactionArgs a,
+                                                                     const int64_t* __restrict__ fiber_offsets,
+                                                                     const double* __restrict__ coef, int n_steps)
+{
+  constexpr int NS = Model::nStates;
+  constexpr int NP = Model::nParameters > 0 ? Model::nParameters : 1;
+  constexpr int NSM = NS > 1 ? NS - 1 : 1;
+  __shared__ double vs[WINDOW_T * M];
+  __shared__ double sF[2 * (WINDOW_T / 32)], sG[2 * (WINDOW_T / 32)];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = (int)cluster.block_rank(), csize = (int)cluster.num_blocks();
+  const int f = blockIdx.x / csize;
+  const int64_t o = fiber_offsets[f];
   const int n = (int)(fiber_offsets[f + 1] - o);
-  const int L = (n + DIFFUSION_T - 1) / DIFFUSION_T;
-  const int lo = min((int)threadIdx.x * L, n);
-  const int cnt = min(L, n - lo);
-  const double* c0 = coef + o + lo;
-  double* v = vm + o + lo;
-  double F[M], G[M], C[M];
-  double u[M + 2];
+  const int npc = (n + csize - 1) / csize;   // nodes per CTA, at most WINDOW_T
+  const int q = crank * npc + (int)threadIdx.x;
+  const bool ok = (int)threadIdx.x < npc && q < n;
+  const int64_t i = o + (ok ? q : 0);
+  double* home = cluster.map_shared_rank(vs, 0);
+  double* st = (double*)a.states;
+  const double* pr = (const double*)a.params;
+  double V = a.vm[i], S[NSM], Lo[NSM], P[NP], Pstim[NP];
 #pragma unroll
-  for (int j = 0; j < M + 2; j++)
-    u[j] = (j <= cnt + 1 && lo + j >= 1 && lo + j <= n) ? v[j - 1] : 0.0;
+  for (int s = 1; s < NS; s++) {
+    S[s - 1] = st[(s - 1) * a.stride + i];
+    Lo[s - 1] = 0.0;
+  }
 #pragma unroll
-  for (int j = 0; j < M; j++) {
-    if (j < cnt) {
-      F[j] = c0[j];
-      C[j] = c0[2 * stride + j];
-      G[j] = c0[stride + j] *
-             (c0[3 * stride + j] * u[j] + c0[4 * stride + j] * u[j + 1] + c0[5 * stride + j] * u[j + 2]);
-    } else {
-      F[j] = 1.0;   // the identity map
-      C[j] = -1.0;
-      G[j] = 0.0;
+  for (int p = 0; p < Model::nParameters; p++) {
+    P[p] = pr[p * a.stride + i];
+    Pstim[p] = (a.stimulus_mode == 1 && p == a.stimulus_parameter) ? a.stimulus_value : P[p];
+  }
+  const int cf = ok ? a.clamp_fiber[i] : -1;
+  const int slot = ok && a.trace_slot ? a.trace_slot[i] : -1;
+  DiffusionChunk<M> chunk;
+  chunk.load(coef, a.stride, o, crank == 0 ? n : 0);
+#pragma unroll 1
+  for (int hs = 0; hs < 2 * n_steps; hs++) {
+    const SplitStep s = a.steps[hs >> 1];
+    const double t0 = (hs & 1) ? s.mid : s.t;
+    const int base = hs * a.nsub_stride;
+    const int first = a.gate ? gate_first(a.gate_start, a.gate_stride, a.gate[i], hs) : 0;
+    const bool store = a.store_alg && hs == 2 * n_steps - 1;
+    if (ok) {
+#pragma unroll 1
+      for (int k = first; k < s.n0; k++) {
+        const double t = xadd(t0, xmul((double)k, s.dt0));
+        const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
+        const bool vclamp = stim && a.stimulus_mode == 0;
+        double Pk[NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+          Pk[p] = (stim && a.stimulus_mode == 1) ? Pstim[p] : P[p];
+        if (store && k == s.n0 - 1) {
+          double alg[Model::nAlgebraics];
+          heun_step<Model, double, Math, true>(V, S, Lo, Pk, t, s.dt0, vclamp, a.vstim, alg);
+          store_algebraics<Model>(alg, a.n_alg_out, a.alg_indices, a.alg_out, a.n_nodes, i);
+        } else {
+          heun_step<Model, double, Math, false>(V, S, Lo, Pk, t, s.dt0, vclamp, a.vstim, nullptr);
+        }
+      }
     }
+    if (hs & 1) {
+      if (slot >= 0)
+        record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, V);
+      continue;
+    }
+    // (a slot of home is read back by the thread that fills it: no barrier is needed before the next fill)
+    if (ok)
+      home[q] = V;
+    cluster.sync();
+    if (crank == 0)
+      chunk.solve(vs, sF, sG);
+    cluster.sync();
+    if (ok)
+      V = home[q];
   }
-  Affine acc{1.0, 0.0};
+  if (ok) {
+    a.vm[i] = V;
 #pragma unroll
-  for (int j = 0; j < M; j++)
-    acc = compose(acc, Affine{F[j], G[j]});
-  // its barrier follows every read of the old Vm
-  double d = block_scan_incoming<DIFFUSION_T, false>(acc, sF, sG);
-  Affine bacc{1.0, 0.0};
-#pragma unroll
-  for (int j = 0; j < M; j++) {
-    d = F[j] * d + G[j];
-    G[j] = j < cnt ? d : 0.0;
+    for (int s = 1; s < NS; s++)
+      st[(s - 1) * a.stride + i] = S[s - 1];
   }
-#pragma unroll
-  for (int j = M - 1; j >= 0; j--)
-    bacc = compose(bacc, Affine{-C[j], G[j]});
-  double x = block_scan_incoming<DIFFUSION_T, true>(bacc, sF + DIFFUSION_T / 32, sG + DIFFUSION_T / 32);
-#pragma unroll
-  for (int j = M - 1; j >= 0; j--) {
-    x = -C[j] * x + G[j];
-    if (j < cnt)
-      v[j] = x;
-  }
+  cluster.sync();   // the first CTA's shared memory outlives the others' reads
 }
 
 } // namespace fdm

@@ -142,6 +142,7 @@ struct fdm_solver {
   // fused bins
   int shape = -1;    // index into fused_shapes, or into cluster_shapes when cluster > 1
   int cluster = 1;   // CTAs per fiber (thread-block cluster mode when > 1)
+  int window_cluster = 0;   // split method: CTAs per fiber of window_cluster_kernel (0: launches per half step)
   int n_bins = 0;
   std::vector<int> bin_start, bin_fibers;
 
@@ -833,6 +834,8 @@ static int set_fibers(fdm_solver* s, int n_fibers, const int64_t* fiber_offsets,
 
   // fused bins
   s->cluster = 1;
+  s->window_cluster = s->cfg.method == FDM_METHOD_SPLIT && s->real_bytes == 8
+                          ? window_cluster_size(s->cfg.model, n_fibers, maxlen) : 0;
   if (s->cfg.method == FDM_METHOD_FUSED && n_fibers > 0) {
     const int regular = s->cfg.cluster_size >= 2 ? -1 : choose_shape(s);
     if (regular >= 0) {
@@ -2286,6 +2289,15 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
       return cudaSuccess;
     };
     return replay_or_launch(eq_launches, &n_launches);
+  }
+  // few fibers: the whole window in one launch
+  // (not with profiling, which times the reaction's launches alone)
+  if (s->window_cluster > 0 && rk == REAL_F64 && !s->adj_forward && !prof) {
+    ra.store_alg = store_alg && s->n_alg_out > 0;
+    FDM_CUDA(launch_window(s->cfg.model, mk, ra, s->n_fibers, s->window_cluster, s->max_fiber_len, s->off_d.p,
+                           s->coef.p, n_steps, s->stream));
+    s->launches++;
+    return FDM_OK;
   }
   // Launches of the window: the first half step, the diffusion solve, then per following split step one launch of the
   // second half step and the next one's first (nothing lies between them: one launch and one pass over the states

@@ -54,6 +54,13 @@ typedef int (*ModelModuleEntry)(ModelModule* out);
 int register_model_module(const ModelModule& m);
 
 // split path
+// how many clusters of csize CTAs the current device holds at once with an SM for every CTA
+int clusters_with_own_sms(int csize);
+// CTAs per fiber with which launch_window can run whole windows of the split method (0: it cannot or should not)
+int window_cluster_size(int model, int n_fibers, int64_t max_fiber_len);
+// n_steps split steps of every fiber in one launch (FP64; fdm_diffusion.cuh)
+cudaError_t launch_window(int model, MathKind mk, const ReactionArgs& a, int n_fibers, int csize, int64_t max_fiber_len,
+                          const int64_t* fiber_offsets, const double* coef, int n_steps, cudaStream_t s);
 cudaError_t launch_reaction(int model, RealKind rk, MathKind mk, const ReactionArgs& a, cudaStream_t s);
 // at most max_iterations RK4 steps of the equilibrium search of one instance (u in/out, u0 the initial values)
 cudaError_t launch_equilibrium_search(int model, MathKind mk, double* u, const double* u0, const double* params,

@@ -229,6 +229,93 @@ cudaError_t launch_diffusion(int n_fibers, const int64_t* fiber_offsets, const d
   return cudaGetLastError();
 }
 
+// Clusters stay within a group of SMs that share a network port, and the groups' sizes differ: on a B200 there is room
+// for 15 clusters of 8 CTAs, 22 of 6, 26 of 5, 33 of 4, 45 of 3, 74 of 2 with an SM for every CTA (the shared memory
+// asked for leaves none for a second one).
+__global__ void own_sm_probe_kernel()
+{
+}
+
+int clusters_with_own_sms(int csize)
+{
+  constexpr int HALF_SM = 120 * 1024;
+  int n = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)csize);
+  cfg.blockDim = dim3(WINDOW_T);
+  cfg.dynamicSmemBytes = HALF_SM;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(own_sm_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HALF_SM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, own_sm_probe_kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+// The few fibers a window kernel is for: a CTA for at most WINDOW_T nodes and an SM for every CTA; the most CTAs per fiber
+// (at most 8, down to 128 nodes each) with which that holds.  Where CTAs share an SM, the launches cost less than that:
+// per step of 5 substeps a half step 16 fibers of 1481 nodes take 10.6 us with clusters of 6, 19.7 with clusters of 8 (one
+// more than fit) and 15.0 with a launch per half step and solve; 24 fibers 20.3 with clusters of 6 (22 fit) and 14.9.
+int window_cluster_size(int model, int n_fibers, int64_t max_fiber_len)
+{
+  const int least = (int)std::min<int64_t>((max_fiber_len + WINDOW_T - 1) / WINDOW_T, FDM_MAX_CLUSTER + 1);
+  const int most = (int)std::min<int64_t>((max_fiber_len + 127) / 128, FDM_MAX_CLUSTER);
+  if (model != 0 || n_fibers < 1)
+    return 0;
+  for (int c = most; c >= std::max(least, 1); c--)
+    if (clusters_with_own_sms(c) >= n_fibers)
+      return c;
+  return 0;
+}
+
+template<class Math, int M>
+static cudaError_t window_launch(const ReactionArgs& a, int n_fibers, int csize, const int64_t* fiber_offsets,
+                                 const double* coef, int n_steps, cudaStream_t s)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(n_fibers * csize));
+  cfg.blockDim = dim3(WINDOW_T);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, window_cluster_kernel<HH, Math, M>, a, fiber_offsets, coef, n_steps);
+}
+
+template<class Math>
+static cudaError_t window_shape(const ReactionArgs& a, int n_fibers, int csize, int64_t max_fiber_len,
+                                const int64_t* fiber_offsets, const double* coef, int n_steps, cudaStream_t s)
+{
+  switch ((max_fiber_len + 2 * WINDOW_T - 1) / (2 * WINDOW_T)) {
+  case 1: return window_launch<Math, 2>(a, n_fibers, csize, fiber_offsets, coef, n_steps, s);
+  case 2: return window_launch<Math, 4>(a, n_fibers, csize, fiber_offsets, coef, n_steps, s);
+  case 3: return window_launch<Math, 6>(a, n_fibers, csize, fiber_offsets, coef, n_steps, s);
+  case 4: return window_launch<Math, 8>(a, n_fibers, csize, fiber_offsets, coef, n_steps, s);
+  default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_window(int model, MathKind mk, const ReactionArgs& a, int n_fibers, int csize, int64_t max_fiber_len,
+                          const int64_t* fiber_offsets, const double* coef, int n_steps, cudaStream_t s)
+{
+  if (model != 0 || csize < 1)
+    return cudaErrorInvalidValue;
+  return mk == MATH_EXACT
+             ? window_shape<fdm_math_exact>(a, n_fibers, csize, max_fiber_len, fiber_offsets, coef, n_steps, s)
+             : window_shape<fdm_math_approx>(a, n_fibers, csize, max_fiber_len, fiber_offsets, coef, n_steps, s);
+}
+
 // ---- equilibrium skip ----
 cudaError_t launch_equilibrium_half(int model, RealKind rk, MathKind mk, const ReactionArgs& a, const EqLayout& L,
                                     const EqSpec& e, int n_states, int* n_launches, cudaStream_t s)

@@ -147,3 +147,35 @@ def test_cluster_halos(dt, threads, per_thread):
             slv.advanceTimeSpan()
             got = slv.states()
         assert np.max(np.abs(got[0] - ref[0])) < tol[0] and np.max(np.abs(got[1:] - ref[1:])) < tol[1]
+
+
+# whole windows in one launch (few fibers: at most 2048 nodes, clusters of 1 to 8 CTAs with an SM each): one to eight
+# CTAs, nodes per CTA from 2 to 256, fibers shorter than the cluster's first CTA, the last number of fibers that still
+# fits 8 and 1 CTAs and the first that does not, 2049 nodes (a launch per half step and solve); windows of 1, 7, 20 steps
+@pytest.mark.parametrize("lengths", [[2], [3, 2], [128], [129], [256, 257], [1481], [2048, 2, 255, 1024, 1025],
+                                     [1024] * 15, [1024] * 16, [2041] * 16, [100] * 148, [100] * 149, [2049, 40]])
+@pytest.mark.parametrize("approximate", [False, True])
+def test_window_partitions(lengths, approximate):
+    rng = np.random.default_rng(7)
+    s = S.uniform_fibers(H.HH, lengths, 0.01, 3.828 / 500, call_frequency=0.5, repeat_after_first_call=0.1,
+                         call_enable_begin=0.0, end_time=0.02, dt_0d=2e-4, dt_1d=1e-3, dt_splitting=1e-3,
+                         dt_repeated_call=1e-3, clamp_rule="center", approximate_exponential_function=approximate,
+                         algebraics_for_transfer=[0, 4, 8])
+    s = H.complete(s)
+    s.states = s.states.copy()
+    s.states[0] += rng.uniform(0.0, 40.0, s.n_nodes)
+    ref = H.run_oracle(s.copy())[0]
+    nodes = sorted({0, s.n_nodes // 2, s.n_nodes - 1})
+    got = {}
+    # with profiling the same steps run as a launch per half step and solve
+    for profile, per_launch in ((True, 0), (False, 0), (False, 1), (False, 7)):
+        with S.FastMonodomainSolver(s.copy(), method="split", precision="fp64", profile=profile,
+                                    steps_per_launch=per_launch, trace_nodes=nodes, trace_capacity=20) as slv:
+            slv.advanceTimeSpan()
+            got[profile, per_launch] = slv.states(), slv.algebraics(), slv.trace()
+    # 400 right-hand sides: roundings of 1e-14 of Vm and, with the approximate exponential, its 1024th power's 1e-13
+    first = got[True, 0]
+    for values in got.values():
+        assert np.max(np.abs(values[0] - ref)) < 1e-8
+        for v, v0 in zip(values, first):
+            assert v.shape == v0.shape and np.max(np.abs(v - v0)) < 1e-9
