@@ -89,3 +89,12 @@ def test_autotuner_considers_cluster_shapes():
     assert lay["cluster_size"] == slv.tuning["cluster_size"]
     ref, _, _, _ = H.run_oracle(s.copy())
     assert np.max(np.abs(st[0] - ref[0])) <= GP.VM_TOL_FP64
+
+
+# the last numbers of fibers of 1481 nodes for which all clusters of 8 (192 threads) and of 6 (256) have an SM per CTA,
+# and the first ones beyond
+@pytest.mark.parametrize("n_fibers,csize", [(15, 8), (16, 6), (22, 6), (23, 3)])
+def test_cluster_size_leaves_every_cta_an_sm(n_fibers, csize):
+    s = H.c1_system(n_fibers=n_fibers, n_nodes=1481, end_time=0.05)
+    assert _layout(s)["cluster_size"] == csize
+    GP.compare(s, "fused", "fp64", GP.VM_TOL_FP64, 1e-8)
