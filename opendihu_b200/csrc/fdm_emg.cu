@@ -710,6 +710,197 @@ __global__ void __launch_bounds__(EMG_T) cg_update_kernel(int64_t N, double* __r
   }
 }
 
+// ---- persistent conjugate gradients (Jacobi) for meshes that fit on the chip --------------------------------
+// All iterations of a solve in one cooperative launch: CTA c owns CGP_T consecutive nodes, a thread each, with x, r, p,
+// q, z, dinv and 10 of the 27 coefficients in registers and the others in shared memory, so an iteration moves only z
+// (L2) and the partial sums.  Same recurrences and the same check after every CGP_CHECK iterations as the
+// launch-per-step form; the sums add the CTAs' partials in CTA order.
+// A CTA publishes a partial sum in its slot and waits until all slots of that sum are filled: the wait is also the grid
+// barrier (between the p.q sum and the update every neighbour has read the old z, between the r.z sum and the next
+// product every z is written).  Three sets of slots rotate: a CTA clears its slot of the previous sum's set once the
+// current sum is complete (everyone has left the previous one), two sums before it is filled again.  A CTA waits at
+// most CGP_SPINS polls, then the kernel ends with CGP_TIMED_OUT.
+// Bound by latency (two grid-wide sums per iteration).  Per iteration, against two launches: 1701 nodes 10.8 us (13.5), 28,033
+// 10.7 (12.9), 93,125 11.7 (17.3), 113,256 12.3 (17.4).
+constexpr int CGP_T = 768;
+constexpr int CGP_REG = 10;                       // centre and forward coefficients in registers
+constexpr int CGP_SM = 13 + EMG_NC - CGP_REG;     // the others in shared memory: backward, then forward
+constexpr int CGP_CHECK = 8;
+constexpr int CGP_SPINS = 1 << 24;
+// a CTA's slots in 128 B of its own: with all CTAs' slots side by side a sum takes 5.2 us on 122 CTAs, so 2.9
+constexpr int CGP_SLOT = 16, CGP_SECOND = 8;      // 64-bit words per CTA; the second value's offset
+constexpr unsigned long long CGP_EMPTY = ~0ull;   // a NaN pattern that no arithmetic produces
+enum { CGP_CONVERGED = 1, CGP_TIMED_OUT = 2 };
+
+struct CgpArgs {
+  Grid g;
+  const double* U;
+  const unsigned char* mask;
+  const double* dinv;
+  double *x, *r, *z;
+  double* S;                      // scalars: CG_RZ and CG_RR in and out
+  unsigned long long* slots;      // [3][gridDim][CGP_SLOT], filled with CGP_EMPTY
+  int* result;                    // [0] status, [1] iterations
+  double target;                  // stop at ||r|| <= target
+  int max_iterations;
+};
+
+// the sum over the CTA of v (the same in all threads); red: one double per warp, free again after the next barrier
+__device__ __forceinline__ double cgp_cta_sum(double v, double* red)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0)
+    red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = (threadIdx.x & 31) < CGP_T / 32 ? red[threadIdx.x & 31] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// K (1 or 2) sums over all CTAs (the same in all threads of all CTAs); false if the wait ran out.  K gridDim.x <= CGP_T
+template<int K>
+__device__ bool cgp_grid_sum(double (&v)[K], const CgpArgs& a, int phase, double (*red)[CGP_T / 32], int* abort)
+{
+  const int G = gridDim.x, t = threadIdx.x;
+  unsigned long long* set = a.slots + (size_t)(phase % 3) * G * CGP_SLOT;
+  double own[K];
+#pragma unroll
+  for (int c = 0; c < K; c++)
+    own[c] = cgp_cta_sum(v[c], red[c]);
+  // (the barrier inside cgp_cta_sum follows every thread's writes of z; the fence publishes them with the sum)
+  if (t == 0) {
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < K; c++)
+      asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(set + (size_t)blockIdx.x * CGP_SLOT + c * CGP_SECOND),
+                   "l"(__double_as_longlong(own[c])) : "memory");
+  }
+  double got = 0.0;
+  if (t < K * G) {
+    const bool second = K == 2 && t >= G;
+    const unsigned long long* slot = set + (size_t)(second ? t - G : t) * CGP_SLOT + (second ? CGP_SECOND : 0);
+    unsigned long long u = CGP_EMPTY;
+    for (int spins = 0; spins < CGP_SPINS && u == CGP_EMPTY; spins++)
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(slot) : "memory");
+    if (u == CGP_EMPTY)
+      *abort = 1;
+    got = __longlong_as_double((long long)u);
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  }
+  __syncthreads();
+  if (*abort)
+    return false;
+#pragma unroll
+  for (int c = 0; c < K; c++)
+    v[c] = cgp_cta_sum(t >= c * G && t < (c + 1) * G ? got : 0.0, red[K + c]);
+  if (t == 0) {
+    // the set of the sum before this one
+    unsigned long long* old = a.slots + ((size_t)((phase + 2) % 3) * G + blockIdx.x) * CGP_SLOT;
+    old[0] = CGP_EMPTY;
+    old[CGP_SECOND] = CGP_EMPTY;
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(CGP_T, 1) cg_persistent_kernel(CgpArgs a)
+{
+  extern __shared__ double sm[];
+  double(*sc)[CGP_T] = (double(*)[CGP_T])sm;                            // CGP_SM coefficients
+  double(*sv)[CGP_T + 2] = (double(*)[CGP_T + 2])(sm + CGP_SM * CGP_T); // 9: rows of z around the CTA's nodes
+  __shared__ double red[4][CGP_T / 32];
+  __shared__ int abort;
+  const int t = threadIdx.x;
+  const int64_t N = a.g.n_nodes();
+  const int64_t sy = a.g.nx, sz = (int64_t)a.g.nx * a.g.ny;
+  const int64_t n0 = (int64_t)blockIdx.x * CGP_T, n = n0 + t;
+  const bool ok = n < N;
+  double fwd[CGP_REG];
+#pragma unroll
+  for (int q = 0; q < EMG_NC; q++) {
+    const double u = ok ? a.U[q * N + n] : 0.0;
+    if (q < CGP_REG)
+      fwd[q] = u;
+    else
+      sc[13 + q - CGP_REG][t] = u;
+  }
+#pragma unroll
+  for (int q = 14; q < 27; q++) {
+    int dx, dy, dz;
+    stencil_offset(q, dx, dy, dz);
+    const int64_t b = n - (dx + dy * sy + dz * sz);
+    sc[q - 14][t] = ok && b >= 0 ? a.U[(q - 13) * N + b] : 0.0;
+  }
+  const bool free_row = ok && !(a.mask && a.mask[n]);
+  const double dinv = ok ? a.dinv[n] : 0.0;
+  double x = ok ? a.x[n] : 0.0, r = ok ? a.r[n] : 0.0, z = ok ? a.z[n] : 0.0, p = 0.0, q = 0.0;
+  double rz = a.S[CG_RZ], rr = a.S[CG_RR], beta = 0.0;
+  if (t == 0)
+    abort = 0;
+  int it = 0, status = 0, phase = 0;
+  while (sqrt(rr) > a.target && it < a.max_iterations) {
+    const int chunk = min(CGP_CHECK, a.max_iterations - it);
+    for (int c = 0; c < chunk && !status; c++) {
+      // w = K z
+      for (int e = t; e < 9 * (CGP_T + 2); e += CGP_T) {
+        const int row = e / (CGP_T + 2), k = e % (CGP_T + 2);
+        const int64_t m = n0 + (row % 3 - 1) * sy + (row / 3 - 1) * sz + k - 1;
+        sv[row][k] = (m >= 0 && m < N) ? __ldcg(a.z + m) : 0.0;
+      }
+      __syncthreads();
+      double w = fwd[0] * z;
+#pragma unroll
+      for (int k = 14; k < 27; k++) {
+        int dx, dy, dz;
+        stencil_offset(k, dx, dy, dz);
+        const double f = k - 13 < CGP_REG ? fwd[k - 13 < CGP_REG ? k - 13 : 0] : sc[k - CGP_REG][t];
+        w += f * sv[(dy + 1) + 3 * (dz + 1)][t + 1 + dx] +
+             sc[k - 14][t] * sv[(1 - dy) + 3 * (1 - dz)][t + 1 - dx];
+      }
+      w = free_row ? w : 0.0;
+      p = z + beta * p;
+      q = w + beta * q;
+      double pq[1] = {p * q};
+      if (!cgp_grid_sum<1>(pq, a, phase++, red, &abort)) {
+        status = CGP_TIMED_OUT;
+        break;
+      }
+      const double alpha = pq[0] != 0.0 ? rz / pq[0] : 0.0;
+      x += alpha * p;
+      r -= alpha * q;
+      z = r * dinv;
+      if (ok)
+        __stcg(a.z + n, z);
+      double s2[2] = {r * z, r * r};
+      if (!cgp_grid_sum<2>(s2, a, phase++, red, &abort)) {
+        status = CGP_TIMED_OUT;
+        break;
+      }
+      beta = rz != 0.0 ? s2[0] / rz : 0.0;
+      rz = s2[0];
+      rr = s2[1];
+    }
+    it += chunk;
+    if (status || !isfinite(rr))
+      break;
+  }
+  if (ok) {
+    a.x[n] = x;
+    a.r[n] = r;
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    a.S[CG_RZ] = rz;
+    a.S[CG_RR] = rr;
+    a.result[0] = status ? status : CGP_CONVERGED;
+    a.result[1] = it;
+  }
+}
+
+constexpr size_t CGP_SMEM = sizeof(double) * (CGP_SM * CGP_T + 9 * (CGP_T + 2));
+
 // S[SUM] = sum x, S[BB] = b.b (b may be null)
 __global__ void __launch_bounds__(EMG_T) sum_kernel(int64_t N, const double* __restrict__ x,
                                                     const double* __restrict__ b, double* S, double* partial,
@@ -1102,6 +1293,8 @@ struct fdm_emg {
       scal, tensor_i, tensor_e, tmp;
   Buf<unsigned char> mask;
   Buf<unsigned> counter;                       // last-block counter of the grid reductions
+  Buf<unsigned long long> cgp_slots;           // cg_persistent_kernel: slots of the grid-wide sums, result
+  int cgp_ctas = -1;                           // its CTAs that can be resident together (-1: not asked yet)
   cudaGraphExec_t graphs[1] = {nullptr};       // CG chunk of the bidomain solve
   int precond = FDM_EMG_PRECOND_MULTIGRID;     // of the bidomain solve
   StencilTiles tiles{};                        // of the fine grid (chunks == 0: node-per-thread passes)
@@ -1367,6 +1560,46 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
   if (!m->tiles.chunks)
     if (const int rc = choose_tiles(m, g, &m->tiles))
       return rc;
+  // small meshes, Jacobi: all iterations in one cooperative launch, as long as a CTA per CGP_T nodes is resident
+  // (113,664 nodes on 148 SMs); beyond that a launch per pass
+  if (!use_mg && m->cgp_ctas < 0) {
+    int coop = 0, sms = 0, per_sm = 0;
+    EMG_CUDA(m, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device));
+    EMG_CUDA(m, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
+    EMG_CUDA(m, cudaFuncSetAttribute(cg_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CGP_SMEM));
+    EMG_CUDA(m, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_persistent_kernel, CGP_T, CGP_SMEM));
+    m->cgp_ctas = coop ? std::min(sms * per_sm, CGP_T / 2) : 0;
+  }
+  const int64_t ctas = (N + CGP_T - 1) / CGP_T;
+  if (!use_mg && ctas <= m->cgp_ctas && rn > target) {
+    const size_t n_slots = 3 * CGP_SLOT * (size_t)ctas;
+    EMG_CUDA(m, m->cgp_slots.alloc(n_slots + 1));
+    EMG_CUDA(m, cudaMemsetAsync(m->cgp_slots.p, 0xff, sizeof(unsigned long long) * n_slots, s));
+    int result[2];
+    CgpArgs ca{g, U, mask, m->dinv.p, x, m->r.p, m->z.p, S, m->cgp_slots.p, (int*)(m->cgp_slots.p + n_slots), target,
+               max_it};
+    void* args[] = {&ca};
+    EMG_CUDA(m, cudaFuncSetAttribute(cg_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CGP_SMEM));
+    EMG_CUDA(m, cudaLaunchCooperativeKernel(cg_persistent_kernel, dim3((unsigned)ctas), dim3(CGP_T), args, CGP_SMEM,
+                                            s));
+    if (nullspace) {
+      sum_kernel<<<nb, EMG_T, 0, s>>>(N, x, nullptr, S, P, C);
+      subtract_mean_kernel<<<nb, EMG_T, 0, s>>>(N, x, x, S);
+    }
+    EMG_CUDA(m, cudaMemcpyAsync(hs, S, sizeof(hs), cudaMemcpyDeviceToHost, s));
+    EMG_CUDA(m, cudaMemcpyAsync(result, ca.result, sizeof(result), cudaMemcpyDeviceToHost, s));
+    EMG_CUDA(m, cudaStreamSynchronize(s));
+    if (result[0] == CGP_TIMED_OUT)
+      return emg_fail(m, FDM_ERR_TIMEOUT, "conjugate gradients: a wait between the blocks ran out");
+    rn = std::sqrt(hs[CG_RR]);
+    if (!std::isfinite(rn))
+      return emg_fail(m, FDM_ERR_NAN, "conjugate gradients: non-finite residual");
+    if (iterations)
+      *iterations = result[1];
+    if (residual)
+      *residual = rn;
+    return FDM_OK;
+  }
   // one iteration: direction and product, then the update
   auto iteration = [&]() {
     if (!mask && m->tiles.chunks) {
