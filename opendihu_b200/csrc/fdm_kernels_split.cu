@@ -390,6 +390,9 @@ cudaError_t launch_adjoint_diffusion(int n_fibers, const int64_t* fiber_offsets,
     if (max_fiber_len <= 1024)
       return adjoint_diffusion_block<256, 4>(n_fibers, fiber_offsets, element_lengths, coef, stride, lam, u, x,
                                              implicit_euler, grad_prefactor, s);
+    if (max_fiber_len <= 1536)
+      return adjoint_diffusion_block<256, 6>(n_fibers, fiber_offsets, element_lengths, coef, stride, lam, u, x,
+                                             implicit_euler, grad_prefactor, s);
     if (max_fiber_len <= 2048)
       return adjoint_diffusion_block<256, 8>(n_fibers, fiber_offsets, element_lengths, coef, stride, lam, u, x,
                                              implicit_euler, grad_prefactor, s);

@@ -179,3 +179,32 @@ def test_window_partitions(lengths, approximate):
         assert np.max(np.abs(values[0] - ref)) < 1e-8
         for v, v0 in zip(values, first):
             assert v.shape == v0.shape and np.max(np.abs(v - v0)) < 1e-9
+
+
+# the reverse diffusion with a fiber per CTA: 128 x 4, 256 x 4, 256 x 6, 256 x 8, 512 x 8 nodes and one node more; against
+# central differences in each fiber's conductivity
+@pytest.mark.parametrize("n_nodes", [512, 513, 1024, 1025, 1536, 1537, 2048, 2049])
+@pytest.mark.parametrize("scheme", ["ImplicitEuler", "CrankNicolson"])
+def test_adjoint_diffusion_shapes(n_nodes, scheme):
+    from opendihu_b200 import adjoint as ADJ
+    from opendihu_b200 import workloads as WL
+    s = H.complete(H.c1_system(n_fibers=2, n_nodes=n_nodes, end_time=0.02, diffusion_scheme=scheme))
+    s.states = s.states.copy()
+    s.states[0] += np.random.default_rng(6).uniform(0.0, 40.0, s.n_nodes)
+    sensors = np.array([0, n_nodes // 2, n_nodes - 1, n_nodes, 2 * n_nodes - 1])
+    pf = np.array([3.0, 4.5]) / 500
+    s.prefactor = pf.copy()
+    s.parameters = WL.hh_parameters(s, np.ones(2), np.ones(2))
+    eng = ADJ.AdjointEngine(s, sensors, checkpoint_every=7)
+    try:
+        trace = eng.forward(pf, s.parameters)
+        w = np.random.default_rng(8).standard_normal(np.shape(trace))
+        g = eng.backward(w)["prefactor"]
+        for f in range(2):
+            e = np.zeros(2)
+            e[f] = 1e-5 * pf[f]
+            d = (np.sum(w * eng.forward(pf + e, s.parameters)) - np.sum(w * eng.forward(pf - e, s.parameters))) / 2e-5
+            # the loss is rounded at 1e-13 of some 1e3, the difference quotient at 1e-10 / 1e-5
+            assert abs(g[f] * pf[f] - d) < 1e-4 + 1e-5 * abs(d)
+    finally:
+        eng.close()
