@@ -155,72 +155,83 @@ __global__ void __launch_bounds__(SCHEDULE_T) stimulation_schedule_kernel(StimAr
   bool cur = a.currently && a.currently[f];              // the decision of the substep before the next valid bit
   int first_bit = -1;                                    // the first stimulating bit of the window
   uint32_t out = 0u;                                     // lane k: word k of the current group of 32 words
-  for (int w = 0; w < a.words_per_fiber; w++) {
-    const int bit = w * 32 + lane;
-    const int hs = bit / a.nsub_stride, k = bit - hs * a.nsub_stride;
-    const int j = hs >> 1;
-    bool valid = j < n_steps;
-    double t = 0.0;
-    bool fires = false;
-    if (valid) {
+  // SCHEDULE_AHEAD words at a time: their loads (the step, then the firing event of its row) are in flight together
+  // (16 fibers, 1000 substeps: 24.9 -> 21.1 us)
+  constexpr int SCHEDULE_AHEAD = 4;
+  for (int w0 = 0; w0 < a.words_per_fiber; w0 += SCHEDULE_AHEAD) {
+    bool valids[SCHEDULE_AHEAD], fire[SCHEDULE_AHEAD];
+    double times[SCHEDULE_AHEAD];
+#pragma unroll
+    for (int i = 0; i < SCHEDULE_AHEAD; i++) {
+      const int bit = (w0 + i) * 32 + lane;
+      const int hs = bit / a.nsub_stride, k = bit - hs * a.nsub_stride;
+      const int j = min(hs >> 1, n_steps - 1);
       const SplitStep s = steps[j];
-      valid = k < s.n0;
-      t = xadd((hs & 1) ? s.mid : s.t, xmul((double)k, s.dt0));
-      int row = (int)round(xmul(t, freq)) % a.rows;
+      valids[i] = w0 + i < a.words_per_fiber && (hs >> 1) < n_steps && k < s.n0;
+      times[i] = xadd((hs & 1) ? s.mid : s.t, xmul((double)k, s.dt0));
+      int row = valids[i] ? (int)round(xmul(times[i], freq)) % a.rows : 0;
       if (row < 0)
         row += a.rows;
-      fires = a.firing_events[(int64_t)row * a.cols + col] != 0;
+      fire[i] = a.firing_events[(int64_t)row * a.cols + col] != 0;
     }
-    const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    unsigned todo = vmask;   // the bits not decided yet
-    unsigned stim = 0u;
-    while (todo) {
-      const bool check = valid && t >= next && t >= begin;
-      const bool ends = check && repeat != 0 && xsub(t, next) > repeat;
-      const unsigned emask = __ballot_sync(0xffffffffu, ends) & todo;
-      const unsigned smask = __ballot_sync(0xffffffffu, check && fires) & todo;
-      if (!emask) {
-        stim |= smask;
+#pragma unroll
+    for (int i = 0; i < SCHEDULE_AHEAD; i++) {
+      const int w = w0 + i;
+      if (w >= a.words_per_fiber)
         break;
-      }
-      const unsigned e = emask & (0u - emask);   // the first substep that ends the phase
-      stim |= smask & (e - 1u);
-      last = next;
-      double jf = 0.0;
-      if (a.n_jitter > 0)
-        jf = a.jitter[(int64_t)f * a.n_jitter + jidx % a.n_jitter];
-      jit = xmul(jf, freq);
-      jidx++;
-      next = xadd(last, xdiv(1.0, xadd(freq, jit)));
-      todo &= ~(e | (e - 1u));
-    }
-    if (stim && first_bit < 0)
-      first_bit = w * 32 + __ffs(stim) - 1;
-    if (a.log_count) {
-      // StimulationLogging::logStimulationBegin at the first stimulating decision (compute.tpp:603-607), in
-      // substep order
-      for (unsigned m = stim; m; m &= m - 1u) {
-        const int l = __ffs(m) - 1;
-        const unsigned before = vmask & ((1u << l) - 1u);
-        const bool prev = before ? ((stim >> (31 - __clz(before))) & 1u) : cur;
-        if (!prev && lane == l) {
-          const unsigned long long idx = atomicAdd(a.log_count, 1ull);
-          if (idx < (unsigned long long)a.log_capacity) {
-            a.log_time[idx] = t;
-            a.log_fiber[idx] = f;
-          }
+      const bool valid = valids[i], fires = fire[i];
+      const double t = times[i];
+      const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+      unsigned todo = vmask;   // the bits not decided yet
+      unsigned stim = 0u;
+      while (todo) {
+        const bool check = valid && t >= next && t >= begin;
+        const bool ends = check && repeat != 0 && xsub(t, next) > repeat;
+        const unsigned emask = __ballot_sync(0xffffffffu, ends) & todo;
+        const unsigned smask = __ballot_sync(0xffffffffu, check && fires) & todo;
+        if (!emask) {
+          stim |= smask;
+          break;
         }
-        __syncwarp();
+        const unsigned e = emask & (0u - emask);   // the first substep that ends the phase
+        stim |= smask & (e - 1u);
+        last = next;
+        double jf = 0.0;
+        if (a.n_jitter > 0)
+          jf = a.jitter[(int64_t)f * a.n_jitter + jidx % a.n_jitter];
+        jit = xmul(jf, freq);
+        jidx++;
+        next = xadd(last, xdiv(1.0, xadd(freq, jit)));
+        todo &= ~(e | (e - 1u));
       }
-    }
-    if (vmask)
-      cur = (stim >> (31 - __clz(vmask))) & 1u;
-    if (lane == (w & 31))
-      out = stim;
-    if ((w & 31) == 31 || w == a.words_per_fiber - 1) {
-      const int wl = (w & ~31) + lane;
-      if (wl <= w)
-        fl[wl] = out;
+      if (stim && first_bit < 0)
+        first_bit = w * 32 + __ffs(stim) - 1;
+      if (a.log_count) {
+        // StimulationLogging::logStimulationBegin at the first stimulating decision (compute.tpp:603-607), in
+        // substep order
+        for (unsigned m = stim; m; m &= m - 1u) {
+          const int l = __ffs(m) - 1;
+          const unsigned before = vmask & ((1u << l) - 1u);
+          const bool prev = before ? ((stim >> (31 - __clz(before))) & 1u) : cur;
+          if (!prev && lane == l) {
+            const unsigned long long idx = atomicAdd(a.log_count, 1ull);
+            if (idx < (unsigned long long)a.log_capacity) {
+              a.log_time[idx] = t;
+              a.log_fiber[idx] = f;
+            }
+          }
+          __syncwarp();
+        }
+      }
+      if (vmask)
+        cur = (stim >> (31 - __clz(vmask))) & 1u;
+      if (lane == (w & 31))
+        out = stim;
+      if ((w & 31) == 31 || w == a.words_per_fiber - 1) {
+        const int wl = (w & ~31) + lane;
+        if (wl <= w)
+          fl[wl] = out;
+      }
     }
   }
   if (gate) {
