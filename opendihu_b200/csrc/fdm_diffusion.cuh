@@ -41,29 +41,32 @@ struct ElementTerms {
 // A tile of FACTOR_TILE nodes lives in shared memory (longer fibers: tile after tile, in FACTOR_SOLVE with d' and cp
 // in scratch between the two sweeps).  Threads hold an odd number of consecutive nodes, so that their shared-memory
 // accesses, that many doubles apart, meet no bank twice.
-// Bound by FP64 work (two divisions per element, two to three per node with the warm-up) and latency; a thread per
-// fiber, with six divisions and six uncoalesced stores per node, took 2519 us for the factorization of 4096 fibers of
-// 500 to 2500 nodes and a solve 524 us more; FACTOR_SOLVE does both in 214 us.  (64 fibers of 1481 nodes: 1129 us,
-// now 8.)
+// Bound by FP64 work (two divisions per element, two to three per node with the warm-up) and latency, so what counts is
+// that three CTAs share an SM: three arrays of a tile in shared memory, the reciprocals of the chain's divisions kept for
+// the sweeps, the branch-free division.  A thread per fiber, with six divisions and six uncoalesced stores per node, took
+// 2519 us for the factorization of 4096 fibers of 500 to 2500 nodes and a solve 524 us more; FACTOR_SOLVE does both in
+// 169 us (214 with four arrays, CUDA's division and another reciprocal per node).  (Factorization of 64 fibers of 1481
+// nodes: 1129 us, now 8.)
 constexpr int FACTOR_T = 256;
 constexpr int FACTOR_M = 11;          // most nodes per thread (odd)
 constexpr int FACTOR_TILE = 2560;
 constexpr int FACTOR_WARMUP = 12;
 enum FactorWhat { FACTOR, FACTOR_SOLVE };
 
-inline size_t factor_smem_bytes(int tile) { return sizeof(double) * (size_t)(2 * (tile + 1) + 2 * tile); }
+constexpr int FACTOR_PER = FACTOR_TILE / FACTOR_T;   // most nodes per thread of the assembly
+
+inline size_t factor_smem_bytes(int tile) { return sizeof(double) * (size_t)(2 * (tile + 1) + tile); }
 
 template<int WHAT>
-__global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
+__global__ void __launch_bounds__(FACTOR_T, 3) diffusion_factor_kernel(
     const int64_t* __restrict__ fiber_offsets, const double* __restrict__ element_lengths,
     const double* __restrict__ prefactor, double dt, int implicit_euler, double* __restrict__ coef, int64_t stride,
     double* __restrict__ vm, double* __restrict__ scratch, int tile)
 {
   extern __shared__ double smem[];
-  double* ek = smem;             // tile + 1: element left of local node i at i, right of it at i + 1
-  double* em = ek + tile + 1;    // tile + 1
-  double* sb = em + tile + 1;    // tile: diagonal (FACTOR_SOLVE: then the solution)
-  double* sr = sb + tile;        // tile: right-hand side (FACTOR: then cp)
+  double* so = smem;             // tile + 1: off-diagonal of the element left of local node i at i (first its k)
+  double* sb = so + tile + 1;    // tile + 1: diagonal of node i (first the element's m)
+  double* sr = sb + tile + 1;    // tile: FACTOR_SOLVE: right-hand side, then d', then the solution; FACTOR: cp
   __shared__ double sexit[FACTOR_T];
   __shared__ double sF[2 * (FACTOR_T / 32)], sG[2 * (FACTOR_T / 32)];
   const int f = blockIdx.x;
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
   const double pf = prefactor[f];
   const ElementTerms et(dt, implicit_euler);
   double carry_cp = 0.0, carry_d = 0.0;
-  double cp[FACTOR_M], den[FACTOR_M];
+  double cp[FACTOR_M], inv[FACTOR_M];
   for (int64_t base = 0; base < n; base += tile) {
     const int cnt = (int)min((int64_t)tile, n - base);
     const int m = ((cnt + FACTOR_T - 1) / FACTOR_T) | 1;
@@ -82,40 +85,66 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
       const int64_t g = base - 1 + e;
       const bool ok = g >= 0 && g < n - 1;
       const double hh = ok ? h[g] : 1.0;
-      ek[e] = ok ? 1. / hh * pf : 0.0;
-      em[e] = ok ? hh / 6 : 0.0;
+      so[e] = ok ? fdm_rcp64(hh) * pf : 0.0;
+      sb[e] = ok ? fdm_div64(hh, 6.0) : 0.0;
     }
     __syncthreads();
-    for (int i = tid; i < cnt; i += FACTOR_T) {
-      sb[i] = et.diag(ek[i], em[i]) + et.diag(ek[i + 1], em[i + 1]);
-      if (WHAT == FACTOR_SOLVE) {
-        const int64_t v = base + i;
+    double off[FACTOR_PER], diag[FACTOR_PER];
+    double last_off = 0.0;
+#pragma unroll
+    for (int j = 0; j < FACTOR_PER; j++) {
+      const int i = tid + j * FACTOR_T;
+      if (i >= cnt)
+        continue;
+      const double k0 = so[i], m0 = sb[i], k1 = so[i + 1], m1 = sb[i + 1];
+      off[j] = et.off(k0, m0);
+      diag[j] = et.diag(k0, m0) + et.diag(k1, m1);
+      if (i == cnt - 1)
+        last_off = et.off(k1, m1);
+      const double l = et.rhs_off(k0, m0), c = et.rhs_diag(k0, m0) + et.rhs_diag(k1, m1), r = et.rhs_off(k1, m1);
+      const int64_t v = base + i;
+      if (WHAT == FACTOR) {
+        coef[3 * stride + o + v] = l;
+        coef[4 * stride + o + v] = c;
+        coef[5 * stride + o + v] = r;
+      } else {
         const double um = v > 0 ? vm[o + v - 1] : 0.0, up = v < n - 1 ? vm[o + v + 1] : 0.0;
-        sr[i] = et.rhs_off(ek[i], em[i]) * um +
-                (et.rhs_diag(ek[i], em[i]) + et.rhs_diag(ek[i + 1], em[i + 1])) * vm[o + v] +
-                et.rhs_off(ek[i + 1], em[i + 1]) * up;
+        sr[i] = l * um + c * vm[o + v] + r * up;
       }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < FACTOR_PER; j++) {
+      const int i = tid + j * FACTOR_T;
+      if (i >= cnt)
+        continue;
+      so[i] = off[j];
+      sb[i] = diag[j];
+      if (i == cnt - 1)
+        so[cnt] = last_off;
     }
     __syncthreads();
     // the chunk [lo, hi) of this thread
     const int lo = min(tid * m, cnt), hi = min(lo + m, cnt);
-    auto link = [&](int i, double before, double& d) -> double {
-      d = sb[i] - before * et.off(ek[i], em[i]);
-      return et.off(ek[i + 1], em[i + 1]) / d;
+    auto link = [&](int i, double before, double& reciprocal) -> double {
+      const double d = sb[i] - before * so[i], c = so[i + 1];
+      reciprocal = fdm_rcp64(d);
+      const double q = c * reciprocal;
+      return fma(fma(-d, q, c), reciprocal, q);   // c / d as fdm_div64
     };
     auto chunk = [&](double x) -> double {
 #pragma unroll
       for (int j = 0; j < FACTOR_M; j++)
         if (lo + j < hi) {
-          x = link(lo + j, x, den[j]);
+          x = link(lo + j, x, inv[j]);
           cp[j] = x;
         }
       return x;
     };
     double entry = lo <= FACTOR_WARMUP ? carry_cp : 0.0;
     for (int i = max(0, lo - FACTOR_WARMUP); i < lo; i++) {
-      double d;
-      entry = link(i, entry, d);
+      double r;
+      entry = link(i, entry, r);
     }
     sexit[tid] = chunk(entry);
     __syncthreads();
@@ -139,42 +168,34 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
       __syncthreads();
       for (int i = tid; i < cnt; i += FACTOR_T) {
         const int64_t g = o + base + i;
-        const double a = et.off(ek[i], em[i]);
-        const double inv = 1.0 / (sb[i] - (i > 0 ? sr[i - 1] : carry_cp) * a);
-        coef[0 * stride + g] = base + i > 0 ? -a * inv : 0.0;
-        coef[1 * stride + g] = inv;
+        const double a = so[i];
+        const double r = fdm_rcp64(sb[i] - (i > 0 ? sr[i - 1] : carry_cp) * a);
+        coef[0 * stride + g] = base + i > 0 ? -a * r : 0.0;
+        coef[1 * stride + g] = r;
         coef[2 * stride + g] = base + i < n - 1 ? sr[i] : 0.0;
-        coef[3 * stride + g] = et.rhs_off(ek[i], em[i]);
-        coef[4 * stride + g] = et.rhs_diag(ek[i], em[i]) + et.rhs_diag(ek[i + 1], em[i + 1]);
-        coef[5 * stride + g] = et.rhs_off(ek[i + 1], em[i + 1]);
       }
     } else {
-      // forward sweep: den becomes d'
+      // forward sweep
       Affine acc{1.0, 0.0};
-      double mf[FACTOR_M];
 #pragma unroll
       for (int j = 0; j < FACTOR_M; j++)
-        if (lo + j < hi) {
-          const double inv = 1.0 / den[j];
-          mf[j] = -et.off(ek[lo + j], em[lo + j]) * inv;
-          den[j] = inv * sr[lo + j];
-          acc = compose(acc, Affine{mf[j], den[j]});
-        }
+        if (lo + j < hi)
+          acc = compose(acc, Affine{-so[lo + j] * inv[j], inv[j] * sr[lo + j]});
       Affine total;
       const Affine pre = block_scan_map<FACTOR_T, false>(acc, sF, sG, &total);
       double d = fma(pre.F, carry_d, pre.G);
 #pragma unroll
       for (int j = 0; j < FACTOR_M; j++)
         if (lo + j < hi) {
-          d = mf[j] * d + den[j];
-          den[j] = d;
+          d = -so[lo + j] * inv[j] * d + inv[j] * sr[lo + j];
+          sr[lo + j] = d;
         }
       carry_d = fma(total.F, carry_d, total.G);
       if (n > tile) {
 #pragma unroll
         for (int j = 0; j < FACTOR_M; j++)
           if (lo + j < hi) {
-            scratch[o + base + lo + j] = den[j];
+            scratch[o + base + lo + j] = sr[lo + j];
             scratch[stride + o + base + lo + j] = cp[j];
           }
       }
@@ -184,7 +205,7 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
       __syncthreads(); // the tile's shared arrays and scan slots are free
   }
   if (WHAT == FACTOR_SOLVE && n > 0) {
-    // back substitution, from the last tile (still in registers) to the first
+    // back substitution, from the last tile (its d' and cp still in place) to the first
     double carry_x = 0.0;
     for (int64_t base = (n - 1) / tile * tile; base >= 0; base -= tile) {
       const int cnt = (int)min((int64_t)tile, n - base);
@@ -194,7 +215,7 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
 #pragma unroll
         for (int j = 0; j < FACTOR_M; j++)
           if (lo + j < hi) {
-            den[j] = scratch[o + base + lo + j];
+            sr[lo + j] = scratch[o + base + lo + j];
             cp[j] = scratch[stride + o + base + lo + j];
           }
       }
@@ -202,7 +223,7 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
 #pragma unroll
       for (int j = FACTOR_M - 1; j >= 0; j--)
         if (lo + j < hi)
-          acc = compose(acc, Affine{-cp[j], den[j]});
+          acc = compose(acc, Affine{-cp[j], sr[lo + j]});
       Affine total;
       const Affine pre =
           block_scan_map<FACTOR_T, true>(acc, sF + FACTOR_T / 32, sG + FACTOR_T / 32, &total);
@@ -210,13 +231,13 @@ __global__ void __launch_bounds__(FACTOR_T) diffusion_factor_kernel(
 #pragma unroll
       for (int j = FACTOR_M - 1; j >= 0; j--)
         if (lo + j < hi) {
-          x = -cp[j] * x + den[j];
-          sb[lo + j] = x;
+          x = -cp[j] * x + sr[lo + j];
+          sr[lo + j] = x;
         }
       carry_x = fma(total.F, carry_x, total.G);
       __syncthreads();
       for (int i = tid; i < cnt; i += FACTOR_T)
-        vm[o + base + i] = sb[i];
+        vm[o + base + i] = sr[i];
       if (n > tile)
         __syncthreads();
     }
