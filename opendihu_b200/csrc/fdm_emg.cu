@@ -540,9 +540,9 @@ __global__ void __launch_bounds__(EMG_T, 4) cg_direction_kernel(Grid g, const do
 // With a node per thread and no tiles (mg_jacobi_kernel and so on) every coefficient comes from L2 twice, once
 // for each end of its edge, 312 B per node, which bounds those; here 195 B, of which 144 B are from HBM.  On 97 x 97 x 297
 // nodes a direction pass takes 115 us against 146 (0.56 of the measured copy rate), a V-cycle's passes over the two
-// finest levels 457 against 593.
+// finest levels, both marching, 457 against 593.
 constexpr int ST_T = 352;              // threads: (tx + 2) (ty + 2) <= ST_T
-constexpr int64_t ST_MIN_NODES = 100000;
+constexpr int64_t ST_MIN_NODES = 600000;
 enum StencilOp { ST_RESIDUAL, ST_JACOBI, ST_DIRECTION };
 
 struct StencilTiles {
@@ -1405,7 +1405,9 @@ std::vector<int> coarse_indices(int n)
 }
 
 // the tiles of a grid's stencil passes; grids below ST_MIN_NODES, which have too few planes and
-// columns for the chip, take the node-per-thread passes
+// columns for the chip, take the node-per-thread passes.  Per iteration, marching against a thread per node: Jacobi,
+// 114,345 nodes 21.5 us against 18.0, 384,160 36.4 / 34.6, 720,000 56.2 / 55.1, 1,408,000 94 / 99; multigrid 147 / 134,
+// 243 / 237, 333 / 341, 524 / 557.
 int choose_tiles(fdm_emg* m, const Grid& g, StencilTiles* tiles)
 {
   *tiles = StencilTiles{};

@@ -54,8 +54,9 @@ def test_jacobi_residual(shape):
 
 
 # tiles that do and do not divide the grid, a single tile, more tiles than planes, a thin grid
-@pytest.mark.parametrize("shape", [(101, 37, 29), (33, 65, 49), (16, 18, 360), (350, 150, 2), (2, 300, 190),
-                                   (1100, 3, 40)])
+# (the march along z takes grids from 600,000 nodes, the last six)
+@pytest.mark.parametrize("shape", [(101, 37, 29), (16, 18, 360), (2, 300, 190), (101, 97, 65), (65, 97, 97),
+                                   (16, 18, 2100), (550, 560, 2), (2, 500, 610), (1100, 3, 190)])
 def test_multigrid_residual(shape):
     with _solver(shape, "multigrid", 1e-8) as s:
         vm = np.random.default_rng(1).uniform(-80.0, 40.0, s.n_nodes)
