@@ -454,38 +454,6 @@ __device__ __forceinline__ void heun_step2_pairs(fdm_f2 (&Vf)[MP], fdm_f2 (&LV)[
   }
 }
 
-// heun_step2 for one node alone (scalar FP32): the same carrying of Vm and the states within a half step, against a Fast2Sum
-// per state and substep and the conversions and FP64 additions of Vm in heun_step.  In cluster mode, one node per
-// thread, that shortens the chain that bounds the step: 5.32 -> 5.18 us per Strang step (16 x 1481 fibers).
-template<class Model>
-__device__ __forceinline__ void heun_step1(float& Vf, float& LV, double& V, const float* __restrict__ S,
-                                           float* __restrict__ L, const float* __restrict__ P, float t, float dt,
-                                           bool clamp, double vstim)
-{
-  constexpr int NS = Model::nStates;
-  float y[NS], r[NS], ys[NS], r2[NS], alg[Model::nAlgebraics];
-  y[0] = Vf + LV;
-#pragma unroll
-  for (int s = 1; s < NS; s++)
-    y[s] = S[s - 1] + L[s - 1];
-  Model::template rates_fast<float, fdm_math_exact>(t, y, P, r, alg);
-#pragma unroll
-  for (int s = 0; s < NS; s++)
-    ys[s] = fmaf(dt, r[s], y[s]);
-  if (clamp)
-    ys[0] = (float)vstim;
-  Model::template rates_fast<float, fdm_math_exact>(t, ys, P, r2, alg);
-#pragma unroll
-  for (int s = 1; s < NS; s++)
-    L[s - 1] = fmaf(0.5f * dt, r[s] + r2[s], L[s - 1]);
-  LV = fmaf(0.5f * dt, r[0] + r2[0], LV);
-  if (clamp) {
-    V = vstim;
-    Vf = (float)vstim;
-    LV = 0.f;
-  }
-}
-
 // (S, L) -> (S + L rounded, the rounding error): the Fast2Sum normalization of a compensated pair
 __device__ __forceinline__ void normalize_pair(fdm_f2& S, fdm_f2& L)
 {
@@ -1767,21 +1735,10 @@ __global__ void __launch_bounds__(CLUSTER ? T + 64 : T, 1) fused_kernel(FusedArg
       }
     }
   };
-  // FP32: Vm of an odd last node over the half step, as of the pairs
-  constexpr bool LONE = PAIR && M % 2 == 1;
-  float Vf1 = 0.f, LV1 = 0.f;
   // one Heun substep of a node that runs alone
   auto scalar_node = [&](int j, double t, double dt0, int bit) {
     const bool stim = node_stim(j, bit);
-    if constexpr (LONE) {
-      const bool current = stim && a.stimulus_mode == 1;
-      float Pk[NP];
-#pragma unroll
-      for (int p = 0; p < NP; p++)
-        Pk[p] = current && p == a.stimulus_parameter ? (float)a.stimulus_value : (float)P[M - 1][p];
-      heun_step1<Model>(Vf1, LV1, V[M - 1], (const float*)S[M - 1], (float*)L[M - 1], Pk, (float)t, (float)dt0,
-                        stim && a.stimulus_mode == 0, a.vstim);
-    } else if (stim && a.stimulus_mode == 1) {
+    if (stim && a.stimulus_mode == 1) {
       // stimulus current: the junction nodes see the stimulus parameter while stimulated
       RR Pk[NP];
 #pragma unroll
@@ -1863,10 +1820,6 @@ __global__ void __launch_bounds__(CLUSTER ? T + 64 : T, 1) fused_kernel(FusedArg
           Vf[p] = fdm_f2((float)V[2 * p], (float)V[2 * p + 1]);
           LV[p] = fdm_f2(0.f, 0.f);
         }
-      }
-      if constexpr (LONE) {
-        Vf1 = (float)V[M - 1];
-        LV1 = 0.f;
       }
 #pragma unroll 1
       for (int k = 0; k < (halo < 0 ? k_end : 0); k++) {
@@ -1987,15 +1940,6 @@ __global__ void __launch_bounds__(CLUSTER ? T + 64 : T, 1) fused_kernel(FusedArg
 #pragma unroll
           for (int q = 0; q < NSM; q++)
             normalize_pair(S2[p][q], L2[p][q]);
-        }
-        if constexpr (LONE) {
-          V[M - 1] += (double)LV1;
-#pragma unroll
-          for (int q = 0; q < NSM; q++) {
-            const RR sum = S[M - 1][q] + L[M - 1][q];
-            L[M - 1][q] = L[M - 1][q] - (sum - S[M - 1][q]);
-            S[M - 1][q] = sum;
-          }
         }
         if constexpr (!gate_on) {
           // nodes beyond the bin carry Vm = 0 into the diffusion (zero coefficients, finite values); only the
