@@ -337,8 +337,8 @@ __global__ void __launch_bounds__(DIFFUSION_T) diffusion_reg_kernel(const int64_
 // the factors in registers, and the others fetch theirs back: two cluster barriers per step.  Same functions and
 // partition as the kernels it stands in for, so the same values whichever form the number of fibers leads to.
 // Bound by the latency of a node's Heun chain, 1.6 us of the 1.8 + 1.6 n0 us per step at n0 substeps a half step.  16
-// fibers of 1481 nodes (clusters of 6), 400 steps: 7.06 -> 4.38 ms; one of 101 nodes, 50 steps: 588 -> 412 us; 74 of 500:
-// 13.2 -> 8.8 us per step.
+// fibers of 1481 nodes (clusters of 6), 400 steps: 7.06 -> 4.38 ms; one of 101 nodes, 50 steps: 588 -> 412 us; 74 of
+// 500: 13.2 -> 8.8 us per step.
 constexpr int WINDOW_T = DIFFUSION_T;
 
 template<class Model, class Math, int M>

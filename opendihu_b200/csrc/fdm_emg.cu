@@ -532,14 +532,14 @@ __global__ void __launch_bounds__(EMG_T, 4) cg_direction_kernel(Grid g, const do
 }
 
 // ---- the stencil passes of large grids, marching along z ---------------------------------------------------
-// A CTA owns a tile of tx x ty columns and a thread per column of the tile and of the ring around it; it walks a chunk of
-// planes.  Of each node every coefficient is read once per tile: the thread multiplies its 13 forward coefficients with
+// A CTA owns a tile of tx x ty columns and a thread per column of the tile and of the ring around it; it walks a chunk
+// of planes.  Of each node every coefficient is read once per tile: the thread multiplies its 13 forward coefficients with
 // its own value and leaves the products in shared memory, where the nodes they lead to collect them (the five of
 // the same plane at once, the nine towards the next plane as the carry of its nodes), and adds its own forward part
 // with the values of the planes z and z + 1.  The next plane's coefficients are loaded meanwhile.
 // With a node per thread and no tiles (mg_jacobi_kernel and so on) every coefficient comes from L2 twice, once
-// for each end of its edge, 312 B per node, which bounds those; here 195 B, of which 144 B are from HBM.  On 97 x 97 x 297
-// nodes a direction pass takes 115 us against 146 (0.56 of the measured copy rate), a V-cycle's passes over the two
+// for each end of its edge, 312 B per node, which bounds those; here 195 B, of which 144 B are from HBM.  On
+// 97 x 97 x 297 nodes a direction pass takes 115 us against 146 (0.56 of the measured copy rate), a V-cycle's passes over the two
 // finest levels, both marching, 457 against 593.
 constexpr int ST_T = 352;              // threads: (tx + 2) (ty + 2) <= ST_T
 constexpr int64_t ST_MIN_NODES = 600000;
@@ -720,8 +720,8 @@ __global__ void __launch_bounds__(EMG_T) cg_update_kernel(int64_t N, double* __r
 // product every z is written).  Three sets of slots rotate: a CTA clears its slot of the previous sum's set once the
 // current sum is complete (everyone has left the previous one), two sums before it is filled again.  A CTA waits at
 // most CGP_SPINS polls, then the kernel ends with CGP_TIMED_OUT.
-// Bound by latency (two grid-wide sums per iteration).  Per iteration, against two launches: 1701 nodes 10.8 us (13.5), 28,033
-// 10.7 (12.9), 93,125 11.7 (17.3), 113,256 12.3 (17.4).
+// Bound by latency (two grid-wide sums per iteration).  Per iteration, against two launches: 1701 nodes 10.8 us (13.5),
+// 28,033 10.7 (12.9), 93,125 11.7 (17.3), 113,256 12.3 (17.4).
 constexpr int CGP_T = 768;
 constexpr int CGP_REG = 10;                       // centre and forward coefficients in registers
 constexpr int CGP_SM = 13 + EMG_NC - CGP_REG;     // the others in shared memory: backward, then forward
@@ -761,7 +761,7 @@ __device__ __forceinline__ double cgp_cta_sum(double v, double* red)
   return v;
 }
 
-// K (1 or 2) sums over all CTAs (the same in all threads of all CTAs); false if the wait ran out.  K gridDim.x <= CGP_T
+// K (1 or 2) sums over all CTAs (the same in all threads); false if the wait ran out.  K gridDim.x <= CGP_T
 template<int K>
 __device__ bool cgp_grid_sum(double (&v)[K], const CgpArgs& a, int phase, double (*red)[CGP_T / 32], int* abort)
 {

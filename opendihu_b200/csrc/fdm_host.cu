@@ -3281,7 +3281,8 @@ extern "C" int fdm_adjoint_forward(fdm_solver* s, double t_start, double t_end, 
   plan_advance(s, t_start, t_end, A.steps, A.dt1s);
   const int64_t NT = (int64_t)A.steps.size();
   // A run of the last run's shape (an optimization loop) keeps its checkpoints and tapes: freeing and allocating the
-  // several GB of them took 10 of 26 ms (64 x 1481 fibers, 100 steps).  Any other shape starts from nothing, so no more is held than it needs.
+  // several GB of them took 10 of 26 ms (64 x 1481 fibers, 100 steps).  Any other shape starts from nothing, so no
+  // more is held than it needs.
   bool same = A.kc > 0 && last_kc == checkpoint_every && last_steps.size() == A.steps.size();
   for (size_t j = 0; same && j < A.steps.size(); j++)
     same = last_steps[j].n0 == A.steps[j].n0;

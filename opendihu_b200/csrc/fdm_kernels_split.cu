@@ -259,10 +259,10 @@ int clusters_with_own_sms(int csize)
   return n;
 }
 
-// The few fibers a window kernel is for: a CTA for at most WINDOW_T nodes and an SM for every CTA; the most CTAs per fiber
-// (at most 8, down to 128 nodes each) with which that holds.  Where CTAs share an SM, the launches cost less than that:
-// per step of 5 substeps a half step 16 fibers of 1481 nodes take 10.6 us with clusters of 6, 19.7 with clusters of 8 (one
-// more than fit) and 15.0 with a launch per half step and solve; 24 fibers 20.3 with clusters of 6 (22 fit) and 14.9.
+// The few fibers a window kernel is for: a CTA for at most WINDOW_T nodes and an SM for every CTA; the most CTAs per
+// fiber (at most 8, down to 128 nodes each) with which that holds.  Where CTAs share an SM, the launches cost less than that:
+// per step of 5 substeps a half step 16 fibers of 1481 nodes take 10.6 us with clusters of 6, 19.7 with clusters of 8
+// (one more than fit) and 15.0 with a launch per half step and solve; 24 fibers 20.3 with clusters of 6 (22 fit) and 14.9.
 int window_cluster_size(int model, int n_fibers, int64_t max_fiber_len)
 {
   const int least = (int)std::min<int64_t>((max_fiber_len + WINDOW_T - 1) / WINDOW_T, FDM_MAX_CLUSTER + 1);
