@@ -734,8 +734,8 @@ static int choose_cluster(fdm_solver* s, int regular_bins, int* csize_out)
       continue;
     }
     // prefer: all CTAs resident at once with an SM each, fewer nodes per thread, then more CTAs.  (16 fibers of 1481
-    // nodes: clusters of 8, of which 15 fit, 5.61 us per step in FP32 and 18.1 in FP64; clusters of 6 with 256
-    // threads, of which 22 fit, 4.38 and 9.66.)
+    // nodes: clusters of 8, of which 15 fit, 5.71 us per step in FP32 and 18.1 in FP64; clusters of 6 with 256
+    // threads, of which 22 fit, 4.87 and 9.60.  24 fibers: those 9.28 and 18.7, 3 CTAs of 256 x 2 5.12 and 16.8.)
     const int64_t ctas = (int64_t)s->n_fibers * cs;
     const bool resident = s->n_fibers <= clusters_with_own_sms((int)cs);
     const int64_t key = (resident ? 0 : (int64_t)1 << 40) + ((int64_t)sh[i].nodes_per_thread << 20) - ctas;
