@@ -1,6 +1,5 @@
 // Fused-kernel instantiations for one (precision, math policy); included by fdm_fused_*.cu.
 #pragma once
-#include <atomic>
 #include "fdm_internal.h"
 
 #include "generated/hodgkin_huxley_1952_anone_c2_3_4.cuh"
@@ -34,24 +33,6 @@ cudaError_t launch_fused_hh_f64_exact_gate(int shape, const FusedArgs& a, cudaSt
 cudaError_t launch_fused_hh_f64_approx_gate(int shape, const FusedArgs& a, cudaStream_t s);
 cudaError_t launch_fused_hh_f32_exact_gate(int shape, const FusedArgs& a, cudaStream_t s);
 cudaError_t launch_fused_hh_f32_approx_gate(int shape, const FusedArgs& a, cudaStream_t s);
-
-// The dynamic shared memory limit of a kernel is set per device: once on each device (bit d of done; the
-// solvers of several devices may launch from concurrent host threads).
-template<class K>
-static cudaError_t set_smem_once(K kernel, size_t smem, std::atomic<uint64_t>& done)
-{
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess)
-    return e;
-  const uint64_t bit = dev < 64 ? (uint64_t(1) << dev) : 0;
-  if (bit && (done.load(std::memory_order_acquire) & bit))
-    return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && bit)
-    done.fetch_or(bit, std::memory_order_acq_rel);
-  return e;
-}
 
 template<class Model, class RR, class Math, int T, int M, bool GATE>
 static cudaError_t fused_one(const FusedArgs& a, cudaStream_t s)

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 
 #include "fdm_kernels.cuh"
@@ -13,6 +14,24 @@ namespace fdm {
 
 // records msg as the message fdm_last_error(NULL) returns on this thread; returns code
 int fdm_report_error(int code, const std::string& msg);
+
+// The dynamic shared memory limit of a kernel is set per device: once on each device (bit d of done; the
+// solvers of several devices may launch from concurrent host threads).
+template<class K>
+static cudaError_t set_smem_once(K kernel, size_t smem, std::atomic<uint64_t>& done)
+{
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess)
+    return e;
+  const uint64_t bit = dev < 64 ? (uint64_t(1) << dev) : 0;
+  if (bit && (done.load(std::memory_order_acquire) & bit))
+    return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && bit)
+    done.fetch_or(bit, std::memory_order_acq_rel);
+  return e;
+}
 
 enum MathKind { MATH_EXACT = 0, MATH_APPROX = 1 };
 enum RealKind { REAL_F64 = 0, REAL_F32 = 1 };

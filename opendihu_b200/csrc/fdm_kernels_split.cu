@@ -114,12 +114,13 @@ static cudaError_t factor_launch(int n_fibers, int tile, const int64_t* fiber_of
 {
   if (n_fibers == 0)
     return cudaSuccess;
-  const size_t smem = factor_smem_bytes(tile);
-  const cudaError_t e = cudaFuncSetAttribute(diffusion_factor_kernel<WHAT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+  // the limit is the largest tile's, whatever this launch asks for: other solvers of the device, in other host threads,
+  // launch the kernel with tiles of their own
+  static std::atomic<uint64_t> attr_done{0};
+  const cudaError_t e = set_smem_once(diffusion_factor_kernel<WHAT>, factor_smem_bytes(FACTOR_TILE), attr_done);
   if (e != cudaSuccess)
     return e;
-  diffusion_factor_kernel<WHAT><<<(unsigned)n_fibers, FACTOR_T, smem, s>>>(
+  diffusion_factor_kernel<WHAT><<<(unsigned)n_fibers, FACTOR_T, factor_smem_bytes(tile), s>>>(
       fiber_offsets, element_lengths, prefactor, dt, implicit_euler, coef, stride, vm, scratch, tile);
   return cudaGetLastError();
 }

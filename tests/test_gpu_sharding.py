@@ -1,6 +1,9 @@
 """Sharded solves on the GPU: an LPT-sharded system (three shards on one device, concurrent host threads and
 streams) reproduces the unsharded solve, under the layout-dependent "vc" clamp rule too, and its adjoint
 gradients equal the unsharded adjoint's."""
+import concurrent.futures
+import threading
+
 import numpy as np
 import pytest
 
@@ -86,3 +89,31 @@ def test_sequential_shard_adjoint_equals_unsharded():
     np.testing.assert_array_equal(tr2, tr)
     for k in ("prefactor", "parameters", "states0"):
         np.testing.assert_allclose(g2[k], g[k], rtol=1e-12, atol=1e-300)
+
+
+# solvers of one device, their longest fibers different, that factorize again and again from threads of their own: each
+# launches the factorization with shared memory for its own longest fiber
+def test_concurrent_factorizations():
+    go = threading.Barrier(4)
+
+    def refactorize(n_nodes):
+        s = H.complete(S.uniform_fibers(H.HH, [n_nodes] * 3, 0.01, 3.828 / 500, call_frequency=0.1,
+                                        repeat_after_first_call=0.1, call_enable_begin=0.0, end_time=1e-3, dt_0d=5e-4,
+                                        dt_1d=1e-3, dt_splitting=1e-3, dt_repeated_call=1e-3, clamp_rule="center"))
+        first = s.states.copy()
+        pf = np.full(3, 3.828 / 500)
+        with S.FastMonodomainSolver(s, method="split", precision="fp64") as slv:
+            slv.advanceTimeSpan()
+            ref = slv.states()
+            go.wait(60)
+            for _ in range(400):
+                slv.set_states(first)
+                slv.set_prefactor(pf)
+                slv.rewind()
+                slv.setTimeSpan(0.0, 1e-3)
+                slv.advanceTimeSpan()
+            np.testing.assert_array_equal(slv.states(), ref)
+        return n_nodes
+
+    with concurrent.futures.ThreadPoolExecutor(4) as ex:
+        assert list(ex.map(refactorize, (2500, 2300, 600, 64))) == [2500, 2300, 600, 64]
