@@ -37,6 +37,8 @@ import numbers
 import os
 import re
 from dataclasses import dataclass, field
+from decimal import Decimal, localcontext
+from fractions import Fraction
 from typing import Dict, List, Optional, Sequence, Tuple
 
 # ----------------------------------------------------------------------------------------------
@@ -555,36 +557,37 @@ def _ident(model: Model) -> str:
     return re.sub(r"[^A-Za-z0-9_]", "_", model.name)
 
 
-def _affine(e, consts):
+def _affine(e, consts, number=float):
     """e as (coefficients {(kind, idx): a}, constant b) if it is affine in STATES/PARAMS/VOI with numeric
-    coefficients, else None (CONSTANTS count as numbers: they are folded)."""
+    coefficients, else None (CONSTANTS count as numbers: they are folded).  number: the type to calculate in (float, or
+    Fraction for exact coefficients)."""
     t = e[0]
     if t == "num":
-        return {}, e[2]
+        return {}, number(e[2])
     if t == "var":
         if e[1] == "C":
-            return {}, consts[e[2]]
+            return {}, number(consts[e[2]])
         if e[1] in ("S", "P", "T"):
-            return {(e[1], e[2]): 1.0}, 0.0
+            return {(e[1], e[2]): number(1)}, number(0)
         return None
     if t == "neg":
-        a = _affine(e[1], consts)
+        a = _affine(e[1], consts, number)
         return None if a is None else ({k: -v for k, v in a[0].items()}, -a[1])
     if t == "pos":
-        return _affine(e[1], consts)
+        return _affine(e[1], consts, number)
     if t == "bin" and e[1] in "+-":
-        a = _affine(e[2], consts)
-        b = _affine(e[3], consts)
+        a = _affine(e[2], consts, number)
+        b = _affine(e[3], consts, number)
         if a is None or b is None:
             return None
-        sg = 1.0 if e[1] == "+" else -1.0
+        sg = 1 if e[1] == "+" else -1
         c = dict(a[0])
         for k, v in b[0].items():
-            c[k] = c.get(k, 0.0) + sg * v
+            c[k] = c.get(k, 0) + sg * v
         return c, a[1] + sg * b[1]
     if t == "bin" and e[1] in "*/":
-        a = _affine(e[2], consts)
-        b = _affine(e[3], consts)
+        a = _affine(e[2], consts, number)
+        b = _affine(e[3], consts, number)
         if a is None or b is None:
             return None
         if e[1] == "*":
@@ -941,83 +944,96 @@ class _FastEmitter(_Emitter):
         return out
 
 
-def _exp_shares(lines, consts):
-    """Exponentials of the FP64 form that follow from others: {repr(exp node): (base, square, constant)} with
-    exp node = base * constant, or base^2 * constant, and the list of the bases (exp nodes, evaluated as written).
-    Members of one slope (exp(a.x + b_k)) take the first member as their base, so that the argument's rounding
-    error is that of a member's own argument; a slope that doubles another one takes that one's base squared."""
-    found = {}
+#: ln 2 to 70 digits, for the constants of an exponential's argument reduction
+_LN2_EXACT = Fraction("0.6931471805599453094172321214581765680755001343602552541206800094933936")
 
-    def walk(e):
-        t = e[0]
-        if t == "call":
-            if e[1] == "exp":
-                af = _affine(e[2][0], consts)
-                if af is not None and af[0]:
-                    key = tuple(sorted((k, round(v, 15)) for k, v in af[0].items()))
-                    found.setdefault(key, {}).setdefault(repr(e), (e, af[1]))
-            for a in e[2]:
-                walk(a)
-        elif t in ("neg", "pos", "not"):
-            walk(e[1])
-        elif t == "bin":
-            walk(e[2])
-            walk(e[3])
-        elif t == "tern":
-            for x in e[1:4]:
-                walk(x)
-    for _, _, e in lines:
-        walk(e)
-    shares, bases, base_of = {}, [], {}
 
-    def half_of(key):
-        for other in found:
-            if other != key and len(other) == len(key) and all(
-                    k == k2 and abs(v - 2 * v2) <= 4e-15 * abs(v) for (k, v), (k2, v2) in zip(key, other)):
-                return other
-        return None
+def _exp_scale_text(c: Fraction) -> str:
+    """The constants with which exp(c x) is reduced to exp(r) 2^k (fdm_exp_scale of fdm_math.cuh)"""
+    hi = float(_LN2_EXACT / c)
+    m, e = math.frexp(hi)
+    hi = math.ldexp(math.trunc(math.ldexp(m, 42)), e - 42)
+    values = (float(c), float(c - Fraction(float(c))), float(c / _LN2_EXACT), hi, float(_LN2_EXACT - Fraction(hi) * c))
+    return "fdm_exp_scale{" + ", ".join(_hexf(v) for v in values) + "}"
 
-    def base(key):
-        """(index of the base, its constant term) of a slope whose first member is evaluated"""
-        if key not in base_of:
-            e, b = next(iter(found[key].values()))
-            bases.append(e)
-            base_of[key] = (len(bases) - 1, b)
-            shares[repr(e)] = (len(bases) - 1, False, 1.0)
-        return base_of[key]
 
-    for key, members in found.items():
-        half = half_of(key)
-        # one squaring only: the error of the base doubles with it
-        if half is not None and half_of(half) is None:
-            k, b0 = base(half)
-            for r, (_, b) in members.items():
-                shares[r] = (k, True, math.exp(b - 2 * b0))
-        elif len(members) > 1:
-            k, b0 = base(key)
-            for r, (_, b) in members.items():
-                if r not in shares:
-                    shares[r] = (k, False, math.exp(b - b0))
-    return shares, bases
+def _exp_offset_text(b: Fraction) -> str:
+    """e^b in two parts (fdm_exp_offset of fdm_math.cuh)"""
+    with localcontext() as context:
+        context.prec = 60
+        e = Fraction((Decimal(b.numerator) / Decimal(b.denominator)).exp())
+    return "fdm_exp_offset{" + _hexf(float(e)) + ", " + _hexf(float(e - Fraction(float(e)))) + "}"
 
 
 class _Fast64Emitter(_Emitter):
     """FP64 form of the right-hand side, with the branch-free exponential and division of fdm_math.cuh (FDM_EXP,
-    FDM_DIV).  In FP64 an exponential takes about 20 instructions and a division about 10, also one by a constant,
-    so: products and quotients collect their constants into one factor (a division by
-    a constant becomes a multiplication) and exponentials follow from each other (_exp_shares; None: every
-    exponential evaluated, for approximations of it that do not turn sums into products).  Sums, gate terms and
-    divisions by variables stay as the model writes them."""
+    FDM_EXPM1, FDM_DIV).  In FP64 a division takes about 10 instructions, also one by a constant, so products and
+    quotients collect their constants into one factor (a division by a constant becomes a multiplication).  An exponential
+    takes the constant factor of its argument by itself, which costs nothing and saves the rounding of the product.
+    exp(u) - 1 has a function of its own, exact where it cancels: at the removable singularities of the rates
+    (x / (exp(x) - 1)) the quotient keeps its accuracy.  Exponentials in divisors stay finite; those of one slope, exp(u + b_k)
+    with small b_k, follow from one reduction (fdm_exp_group: in two parts, so that the products with e^b_k lose nothing).
+    Sums, gate terms and divisions by variables stay as the model writes them.
 
-    def __init__(self, real, consts, shares=None):
+    lines: the right-hand side (for the groups); the body of a set of them begins with group_lines(set)."""
+
+    def __init__(self, real, consts, lines=()):
         super().__init__(real, consts, "cuda")
-        self.shares = shares or {}
+        self.in_divisor = False
+        self.bases = []      # per group: the base's argument
+        self.members = {}    # repr(argument) -> (group, offset from the base's argument)
+        slopes = {}
+        for _, _, e in lines:
+            for u, minus_one in self._divisor_exponentials(e, False):
+                c, num, den = self.factors(u)
+                af = _affine(u, consts, Fraction)
+                if af is not None and af[0] and len(num) == 1 and not den and 1e-30 < abs(c) < 1e30:
+                    slopes.setdefault(tuple(sorted(af[0].items())), {}).setdefault(repr(u), (u, af[1], minus_one))
+        for found in slopes.values():
+            # the base: an exponential that 1 is subtracted from, if there is one (it is the most exact member)
+            base, b0, _ = max(found.values(), key=lambda m: m[2])
+            near = {r: b - b0 for r, (_, b, _) in found.items() if abs(b - b0) <= 2}
+            if len(near) > 1:
+                for r, b in near.items():
+                    self.members[r] = (len(self.bases), b)
+                self.bases.append(base)
+
+    def _divisor_exponentials(self, e, inside):
+        """(argument, whether 1 is subtracted) of the exponentials inside divisors of e"""
+        t = e[0]
+        om = _one_minus_exp(e, self.consts) if inside else None
+        if om is not None:
+            yield om[1][2][0], True
+        elif t == "call":
+            if inside and e[1] == "exp":
+                yield e[2][0], False
+            for a in e[2]:
+                yield from self._divisor_exponentials(a, inside)
+        elif t in ("neg", "pos", "not"):
+            yield from self._divisor_exponentials(e[1], inside)
+        elif t == "bin":
+            yield from self._divisor_exponentials(e[2], inside)
+            yield from self._divisor_exponentials(e[3], inside or e[1] == "/")
+        elif t == "tern":
+            for x in e[1:4]:
+                yield from self._divisor_exponentials(x, inside)
+
+    def group_lines(self, exprs, indent="    "):
+        """Declarations of the groups that occur in the expressions"""
+        used = sorted({self.members[repr(u)][0] for e in exprs for u, _ in self._divisor_exponentials(e, False)
+                       if repr(u) in self.members})
+        out = []
+        for g in used:
+            c, num, _ = self.factors(self.bases[g])
+            out.append(f"{indent}const typename M::exp_group fdm_g{g}({self.expr(num[0])}, {_exp_scale_text(c)});")
+        return out
 
     def factors(self, e, inverse=False):
-        """(constant, numerators, denominators) of a product / quotient / negation"""
+        """(constant, numerators, denominators) of a product / quotient / negation, the constant exact"""
         af = _affine(e, self.consts)
-        if af is not None and not af[0] and af[1] != 0.0:
-            return (1.0 / af[1] if inverse else af[1]), [], []
+        if af is not None and not af[0] and af[1] != 0.0 and math.isfinite(af[1]):
+            c = Fraction(af[1])
+            return (1 / c if inverse else c), [], []
         if e[0] in ("neg", "pos"):
             c, n, d = self.factors(e[1], inverse)
             return (-c if e[0] == "neg" else c), n, d
@@ -1025,7 +1041,26 @@ class _Fast64Emitter(_Emitter):
             c1, n1, d1 = self.factors(e[2], inverse)
             c2, n2, d2 = self.factors(e[3], inverse != (e[1] == "/"))
             return c1 * c2, n1 + n2, d1 + d2
-        return (1.0, [], [e]) if inverse else (1.0, [e], [])
+        return (Fraction(1), [], [e]) if inverse else (Fraction(1), [e], [])
+
+    def divisor(self, e):
+        outer, self.in_divisor = self.in_divisor, True
+        text = self.expr(e)
+        self.in_divisor = outer
+        return text
+
+    def exponential(self, name, u):
+        """exp(u), or exp(u) - 1"""
+        c, num, den = self.factors(u)
+        if self.in_divisor and repr(u) in self.members:
+            g, b = self.members[repr(u)]
+            offset = f"{_exp_offset_text(b)}, " if b else ""
+            return f"{name}_OF(fdm_g{g}, {offset}{self.expr(num[0])}, {_exp_scale_text(c)})"
+        if self.in_divisor:
+            name += "_SAT"
+        if len(num) == 1 and not den and c != 1 and 1e-30 < abs(c) < 1e30:
+            return f"{name}({self.expr(num[0])}, {_exp_scale_text(c)})"
+        return f"{name}({self.expr(u)})"
 
     def expr(self, e):
         t = e[0]
@@ -1034,6 +1069,9 @@ class _Fast64Emitter(_Emitter):
             return self.lit(af[1])
         if t in ("neg", "pos") or (t == "bin" and e[1] in "*/"):
             c, num, den = self.factors(e)
+            if not 1e-300 < abs(c) < 1e300:   # as the model writes it: the collected constant is out of range
+                return super().expr(e)
+            c = float(c)
             if not num:
                 text, c = self.lit(c), 1.0
             else:
@@ -1043,82 +1081,45 @@ class _Fast64Emitter(_Emitter):
                 for x in num[1:]:
                     text = f"({text} * {self.expr(x)})"
             for x in den:
-                text = f"FDM_DIV({text}, {self.expr(x)})"
+                text = f"FDM_DIV({text}, {self.divisor(x)})"
             return f"(-{text})" if c == -1.0 else text
-        if t == "bin" and e[1] == "-":
-            # 1 - exp(u), exp(u) - 1 with a derived exponential: exactly 0 where u is, as with the exponential itself
-            om = _one_minus_exp(e, self.consts)
-            if om is not None and repr(om[1]) in self.shares and self.shares[repr(om[1])][1:] != (False, 1.0):
-                d = f"({self.expr(om[1])} - (({self.real})1.0))" if om[0] < 0 else \
-                    f"((({self.real})1.0) - {self.expr(om[1])})"
-                return f"({self.expr(om[1][2][0])} == (({self.real})0.0) ? (({self.real})0.0) : {d})"
-        if t == "call" and e[1] == "exp" and repr(e) in self.shares:
-            k, square, c = self.shares[repr(e)]
-            x = f"fdm_q{k}" if square else f"fdm_x{k}"
-            return x if c == 1.0 else f"({x} * {self.lit(c)})"
+        om = _one_minus_exp(e, self.consts)
+        if om is not None:
+            text = self.exponential("FDM_EXPM1", om[1][2][0])
+            return text if om[0] < 0 else f"(-{text})"
+        if t == "call" and e[1] == "exp":
+            return self.exponential("FDM_EXP", e[2][0])
         return super().expr(e)
 
-    def base_lines(self, bases, used, indent="    "):
-        """Declarations of the bases and squares that the shares in `used` (exp nodes' reprs) need"""
-        out = []
-        need = {self.shares[r][0] for r in used}
-        squares = {self.shares[r][0] for r in used if self.shares[r][1]}
-        for k, e in enumerate(bases):
-            if k in need:
-                out.append(f"{indent}const R fdm_x{k} = FDM_EXP({self.expr(e[2][0])});")
-                if k in squares:
-                    out.append(f"{indent}const R fdm_q{k} = fdm_x{k} * fdm_x{k};")
-        return out
 
-
-def _shares_used(exprs, shares) -> set:
-    """The reprs of the shared exponentials that occur in the expressions"""
-    used = set()
-
-    def walk(e):
-        t = e[0]
-        if t == "call":
-            if repr(e) in shares:
-                used.add(repr(e))
-            for a in e[2]:
-                walk(a)
-        elif t in ("neg", "pos", "not"):
-            walk(e[1])
-        elif t == "bin":
-            walk(e[2])
-            walk(e[3])
-        elif t == "tern":
-            for x in e[1:4]:
-                walk(x)
-    for e in exprs:
-        walk(e)
-    return used
-
-
-_MATH_MACROS = ["#define FDM_EXP(x) M::fast_exp(x)", "#define FDM_DIV(x, y) M::fast_div(x, y)", "#define FDM_LOG(x) M::log(x)", "#define FDM_POWF(x, y) M::pow(x, y)",
-                "#define FDM_ABS(x) fabs(x)", "#define FDM_SQRT(x) sqrt(x)"]
+_MATH_MACROS = ["#define FDM_EXP(...) M::fast_exp(__VA_ARGS__)", "#define FDM_EXPM1(...) M::fast_expm1(__VA_ARGS__)",
+                "#define FDM_EXP_SAT(...) M::fast_exp_sat(__VA_ARGS__)",
+                "#define FDM_EXPM1_SAT(...) M::fast_expm1_sat(__VA_ARGS__)",
+                "#define FDM_EXP_OF(...) M::group_exp(__VA_ARGS__)",
+                "#define FDM_EXPM1_OF(...) M::group_expm1(__VA_ARGS__)",
+                "#define FDM_DIV(x, y) M::fast_div(x, y)", "#define FDM_LOG(x) M::log(x)",
+                "#define FDM_POWF(x, y) M::pow(x, y)", "#define FDM_ABS(x) fabs(x)", "#define FDM_SQRT(x) sqrt(x)"]
+_MATH_UNDEFS = ["#undef " + m.split()[1].split("(")[0] for m in _MATH_MACROS]
 
 
 def emit_rates_f64(lines, consts, pows) -> List[str]:
-    """``rates_f64`` (shared exponentials) and ``rates_f64_plain`` (every exponential evaluated): the FP64 forms."""
+    """``rates_f64``: the FP64 form."""
     out = []
-    for name, shared in (("rates_f64", True), ("rates_f64_plain", False)):
-        shares, bases = _exp_shares(lines, consts) if shared else ({}, [])
-        em = _Fast64Emitter("R", consts, shares)
-        out.append("  template<class R, class M>")
-        out.append(f"  __device__ __forceinline__ static void {name}(const R VOI, const R* __restrict__ STATES,"
-                   " const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)")
-        out.append("  {")
-        out.append("    (void)VOI; (void)PARAMS;")
-        out.extend(_MATH_MACROS)
-        out.extend("#define " + x.split("#define ", 1)[1] for x in _pow_macro_defs(pows))
-        out.extend(em.base_lines(bases, _shares_used([e for _, _, e in lines], shares)))
-        for kind, idx, expr in lines:
-            tgt = f"ALGEBRAIC[{idx}]" if kind == "A" else f"RATES[{idx}]"
-            out.append(f"    {tgt} = {em.expr(expr)};")
-        out.extend(f"#undef FDM_POW{n}" for n in pows)
-        out.append("#undef FDM_EXP\n#undef FDM_DIV\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
-        out.append("  }")
+    em = _Fast64Emitter("R", consts, lines)
+    out.append("  template<class R, class M>")
+    out.append("  __device__ __forceinline__ static void rates_f64(const R VOI, const R* __restrict__ STATES,"
+               " const R* __restrict__ PARAMS, R* __restrict__ RATES, R* __restrict__ ALGEBRAIC)")
+    out.append("  {")
+    out.append("    (void)VOI; (void)PARAMS;")
+    out.extend(_MATH_MACROS)
+    out.extend("#define " + x.split("#define ", 1)[1] for x in _pow_macro_defs(pows))
+    out.extend(em.group_lines([e for _, _, e in lines]))
+    for kind, idx, expr in lines:
+        tgt = f"ALGEBRAIC[{idx}]" if kind == "A" else f"RATES[{idx}]"
+        out.append(f"    {tgt} = {em.expr(expr)};")
+    out.extend(f"#undef FDM_POW{n}" for n in pows)
+    out.extend(_MATH_UNDEFS)
+    out.append("  }")
     return out
 
 
@@ -1171,8 +1172,8 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
         out.append(f"#undef FDM_POW{n}")
     out.append("#undef FDM_EXP\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
     out.append("  }")
-    out.append("  // FP64 forms: constants collected into one factor per product, divisions by constants as")
-    out.append("  // multiplications; rates_f64 with exponentials that follow from others (exact exponentials only)")
+    out.append("  // FP64 form: constants collected into one factor per product, divisions by constants as")
+    out.append("  // multiplications, exp(u) - 1 by a function of its own")
     out.extend(emit_rates_f64(lines, model.constants, pows))
     # FP32 variant with shared exponentials
     repl, groups = _exp_groups(lines, model.constants)
@@ -1227,7 +1228,7 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
     out.append("#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
     out.append("  }")
     # the right-hand side split by state (few-node reaction kernel)
-    out.append("  // the right-hand side of one state at a time: rates_group<R, M, G, SHARED> = RATES[G]")
+    out.append("  // the right-hand side of one state at a time: rates_group<R, M, G> = RATES[G]")
     out.extend(emit_group_rates(model, params_alg, params_const))
     # reverse mode (adjoint)
     out.append("  // vector-Jacobian product: LAM_STATES += J^T LAM_RATES, LAM_PARAMS += (dRATES/dPARAMS)^T LAM_RATES")
@@ -1278,16 +1279,16 @@ MAX_GROUP_STATES = 8
 
 
 def emit_group_rates(model: Model, params_alg: Sequence[int], params_const: Sequence[int]) -> List[str]:
-    """The right-hand side split by state: ``rates_group<R, M, G, SHARED>`` computes RATES[G] only, from the lines
-    its cone needs, so that the warps of a node group can each evaluate one state's rate (the reaction kernel for
+    """The right-hand side split by state: ``rates_group<R, M, G>`` computes RATES[G] only, from the lines its
+    cone needs, so that the warps of a node group can each evaluate one state's rate (the reaction kernel for
     few nodes, where one thread per node leaves the SMs short of independent work).  Same expressions as
-    ``rates_f64`` (SHARED) / ``rates_f64_plain``, so the same values."""
+    ``rates_f64``, so the same values."""
     lines = substitute_parameters(model, params_alg, params_const)
     pows = _collect_int_pows(lines)
     out = [f"  static constexpr int nGroups = {model.n_states if model.n_states <= MAX_GROUP_STATES else 0};"]
     if model.n_states > MAX_GROUP_STATES:
         return out
-    out.append("  template<class R, class M, int G, bool SHARED>")
+    out.append("  template<class R, class M, int G>")
     out.append("  __device__ __forceinline__ static R rates_group(const R VOI, const R* __restrict__ STATES,"
                " const R* __restrict__ PARAMS)")
     out.append("  {")
@@ -1296,30 +1297,26 @@ def emit_group_rates(model: Model, params_alg: Sequence[int], params_const: Sequ
     out.append("    (void)ALGEBRAIC;")
     out.extend(_MATH_MACROS)
     out.extend("#define " + s2.split("#define ", 1)[1] for s2 in _pow_macro_defs(pows))
-    first = True
-    for shared in (True, False):
-        shares, bases = _exp_shares(lines, model.constants) if shared else ({}, [])
-        em = _Fast64Emitter("R", model.constants, shares)
-        for g in range(model.n_states):
-            out.append(f"    {'if' if first else 'else if'} constexpr (G == {g} && {'SHARED' if shared else '!SHARED'}) {{")
-            first = False
-            rate = None
-            cone = rate_cone(lines, [g])
-            out.extend(em.base_lines(bases, _shares_used([lines[n][2] for n in cone], shares), "      "))
-            for n in cone:
-                kind, idx, expr = lines[n]
-                if kind == "A":
-                    out.append(f"      ALGEBRAIC[{idx}] = {em.expr(expr)};")
-                else:
-                    rate = em.expr(expr)
-            out.append(f"      return {rate if rate is not None else '(R)0'};")
-            out.append("    }")
+    em = _Fast64Emitter("R", model.constants, lines)
+    for g in range(model.n_states):
+        out.append(f"    {'if' if g == 0 else 'else if'} constexpr (G == {g}) {{")
+        rate = None
+        cone = rate_cone(lines, [g])
+        out.extend(em.group_lines([lines[n][2] for n in cone], "      "))
+        for n in cone:
+            kind, idx, expr = lines[n]
+            if kind == "A":
+                out.append(f"      ALGEBRAIC[{idx}] = {em.expr(expr)};")
+            else:
+                rate = em.expr(expr)
+        out.append(f"      return {rate if rate is not None else '(R)0'};")
+        out.append("    }")
     out.append("    else {")
     out.append("      return (R)0;")
     out.append("    }")
     for n in pows:
         out.append(f"#undef FDM_POW{n}")
-    out.append("#undef FDM_EXP\n#undef FDM_DIV\n#undef FDM_LOG\n#undef FDM_POWF\n#undef FDM_ABS\n#undef FDM_SQRT")
+    out.extend(_MATH_UNDEFS)
     out.append("  }")
     return out
 

@@ -290,21 +290,18 @@ __device__ __forceinline__ void accumulate(RR& s, RR& l, RR inc)
   }
 }
 
-// right-hand side: the exact-exp modes use the model's shared-exponential forms (FP32: fewest SFU operations;
-// FP64: fewest exponentials and no division by a constant).  The approximate exp is not multiplicative: FP64 takes
-// the form without shared exponentials, FP32 the plain one.
+// right-hand side: FP32 with the exact exponential takes the model's shared-exponential form (fewest SFU operations), with
+// the approximate one, which is not multiplicative, the plain form; FP64 the form without divisions by constants.
 // FP64 is bound by its pipe: one Hodgkin-Huxley right-hand side as the model writes it takes 6 exponentials and 10
-// divisions (7 of them by constants, which the compiler keeps as divisions), here 3 and 3.
-// (reaction_kernel, 1,566,410 nodes, 5 substeps: 283 -> 159 us; Shorten, 53,316 nodes, 25 substeps: 2015 -> 956 us.)
+// divisions (7 of them by constants, which the compiler keeps as divisions), here the
+// work of 4 (three come from one reduction) and 3.
 template<class Model, class RR, class Math>
 __device__ __forceinline__ void model_rates(const RR t, const RR* y, const RR* P, RR* r, RR* alg)
 {
   if constexpr (std::is_same<RR, float>::value && std::is_same<Math, fdm_math_exact>::value)
     Model::template rates_fast<RR, Math>(t, y, P, r, alg);
-  else if constexpr (std::is_same<RR, double>::value && std::is_same<Math, fdm_math_exact>::value)
-    Model::template rates_f64<RR, Math>(t, y, P, r, alg);
   else if constexpr (std::is_same<RR, double>::value)
-    Model::template rates_f64_plain<RR, Math>(t, y, P, r, alg);
+    Model::template rates_f64<RR, Math>(t, y, P, r, alg);
   else
     Model::template rates<RR, Math>(t, y, P, r, alg);
 }
@@ -720,7 +717,7 @@ __device__ __forceinline__ double group_rate(int g, double t, const double* y, c
 {
   if constexpr (G < Model::nGroups) {
     if (g == G)
-      return Model::template rates_group<double, Math, G, std::is_same<Math, fdm_math_exact>::value>(t, y, P);
+      return Model::template rates_group<double, Math, G>(t, y, P);
     return group_rate<Model, Math, G + 1>(g, t, y, P);
   } else {
     return 0.0;

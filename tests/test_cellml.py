@@ -1,7 +1,9 @@
 """CellML parser / code generator."""
 import glob
 import os
+import re
 import ctypes as C
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -173,3 +175,29 @@ def test_settings_with_mappings():
     assert list(s.algebraics_for_transfer) == [4]
     # slots of the built variant: i_Stim, g_Na, g_K (g_K keeps its model value 36)
     np.testing.assert_allclose(s.parameters[:, 0], [0.0, 100.0, 36.0])
+
+
+def test_fp64_form_exponentials():
+    # Hodgkin-Huxley in FP64: the three exponentials of slope 1/10 are in divisors and come from one reduction, at offsets 0
+    # (alpha_m), -1.5 (alpha_n) and 0.5 (beta_h); exp(u) - 1 has a function of its own; the other three exponentials stand
+    # alone; in the one-thread form and in the one of a state at a time
+    text = cellml.emit_cuda_model(cellml.builtin_model(H.HH), (), (2, 3, 4))
+    f64 = text[text.index("static void rates_f64("):text.index("// FP32 form")]
+    group = text[text.index("static R rates_group("):text.index("// vector-Jacobian product")]
+    for body, reductions in ((f64, 1), (group, 3)):
+        body = "\n".join(x for x in body.split("\n") if not x.startswith("#"))
+        names = ("M::exp_group", "FDM_EXPM1_OF(", "FDM_EXP_OF(", "FDM_EXP(", "FDM_DIV(")
+        assert [body.count(f) for f in names] == [reductions, 2, 1, 3, 3]
+    for b in (Fraction(-3, 2), Fraction(1, 2)):
+        e, lo = (float.fromhex(x) for x in re.search(r"\{(.*), (.*)\}", cellml._exp_offset_text(b)).groups())
+        assert e == np.exp(float(b)) and cellml._exp_offset_text(b) in f64
+        assert abs(np.longdouble(e) + np.longdouble(lo) - np.exp(np.longdouble(float(b)))) <= 1.1e-19 * e
+
+
+def test_exponentials_far_apart_share_nothing():
+    # offsets above 2 and exponentials outside divisors stand alone
+    lines = [("R", 0, cellml.parse_expression("1.0/(1.0+exp(STATES[0]))+1.0/(1.0+exp(STATES[0]+2.5))+exp(STATES[0]+1.0)")),
+             ("R", 1, cellml.parse_expression("1.0/(1.0+exp(2.0*STATES[0]))+1.0/(2.0+exp(2.0*STATES[0]-1.0))"))]
+    em = cellml._Fast64Emitter("R", [], lines)
+    assert em.bases == [lines[1][2][2][3][3][2][0]]
+    assert sorted(b for _, b in em.members.values()) == [-1, 0]
