@@ -975,11 +975,24 @@ class _Fast64Emitter(_Emitter):
     with small b_k, follow from one reduction (fdm_exp_group: in two parts, so that the products with e^b_k lose nothing).
     Sums, gate terms and divisions by variables stay as the model writes them.
 
-    lines: the right-hand side (for the groups); the body of a set of them begins with group_lines(set)."""
+    FDM_DIV takes no divisor that is 0, infinite or subnormal.  It stands where the divisor's range follows from the
+    equations (1 + exp(u) with exponentials held finite, see range) and the dividend and the quotient are finite, and for
+    x/(exp(c x) - 1), where dividend and divisor vanish together (FDM_DIV0).  Every other division takes any divisor
+    (FDM_DIV_ANY).
+
+    lines: the right-hand side (for the groups and ranges); the body of a set of them begins with group_lines(set)."""
+
+    LARGEST = 2.0 ** 1023      # of a divisor
+    SMALLEST = 2.0 ** -1000
+    VARIABLE = 2.0 ** 400      # taken as the bound of states, parameters and time
 
     def __init__(self, real, consts, lines=()):
         super().__init__(real, consts, "cuda")
         self.in_divisor = False
+        self.algebraic = {}  # ranges of the algebraic variables
+        for kind, idx, e in lines:
+            if kind == "A":
+                self.algebraic[idx] = self.range(e)
         self.bases = []      # per group: the base's argument
         self.members = {}    # repr(argument) -> (group, offset from the base's argument)
         slopes = {}
@@ -992,14 +1005,117 @@ class _Fast64Emitter(_Emitter):
         for found in slopes.values():
             # the base: an exponential that 1 is subtracted from, if there is one (it is the most exact member)
             base, b0, _ = max(found.values(), key=lambda m: m[2])
-            near = {r: b - b0 for r, (_, b, _) in found.items() if abs(b - b0) <= 2}
+            # (exp(u + b) - 1 of another member is off by some 2^-53: too much where u + b = c (x + d) with a small c d comes
+            # closer to 0 than that)
+            near = {r: b - b0 for r, (u, b, minus_one) in found.items()
+                    if u is base or abs(b - b0) <= 2 and not (minus_one and abs(b) < 4)}
             if len(near) > 1:
                 for r, b in near.items():
                     self.members[r] = (len(self.bases), b)
                 self.bases.append(base)
 
+    @staticmethod
+    def _interval(*values):
+        """(smallest, largest), or None if one of them is not a finite number of moderate size"""
+        if any(v is None or not abs(v) <= _Fast64Emitter.LARGEST for v in values):
+            return None
+        return min(values), max(values)
+
+    def range(self, e, held=False):
+        """Bounds of e for states, parameters and times below VARIABLE, or None if it has none (it may be infinite).
+        held: exponentials are held finite, as in divisors."""
+        t = e[0]
+        af = _affine(e, self.consts)
+        if af is not None and not af[0]:
+            return self._interval(af[1])
+        om = _one_minus_exp(e, self.consts)
+        if om is not None:
+            return ((-1.0, 2.0 ** 1020) if om[0] < 0 else (-2.0 ** 1020, 1.0)) if held else None
+        if t == "var":
+            return self.algebraic.get(e[2]) if e[1] == "A" else (-self.VARIABLE, self.VARIABLE)
+        if t == "pos":
+            return self.range(e[1], held)
+        if t == "neg":
+            r = self.range(e[1], held)
+            return None if r is None else (-r[1], -r[0])
+        if t == "bin" and e[1] in "+-":
+            x, y = self.range(e[2], held), self.range(e[3], held)
+            if x is None or y is None:
+                return None
+            return self._interval(x[0] + y[0], x[1] + y[1]) if e[1] == "+" else self._interval(x[0] - y[1], x[1] - y[0])
+        if t == "bin" and e[1] in "*/":
+            return self.quotient(e, held)[3]
+        if t == "call" and e[1] == "exp":
+            return (0.0, 2.0 ** 1020) if held else None
+        if t == "call" and e[1] == "pow":
+            n, r = _int_exponent(e[2][1]), self.range(e[2][0], held)
+            if n is None or n < 1 or r is None:
+                return None
+            ends = [_int_pow_value(abs(v), n) * (-1.0 if v < 0 and n % 2 else 1.0) for v in r]
+            return self._interval(*ends, *([0.0] if r[0] < 0 < r[1] else []))
+        if t == "tern":
+            x, y = self.range(e[2], held), self.range(e[3], held)
+            return None if x is None or y is None else self._interval(*x, *y)
+        return None
+
+    def _times(self, x, y):
+        return None if x is None or y is None else self._interval(*(a * b for a in x for b in y))
+
+    def quotient(self, e, held=False):
+        """(constant, numerators, [(divisor, "" or "0": FDM_DIV or FDM_DIV0, None: FDM_DIV_ANY)], range) of a product"""
+        c, num, den = self.factors(e)
+        if not 1e-300 < abs(c) < 1e300:
+            return c, num, None, None
+        ranges = [self.range(x, held) for x in num]
+        product = (float(c), float(c))
+        for r in ranges:
+            product = self._times(product, r)
+        plan = []
+        for x in den:
+            d = self.range(x, True)
+            how = None
+            if d is not None and (d[0] >= self.SMALLEST or d[1] <= -self.SMALLEST):
+                bound = self._times(product, self._interval(1 / d[0], 1 / d[1]))
+                if bound is not None and max(map(abs, bound)) <= 2.0 ** 1022:
+                    how = ""
+                product = bound
+            else:
+                k = self._vanishing(x, num)
+                rest = (float(c), float(c)) if k is not None and not plan else None
+                for i, r in enumerate(ranges):
+                    rest = rest if i == k else self._times(rest, r)
+                if rest is not None:
+                    slope = abs(float(self.factors(_one_minus_exp(self._unsigned(x), self.consts)[1][2][0])[0]))
+                    size = 2 * max(self.VARIABLE, 1 / slope)
+                    product = self._times(rest, (-size, size))
+                    how = "0" if product is not None else None
+                else:
+                    product = None
+            plan.append((x, how))
+        return c, num, plan, product
+
+    @staticmethod
+    def _unsigned(e):
+        while e[0] in ("neg", "pos"):
+            e = e[1]
+        return e
+
+    def _vanishing(self, divisor, num):
+        """The index of the dividend's factor x = y + d, d != 0, if the divisor is exp(c x) - 1 or its negative: x is 0 or
+        far from subnormal"""
+        om = _one_minus_exp(self._unsigned(divisor), self.consts)
+        if om is None:
+            return None
+        c, args, den = self.factors(om[1][2][0])
+        if len(args) != 1 or den or not 1e-30 < abs(c) < 1e30:
+            return None
+        af = _affine(args[0], self.consts)
+        if af is None or not abs(af[1]) >= 1e-30 or any(abs(v) < 1e-30 for v in af[0].values()):
+            return None
+        return next((i for i, x in enumerate(num) if repr(x) == repr(args[0])), None)
+
     def _divisor_exponentials(self, e, inside):
-        """(argument, whether 1 is subtracted) of the exponentials inside divisors of e"""
+        """(argument, whether 1 is subtracted) of the exponentials of e that are held finite"""
         t = e[0]
         om = _one_minus_exp(e, self.consts) if inside else None
         if om is not None:
@@ -1011,9 +1127,19 @@ class _Fast64Emitter(_Emitter):
                 yield from self._divisor_exponentials(a, inside)
         elif t in ("neg", "pos", "not"):
             yield from self._divisor_exponentials(e[1], inside)
+        elif t == "bin" and e[1] in "*/":
+            _, num, plan, _ = self.quotient(e, inside)
+            if plan is None:
+                for x in e[2:4]:
+                    yield from self._divisor_exponentials(x, inside)
+                return
+            for x in num:
+                yield from self._divisor_exponentials(x, inside)
+            for x, how in plan:
+                yield from self._divisor_exponentials(x, how is not None)
         elif t == "bin":
             yield from self._divisor_exponentials(e[2], inside)
-            yield from self._divisor_exponentials(e[3], inside or e[1] == "/")
+            yield from self._divisor_exponentials(e[3], inside)
         elif t == "tern":
             for x in e[1:4]:
                 yield from self._divisor_exponentials(x, inside)
@@ -1034,6 +1160,13 @@ class _Fast64Emitter(_Emitter):
         if af is not None and not af[0] and af[1] != 0.0 and math.isfinite(af[1]):
             c = Fraction(af[1])
             return (1 / c if inverse else c), [], []
+        if e[0] == "call" and e[1] == "pow" and _int_exponent(e[2][1]) is not None:
+            af = _affine(e[2][0], self.consts)   # a power of a constant
+            if af is not None and not af[0] and 1e-30 < abs(af[1]) < 1e30 and abs(_int_exponent(e[2][1])) <= 8:
+                c = Fraction(af[1]) ** _int_exponent(e[2][1])
+                return (1 / c if inverse else c), [], []
+        if inverse and e[0] == "call" and e[1] == "exp":
+            return Fraction(1), [("call", "exp", [("neg", e[2][0])])], []   # 1/exp(u) = exp(-u)
         if e[0] in ("neg", "pos"):
             c, n, d = self.factors(e[1], inverse)
             return (-c if e[0] == "neg" else c), n, d
@@ -1043,8 +1176,8 @@ class _Fast64Emitter(_Emitter):
             return c1 * c2, n1 + n2, d1 + d2
         return (Fraction(1), [], [e]) if inverse else (Fraction(1), [e], [])
 
-    def divisor(self, e):
-        outer, self.in_divisor = self.in_divisor, True
+    def divisor(self, e, held):
+        outer, self.in_divisor = self.in_divisor, held
         text = self.expr(e)
         self.in_divisor = outer
         return text
@@ -1068,20 +1201,24 @@ class _Fast64Emitter(_Emitter):
         if af is not None and not af[0]:
             return self.lit(af[1])
         if t in ("neg", "pos") or (t == "bin" and e[1] in "*/"):
-            c, num, den = self.factors(e)
-            if not 1e-300 < abs(c) < 1e300:   # as the model writes it: the collected constant is out of range
+            c, num, plan, _ = self.quotient(e, self.in_divisor)
+            if plan is None:   # as the model writes it: the collected constant is out of range
                 return super().expr(e)
             c = float(c)
+            last = any(how is None for _, how in plan)   # the constant last: quotients by one divisor are one division
             if not num:
                 text, c = self.lit(c), 1.0
             else:
                 text = self.expr(num[0])
-                if c not in (1.0, -1.0):
+                if c not in (1.0, -1.0) and not last:
                     text = f"({self.lit(c)} * {text})"
                 for x in num[1:]:
                     text = f"({text} * {self.expr(x)})"
-            for x in den:
-                text = f"FDM_DIV({text}, {self.divisor(x)})"
+            for x, how in plan:
+                d = self.divisor(x, how is not None)
+                text = f"FDM_DIV_ANY({text}, {d})" if how is None else f"FDM_DIV{how}({text}, {d})"
+            if c not in (1.0, -1.0) and num and last:
+                text = f"({self.lit(c)} * {text})"
             return f"(-{text})" if c == -1.0 else text
         om = _one_minus_exp(e, self.consts)
         if om is not None:
@@ -1097,7 +1234,9 @@ _MATH_MACROS = ["#define FDM_EXP(...) M::fast_exp(__VA_ARGS__)", "#define FDM_EX
                 "#define FDM_EXPM1_SAT(...) M::fast_expm1_sat(__VA_ARGS__)",
                 "#define FDM_EXP_OF(...) M::group_exp(__VA_ARGS__)",
                 "#define FDM_EXPM1_OF(...) M::group_expm1(__VA_ARGS__)",
-                "#define FDM_DIV(x, y) M::fast_div(x, y)", "#define FDM_LOG(x) M::log(x)",
+                "#define FDM_DIV(x, y) M::fast_div(x, y)", "#define FDM_DIV0(x, y) M::fast_div0(x, y)",
+                "#define FDM_DIV_ANY(x, y) M::fast_div_any(x, y)",
+                "#define FDM_LOG(x) M::log(x)",
                 "#define FDM_POWF(x, y) M::pow(x, y)", "#define FDM_ABS(x) fabs(x)", "#define FDM_SQRT(x) sqrt(x)"]
 _MATH_UNDEFS = ["#undef " + m.split()[1].split("(")[0] for m in _MATH_MACROS]
 

@@ -299,20 +299,52 @@ struct fdm_exp_group {
     return fma(p, o.e, fma(s, o.e_lo, fma(s, o.e, -h)));
   }
 };
-// 1/d by one Halley step (cubic) from the hardware's approximation; a/b with one residual correction of a (1/b).  For
-// normal b below 2^1022 in magnitude; b = 0 and b infinite give NaN.
-__device__ __forceinline__ double fdm_rcp64(double d)
+// 1/d by one Halley step (cubic) from the hardware's approximation: 0.507 ulp; a/b with one residual correction of a (1/b),
+// correctly rounded in 4 million quotients.  For b normal and finite (beyond 2^1022 in magnitude the quotient is 0), a and
+// the quotient finite; b = 0, subnormal or infinite, and a quotient that overflows, give NaN.
+__device__ __forceinline__ double fdm_rcp_approx(double d)
 {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  return y;
+}
+__device__ __forceinline__ double fdm_halley(double d, double y)
+{
   const double e = fma(-d, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
+__device__ __forceinline__ double fdm_rcp64(double d) { return fdm_halley(d, fdm_rcp_approx(d)); }
 __device__ __forceinline__ double fdm_div64(double a, double b)
 {
   const double y = fdm_rcp64(b);
   const double q = a * y;
   return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ bool fdm_is_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
+// a/b as IEEE arithmetic has it for every a and b.  A divisor that is subnormal or at least 2^1021 is scaled together with
+// the dividend; the hardware's approximation of 1/b is infinite for b = 0 and 0 for infinite b and stays as it is then; what
+// the correction turns into NaN (such b, infinite a, a quotient that overflows) is a (1/b) itself.  Shorten's 26 of them
+// (36 x 1481 nodes, 4 steps): 5.76 ms, with CUDA's division 6.55, with fdm_div64, were it allowed, 5.4.
+__device__ __forceinline__ double fdm_div64_any(double a, double b)
+{
+  const int exponent = __double2hiint(b) & 0x7ff00000;
+  const int scale = exponent == 0 ? (1023 + 54) << 20 : (exponent >= 2044 << 20 ? (1023 - 54) << 20 : 1023 << 20);
+  a *= __hiloint2double(scale, 0);
+  b *= __hiloint2double(scale, 0);
+  const double y0 = fdm_rcp_approx(b);
+  const unsigned ye = (unsigned)__double2hiint(y0) & 0x7ff00000u;
+  const double y = ye - (1u << 20) < (2046u << 20) ? fdm_halley(b, y0) : y0;
+  const double q = a * y;
+  const double c = fma(fma(-b, q, a), y, q);
+  return fdm_is_nan(c) ? q : c;
+}
+// 1/d for every d: where the step would give NaN or the result is not normal, the hardware's approximation, infinite for
+// d = 0 and subnormal d, 0 for infinite d and from 2^1022 on.
+__device__ __forceinline__ double fdm_rcp64_any(double d)
+{
+  const double y = fdm_rcp_approx(d);
+  const unsigned exponent = (unsigned)__double2hiint(d) & 0x7ff00000u;
+  return exponent - (1u << 20) < (2044u << 20) ? fdm_halley(d, y) : y;
 }
 
 struct fdm_math_exact {
@@ -330,7 +362,9 @@ struct fdm_math_exact {
     return fdm_expm1_64<true>(x, f);
   }
   __device__ __forceinline__ static double fast_div(double a, double b) { return fdm_div64(a, b); }
-  __device__ __forceinline__ static double fast_rcp(double d) { return fdm_rcp64(d); }
+  __device__ __forceinline__ static double fast_div0(double x, double e) { return fdm_div64(x, e); }
+  __device__ __forceinline__ static double fast_div_any(double a, double b) { return fdm_div64_any(a, b); }
+  __device__ __forceinline__ static double fast_rcp(double d) { return fdm_rcp64_any(d); }
   // exp(c x + b) of a group: g from the group's base; x, f: the argument as a product c x by itself
   using exp_group = fdm_exp_group;
   __device__ __forceinline__ static double group_exp(const exp_group& g, double, const fdm_exp_scale&) { return g.exp(); }
@@ -339,10 +373,11 @@ struct fdm_math_exact {
   {
     return g.exp(o);
   }
-  __device__ __forceinline__ static double group_expm1(const exp_group& g, const fdm_exp_offset& o, double,
+  // (exactly 0 where the argument is)
+  __device__ __forceinline__ static double group_expm1(const exp_group& g, const fdm_exp_offset& o, double x,
                                                        const fdm_exp_scale&)
   {
-    return g.expm1(o);
+    return x == 0.0 ? 0.0 : g.expm1(o);
   }
   // derivatives for the adjoint: d exp(x)/dx = exp(x), d log(x)/dx = 1/x
   template<class R>
@@ -429,7 +464,10 @@ struct fdm_math_approx {
   __device__ __forceinline__ static double fast_expm1_sat(double x) { return fast_exp_sat(x) - 1.0; }
   __device__ __forceinline__ static double fast_expm1_sat(double x, const fdm_exp_scale& f) { return fast_exp_sat(x, f) - 1.0; }
   __device__ __forceinline__ static double fast_div(double a, double b) { return fdm_div64(a, b); }
-  __device__ __forceinline__ static double fast_rcp(double d) { return fdm_rcp64(d); }
+  // the approximation minus 1 is 0 in a neighbourhood of 0
+  __device__ __forceinline__ static double fast_div0(double x, double e) { return fdm_div64_any(x, e); }
+  __device__ __forceinline__ static double fast_div_any(double a, double b) { return fdm_div64_any(a, b); }
+  __device__ __forceinline__ static double fast_rcp(double d) { return fdm_rcp64_any(d); }
   // (not multiplicative: every member by itself)
   struct exp_group {
     __device__ __forceinline__ exp_group(double, const fdm_exp_scale&) {}

@@ -61,6 +61,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_EXP_OF(...) M::group_exp(__VA_ARGS__)
 #define FDM_EXPM1_OF(...) M::group_expm1(__VA_ARGS__)
 #define FDM_DIV(x, y) M::fast_div(x, y)
+#define FDM_DIV0(x, y) M::fast_div0(x, y)
+#define FDM_DIV_ANY(x, y) M::fast_div_any(x, y)
 #define FDM_LOG(x) M::log(x)
 #define FDM_POWF(x, y) M::pow(x, y)
 #define FDM_ABS(x) fabs(x)
@@ -69,13 +71,13 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_POW3(x) fdm_pow3(x)
 #define FDM_POW4(x) fdm_pow4(x)
     const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-    ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), FDM_EXPM1_OF(fdm_g0, (STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
+    ALGEBRAIC[1] = FDM_DIV0((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), FDM_EXPM1_OF(fdm_g0, (STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
     ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{-0x1.c71c71c71c71cp-5, -0x1.c71c71c71c71cp-59, -0x1.484b13d7c02a9p-4, -0x1.8f40b5ed98000p+3, 0x1.0ba74058e83a2p-45}));
     RATES[1] = ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-5, 0x1.999999999999ap-59, -0x1.2776c50ef9bfep-4, -0x1.bb9d3beb8c800p+3, 0x1.566f7e8b7365ap-47}));
     ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), (FDM_EXP_OF(fdm_g0, fdm_exp_offset{0x1.a61298e1e069cp+0, -0x1.b4690082a4906p-55}, (STATES[0] + ((R)0x1.6800000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}) + ((R)0x1.0000000000000p+0)));
     RATES[2] = ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
-    ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), FDM_EXPM1_OF(fdm_g0, fdm_exp_offset{0x1.c8f87724b5c1dp-3, 0x1.91afa497dc416p-57}, (STATES[0] + ((R)0x1.0400000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
+    ALGEBRAIC[3] = FDM_DIV0((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), FDM_EXPM1_OF(fdm_g0, fdm_exp_offset{0x1.c8f87724b5c1dp-3, 0x1.91afa497dc416p-57}, (STATES[0] + ((R)0x1.0400000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
     ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{0x1.999999999999ap-7, -0x1.999999999999ap-61, 0x1.2776c50ef9bfep-6, 0x1.bb9d3beb8c800p+5, 0x1.566f7e8b7365ap-47}));
     RATES[3] = ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
@@ -92,6 +94,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_EXP_OF
 #undef FDM_EXPM1_OF
 #undef FDM_DIV
+#undef FDM_DIV0
+#undef FDM_DIV_ANY
 #undef FDM_LOG
 #undef FDM_POWF
 #undef FDM_ABS
@@ -194,6 +198,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #define FDM_EXP_OF(...) M::group_exp(__VA_ARGS__)
 #define FDM_EXPM1_OF(...) M::group_expm1(__VA_ARGS__)
 #define FDM_DIV(x, y) M::fast_div(x, y)
+#define FDM_DIV0(x, y) M::fast_div0(x, y)
+#define FDM_DIV_ANY(x, y) M::fast_div_any(x, y)
 #define FDM_LOG(x) M::log(x)
 #define FDM_POWF(x, y) M::pow(x, y)
 #define FDM_ABS(x) fabs(x)
@@ -209,7 +215,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     }
     else if constexpr (G == 1) {
       const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-      ALGEBRAIC[1] = FDM_DIV((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), FDM_EXPM1_OF(fdm_g0, (STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
+      ALGEBRAIC[1] = FDM_DIV0((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), FDM_EXPM1_OF(fdm_g0, (STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
       ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{-0x1.c71c71c71c71cp-5, -0x1.c71c71c71c71cp-59, -0x1.484b13d7c02a9p-4, -0x1.8f40b5ed98000p+3, 0x1.0ba74058e83a2p-45}));
       return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
     }
@@ -221,7 +227,7 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
     }
     else if constexpr (G == 3) {
       const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-      ALGEBRAIC[3] = FDM_DIV((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), FDM_EXPM1_OF(fdm_g0, fdm_exp_offset{0x1.c8f87724b5c1dp-3, 0x1.91afa497dc416p-57}, (STATES[0] + ((R)0x1.0400000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
+      ALGEBRAIC[3] = FDM_DIV0((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), FDM_EXPM1_OF(fdm_g0, fdm_exp_offset{0x1.c8f87724b5c1dp-3, 0x1.91afa497dc416p-57}, (STATES[0] + ((R)0x1.0400000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
       ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{0x1.999999999999ap-7, -0x1.999999999999ap-61, 0x1.2776c50ef9bfep-6, 0x1.bb9d3beb8c800p+5, 0x1.566f7e8b7365ap-47}));
       return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
     }
@@ -238,6 +244,8 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_EXP_OF
 #undef FDM_EXPM1_OF
 #undef FDM_DIV
+#undef FDM_DIV0
+#undef FDM_DIV_ANY
 #undef FDM_LOG
 #undef FDM_POWF
 #undef FDM_ABS

@@ -15,6 +15,7 @@ __global__ void function_kernel(int f, int64_t n, const double* x, const double*
   case 0: out[i] = fdm_math_exact::fast_exp(x[i]); break;
   case 1: out[i] = fdm_math_exact::fast_rcp(x[i]); break;
   case 2: out[i] = fdm_math_exact::fast_div(x[i], y[i]); break;
+  case 11: out[i] = fdm_math_exact::fast_div_any(x[i], y[i]); break;
   case 3: out[i] = fdm_math_exact::fast_expm1(x[i]); break;
   case 4: out[i] = fdm_math_exact::fast_exp(x[i], TEST_SCALE); break;
   case 5: out[i] = fdm_math_exact::fast_expm1(x[i], TEST_SCALE); break;

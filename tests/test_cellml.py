@@ -186,8 +186,8 @@ def test_fp64_form_exponentials():
     group = text[text.index("static R rates_group("):text.index("// vector-Jacobian product")]
     for body, reductions in ((f64, 1), (group, 3)):
         body = "\n".join(x for x in body.split("\n") if not x.startswith("#"))
-        names = ("M::exp_group", "FDM_EXPM1_OF(", "FDM_EXP_OF(", "FDM_EXP(", "FDM_DIV(")
-        assert [body.count(f) for f in names] == [reductions, 2, 1, 3, 3]
+        names = ("M::exp_group", "FDM_EXPM1_OF(", "FDM_EXP_OF(", "FDM_EXP(", "FDM_DIV(", "FDM_DIV0(")
+        assert [body.count(f) for f in names] == [reductions, 2, 1, 3, 1, 2]
     for b in (Fraction(-3, 2), Fraction(1, 2)):
         e, lo = (float.fromhex(x) for x in re.search(r"\{(.*), (.*)\}", cellml._exp_offset_text(b)).groups())
         assert e == np.exp(float(b)) and cellml._exp_offset_text(b) in f64
@@ -201,3 +201,28 @@ def test_exponentials_far_apart_share_nothing():
     em = cellml._Fast64Emitter("R", [], lines)
     assert em.bases == [lines[1][2][2][3][3][2][0]]
     assert sorted(b for _, b in em.members.values()) == [-1, 0]
+
+
+def test_divisions_that_need_no_special_values():
+    # FDM_DIV only where the divisor is known to be finite and away from 0 and the quotient finite; FDM_DIV0 only where dividend
+    # and divisor vanish together
+    model = lambda *texts: [("R", k, cellml.parse_expression(t)) for k, t in enumerate(texts)]
+    lean = ("1.0/(1.0+exp(STATES[0]/10.0))", "STATES[1]/(2.0+exp(STATES[0]))",
+            "3.0/(0.2+5.65*pow((STATES[0]+90.0)/100.0, 2.0))", "2.0/(-1.0-exp(STATES[0]))")
+    general = ("1.0/STATES[0]", "1.0/(1.0+0.5/STATES[1])", "exp(STATES[0])/(1.0+exp(STATES[1]))",
+             "STATES[0]/(STATES[1]+1.0)", "1.0/(exp(STATES[0])-1.0)", "STATES[0]/(1.0-exp(STATES[0]/25.0))",
+             "(STATES[0]+50.0)/(exp((STATES[0]+51.0)/10.0)-1.0)", "1.0/(1.0+log(STATES[0]))",
+             "exp(STATES[1])*(STATES[0]+50.0)/(exp((STATES[0]+50.0)/10.0)-1.0)", "1.0/(1e-305+exp(STATES[0]))")
+    together = ("0.1*(STATES[0]+50.0)/(1.0-exp(-(STATES[0]+50.0)/10.0))", "STATES[1]*(STATES[0]-40.0)/(exp((STATES[0]-40.0)*0.2)-1.0)")
+    for texts, name in ((lean, "FDM_DIV("), (together, "FDM_DIV0("), (general, "FDM_DIV_ANY(")):
+        for text in texts:
+            lines = model(text)
+            out = cellml._Fast64Emitter("R", [], lines).expr(lines[0][2])
+            assert {x for x in ("FDM_DIV(", "FDM_DIV0(", "FDM_DIV_ANY(", " / ") if x in out} == {name}, (text, out)
+    # no division: by constants, by powers of them, by an exponential
+    for text in ("STATES[0]/3.0", "STATES[0]/pow(0.2, 3.0)", "STATES[0]/exp(STATES[1])"):
+        lines = model(text)
+        assert "DIV" not in cellml._Fast64Emitter("R", [], lines).expr(lines[0][2])
+    # a range known from an algebraic variable
+    lines = [("A", 0, cellml.parse_expression("1.0/(1.0+exp(STATES[0]))")), ("R", 0, cellml.parse_expression("1.0/(0.5+ALGEBRAIC[0])"))]
+    assert "FDM_DIV(" in cellml._Fast64Emitter("R", [], lines).expr(lines[1][2])

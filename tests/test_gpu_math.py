@@ -1,4 +1,4 @@
-"""The FP64 arithmetic of the generated right-hand sides against 80-bit arithmetic."""
+"""The FP64 arithmetic of the generated right-hand sides against 80-bit arithmetic and IEEE 754's special values."""
 import ctypes as C
 import os
 import subprocess
@@ -37,6 +37,21 @@ def _pointer(a):
 @pytest.fixture(scope="module")
 def hodgkin_huxley(tmp_path_factory):
     return _library(tmp_path_factory.mktemp("hh"), CM.builtin_model(H.HH), (2, 3, 4))
+
+
+def _model(name, n_algebraics, constants, lines, n_states):
+    return CM.Model(name=name, source=name + ".c", n_states=n_states, n_algebraics=n_algebraics,
+                    n_constants=len(constants), states_initial=[0.0] * n_states, constants=constants, constant_lines=[],
+                    lines=[(kind, k, CM.parse_expression(text)) for kind, k, text in lines])
+
+
+@pytest.fixture(scope="module")
+def hill(tmp_path_factory):
+    """A Hill term, a Boltzmann term and a bare exponential, a quotient of states"""
+    return _library(tmp_path_factory.mktemp("hill"), _model("hill", 3, [0.5], [
+        ("A", 0, "1.00000/(1.00000+CONSTANTS[0]/STATES[1])"), ("A", 1, "1.00000/(1.00000+exp(STATES[0]/3.00000))"),
+        ("A", 2, "exp(STATES[0]/7.00000)"), ("R", 0, "ALGEBRAIC[0]"), ("R", 1, "ALGEBRAIC[1]"), ("R", 2, "ALGEBRAIC[2]"),
+        ("R", 3, "STATES[2]/STATES[1]")], 4))
 
 
 def _function(lib, f, x, y=None):
@@ -118,6 +133,44 @@ def test_exponential_group(hodgkin_huxley):
     assert np.isnan(got[0]) and np.all(got[[1, 3]] == -1.0) and np.all((got[[2, 4]] > 1e300) & (got[[2, 4]] < 1e305))
 
 
+SPECIAL = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1e-310, -3e-320, 2.0 ** -1022, 1e-300, 1.0, -3.5, 1e300,
+                    2.0 ** 1020, 2.0 ** 1021, 2.0 ** 1022, 1e308, -1.7e308])
+
+
+# one rounding of a correction that is exact to 2^-100; the reciprocal's cubic step leaves the third power of the
+# approximation's error, 2^-60 of the result at most
+def test_division_and_reciprocal(hill):
+    rng = np.random.default_rng(2)
+    a, b = (rng.uniform(1.0, 2.0, 1000000) * 2.0 ** rng.integers(-400, 400, 1000000) for _ in range(2))
+    a[::2] *= -1.0
+    exact = a.astype(np.longdouble) / b
+    for f in (2, 11):
+        assert _ulps(_function(hill, f, a, b), exact).max() < 0.51
+    assert _ulps(_function(hill, 1, b), 1 / b.astype(np.longdouble)).max() < 0.52
+    # the quotient's divisor may reach beyond 2^1022, where its reciprocal is subnormal
+    assert np.all(np.abs(_function(hill, 2, np.ones(2), np.array([2.0 ** 1022, 1e308]))) < 1e-307)
+    a, b = (m.ravel() for m in np.meshgrid(SPECIAL, SPECIAL))
+    with np.errstate(all="ignore"):
+        np.testing.assert_allclose(_function(hill, 11, a, b), a / b, rtol=1e-15, atol=5e-324)
+        want = np.where(np.abs(SPECIAL) < 2.0 ** 1021, 1 / SPECIAL, 0.0 * SPECIAL)    # subnormal results flushed
+        want[np.isnan(SPECIAL)], want[np.isinf(SPECIAL)] = np.nan, 0.0
+        np.testing.assert_allclose(_function(hill, 1, SPECIAL), want, rtol=1e-15, atol=2.0 ** -1021)
+
+
+# as IEEE arithmetic has them: 1/(1 + K/c) is 0 at c = 0, 1/(1 + exp(v)) is 0 where exp(v) overflows
+@pytest.mark.parametrize("approximate", [False, True])
+def test_terms_with_vanishing_and_infinite_divisors(hill, approximate):
+    v = np.array([-6000.0, -300.0, -70.0, 0.0, 70.0, 300.0, 1500.0, 2100.0, 4000.0, 1e6])
+    c = np.array([0.0, 1e-310, 1e-300, 1e-3, 0.5, 1.0, 1e3, 1e308, np.inf, 0.0])
+    d = np.array([1.0, 1e-305, 0.0, 2.0, -3.0, 1e300, np.inf, 1e308, 7.0, 0.0])
+    with np.errstate(all="ignore"):
+        e3, e7 = ((1 + v / 3 / 1024) ** 1024, (1 + v / 7 / 1024) ** 1024) if approximate else (np.exp(v / 3), np.exp(v / 7))
+        want = np.stack([1 / (1 + 0.5 / c), 1 / (1 + e3), e7, d / c])
+    for got in _rates(hill, approximate, np.stack([v, c, d, c])):
+        # arguments of up to 857 lose 2^-53 of themselves; the approximate exponential's 1024th power 1e-13
+        np.testing.assert_allclose(got, want, rtol=4e-13, atol=1e-300)
+
+
 # alpha_m = x / (exp(x) - 1) at V = -50 mV, alpha_n at -65 mV, around their removable singularities.  alpha_m is as exact
 # there as elsewhere; 20 mV away, in halves of an ulp: the argument's 2.5 times u e^u / (e^u - 1) = 2.3, the numerator's 2.5,
 # the exponential's 4, quotient, difference, product and sum 4: 17.  alpha_n's exponential is alpha_m's times e^-1.5: before
@@ -131,6 +184,9 @@ def test_rates_at_removable_singularities(hodgkin_huxley, singularity):
     params = np.stack([np.zeros(n), np.full(n, 120.0), np.full(n, 36.0)])
     V, m, h, g = states.astype(np.longdouble)
     tenth = np.longdouble(1) / 10
+    # at the singularity itself the quotient is 0/0, as the equations are
+    at = np.repeat([[singularity], [0.1], [0.5], [0.3]], 2, axis=1)
+    assert np.isnan(_rates(hodgkin_huxley, False, at, params[:, :2])[:, 1 if singularity == -50.0 else 3]).all()
     both = _rates(hodgkin_huxley, False, states, params)
     np.testing.assert_array_equal(both[0], both[1])
     for got in both[:1]:
