@@ -641,10 +641,11 @@ def _exp_groups(lines, consts):
     return repl, groups
 
 
-def _squared_groups(lines, consts, groups):
+def _squared_groups(lines, consts, repl, groups):
     """Groups of _exp_groups whose exponential is the square of one exponential outside them, at half their slope:
     {group: (exp node, its constant term, the positive constant it is multiplied with in the model or 1)}"""
     found = []
+    members = [[b for k, b in repl.values() if k == g] for g in range(len(groups))]
 
     def walk(e, factor=1.0):
         t = e[0]
@@ -670,8 +671,12 @@ def _squared_groups(lines, consts, groups):
     for g, key in enumerate(groups):
         for e, af, factor in found:
             half = tuple(sorted(af[0].items()))
+            # the square is e^base times the group's exponential, a member its square times e^(b - base): in FP32 both
+            # have to stay far from the ends of its range, e^-87 and e^88
+            base = 2 * (af[1] + math.log(factor))
             if len(half) == len(key) and all(k == k2 and abs(v - 2 * v2) <= 4e-15 * abs(v)
-                                             for (k, v), (k2, v2) in zip(key, half)):
+                                             for (k, v), (k2, v2) in zip(key, half)) \
+                    and abs(base) <= 20 and all(abs(b - base) <= 20 for b in members[g]):
                 out.setdefault(g, (e, af[1], factor))
     return out
 
@@ -1345,7 +1350,7 @@ def emit_cuda_model(model: Model, params_alg: Sequence[int], params_const: Seque
     # the same FP32 form over node pairs (packed FP32 instructions)
     fem2 = _FastEmitter("R", model.constants, repl, paired=True,
                         alg_defs={idx: expr for kind, idx, expr in lines if kind == "A"},
-                        squares=_squared_groups(lines, model.constants, groups))
+                        squares=_squared_groups(lines, model.constants, repl, groups))
     out.append("  // paired FP32 form: the FP32 form over two nodes at once (fdm_f2, packed FP32 instructions)")
     out.append("  template<class M>")
     out.append("  __device__ __forceinline__ static void rates_fast2(const fdm_f2 VOI, const fdm_f2* __restrict__ STATES,"

@@ -226,3 +226,17 @@ def test_divisions_that_need_no_special_values():
     # a range known from an algebraic variable
     lines = [("A", 0, cellml.parse_expression("1.0/(1.0+exp(STATES[0]))")), ("R", 0, cellml.parse_expression("1.0/(0.5+ALGEBRAIC[0])"))]
     assert "FDM_DIV(" in cellml._Fast64Emitter("R", [], lines).expr(lines[1][2])
+
+
+def test_squared_exponentials_stay_in_the_range_of_fp32():
+    # the paired FP32 form takes exp(x + b_k) from the square of an exponential of half the slope only where neither the
+    # square nor the factor comes near the ends of FP32: at V = 0 the model below is 1/(1 + e^-5) and so on, with
+    # exp((V - 900)/20)^2 it would be 0 times infinity
+    def squares(shift, factor="1.0"):
+        lines = [("R", 0, cellml.parse_expression(
+            f"1.0/(1.0+exp((STATES[0]-50.0)/10.0))+1.0/(1.0+exp((STATES[0]-20.0)/10.0))"
+            f"+{factor}*exp((STATES[0]-{shift})/20.0)"))]
+        repl, groups = cellml._exp_groups(lines, [])
+        return cellml._squared_groups(lines, [], repl, groups)
+    assert list(squares("75.0")) == [0] and list(squares("75.0", "0.07")) == [0]
+    assert squares("900.0") == {} and squares("-900.0") == {} and squares("75.0", "1e9") == {}
