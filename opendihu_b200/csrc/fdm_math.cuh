@@ -377,7 +377,7 @@ struct fdm_math_exact {
   __device__ __forceinline__ static double group_expm1(const exp_group& g, const fdm_exp_offset& o, double x,
                                                        const fdm_exp_scale&)
   {
-    return x == 0.0 ? 0.0 : g.expm1(o);
+    return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0 ? 0.0 : g.expm1(o);
   }
   // derivatives for the adjoint: d exp(x)/dx = exp(x), d log(x)/dx = 1/x
   template<class R>
