@@ -292,7 +292,7 @@ struct fdm_solver {
   size_t ev_used = 0;
   double main_ms = 0, adv_ms = 0, adj_ms = 0;
   bool finish_pending = false;   // an fdm_advance_async whose timing and NaN check fdm_wait still owes
-  bool adj_forward = false;      // inside fdm_adjoint_forward: the reaction runs one thread per node
+  bool adj_forward = false;      // inside fdm_adjoint_forward: a launch per half step and solve, as the replay
   int adjoint_tape = 1; // FDM_ADJOINT_TAPE=0 selects the re-evaluating reverse step (for measurements)
   int64_t main_launches = 0, launches = 0;
   cudaEvent_t adv_start = nullptr, adv_stop = nullptr;
@@ -2194,7 +2194,6 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
   ra.n_trace = s->n_trace;
   ra.trace_capacity = s->trace_capacity;
   ra.act = activation_rec(s);
-  ra.per_node = s->adj_forward ? 1 : 0;
   // without profiling, a window that stores no algebraics replays a captured CUDA graph of its launches; *n_launches
   // is their number once they were issued
   auto replay_or_launch = [&](auto&& launches, const int* n_launches) -> int {
@@ -3324,9 +3323,8 @@ extern "C" int fdm_adjoint_forward(fdm_solver* s, double t_start, double t_end, 
   }
   s->ev_used = 0;
   FDM_CUDA(cudaEventRecord(s->adv_start, s->stream));
-  // the replay in fdm_adjoint_backward runs the one-thread-per-node reaction kernel; the forward runs it too,
-  // so that the replay reproduces it bit for bit (window graphs captured with the other kernel are dropped)
-  invalidate_graphs(s);
+  // the replay in fdm_adjoint_backward issues the reaction and the solves launch by launch; the forward does so too, so that
+  // the replay reproduces it bit for bit
   s->adj_forward = true;
   for (int c = 0; c < A.n_seg && !rc; c++) {
     rc = copy_state(s, A.ck_vm.p + (size_t)c * N, A.ck_states.p + (size_t)c * N * (NS - 1), A.ck_last.p + (size_t)c * nf,
@@ -3337,7 +3335,6 @@ extern "C" int fdm_adjoint_forward(fdm_solver* s, double t_start, double t_end, 
     rc = run_planned(s, A.steps, A.dt1s, b, e, c == A.n_seg - 1);
   }
   s->adj_forward = false;
-  invalidate_graphs(s);
   if (rc)
     return rc;
   rc = copy_state(s, A.fin_vm.p, A.fin_states.p, A.fin_last.p, A.fin_jit.p, A.fin_jidx.p, A.fin_hbs.p, true);

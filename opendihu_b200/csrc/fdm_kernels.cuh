@@ -5,8 +5,10 @@
 //   one tridiagonal solve per fiber for the diffusion      (compute1D, :256-507)
 //   n0D Heun substeps starting at the mid time             (compute0D)
 // The kernels here implement it in two shapes:
-//   split:  reaction_kernel (one thread per node, states in HBM) + diffusion_warp_kernel (one warp per
-//           fiber, a partitioned Thomas sweep whose forward results go to a scratch array in HBM);
+//   split:  reaction_kernel (one thread per node, states in HBM) + diffusion_reg_kernel (one CTA per fiber, a
+//           thread's nodes in registers, the sweeps of the LU solve as block-wide scans; fdm_diffusion.cuh; many short
+//           or very long fibers: diffusion_warp_kernel, diffusion_block_kernel); few fibers in FP64:
+//           window_cluster_kernel, whole windows in one launch;
 //   fused:  fused_kernel (one CTA per bin of whole fibers; every thread keeps M nodes' states in
 //           registers across all split steps of a launch; the tridiagonal solve is a block-wide
 //           scan of affine maps in FP64; coefficients live in shared memory).
@@ -613,22 +615,23 @@ struct ReactionArgs {
                                   // store_states[(k*nStates + s)*stride + node], or null; a second half step's
   int64_t store_half_stride;      // store_half_stride doubles further
   double* store_vm_out;           // adjoint replay: Vm after the launch's half step 0 also written here, or null
-  int per_node;                   // 1: one thread per node whatever the size (the adjoint's checkpointed
-                                  // forward, which its replay reproduces bit for bit)
   const int* gate;                // onlyComputeIfHasBeenStimulated: per node gate code, or null
   const uint8_t* gate_start;
   int gate_stride;
 };
 
 // CTAs of 128 threads per SM that the registers are held to.  A model of many states spills either way in FP64 (Shorten:
-// 110 registers for its states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 53,316
-// nodes, 25 substeps 980 -> 770 us (four CTAs: 905).  In FP32 its 255 registers hold everything (168: 481 -> 1173 us).
-// Hodgkin-Huxley in FP64 is bound by its dependent FP64 chains: six CTAs, 1,566,410 nodes, 10 substeps: 309 us against 350
-// with four and 318 with five.
+// 110 registers for its states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 4 steps of
+// 53,316 nodes with their transfers 5.73 ms against 5.88 (four CTAs: 6.22).  In FP32 its 255 registers hold everything
+// (168: 481 -> 1173 us).
+// Hodgkin-Huxley in FP64 is bound by the FP64 pipe; four CTAs let the compiler interleave its exponentials: two half steps
+// of 5 substeps of 1,566,720 nodes 304 us against 318 with six and 319 with five (three: 310), of 94,784 nodes 30.3 against
+// 32.5.  So a thread per node is the fastest form for few nodes too: with a warp for each of a node's four states, 32 nodes
+// per CTA, a step took 11.0 us against 9.5 (101 nodes), 13.4 against 11.6 (6000) and 19.2 against 15.5 (23,696).
 template<class Model, class RR>
 constexpr int reaction_min_ctas()
 {
-  return Model::nStates > 16 ? (sizeof(RR) == 8 ? 3 : 1) : (sizeof(RR) == 8 ? 6 : 8);
+  return Model::nStates > 16 ? (sizeof(RR) == 8 ? 3 : 1) : (sizeof(RR) == 8 ? 4 : 8);
 }
 
 template<class Model, class RR, class Math>
@@ -704,94 +707,6 @@ __global__ void __launch_bounds__(128, reaction_min_ctas<Model, RR>()) reaction_
     if (Compensated<RR>::value)
       stl[(s2 - 1) * a.stride + i] = L[s2 - 1];
   }
-}
-
-// Split-path reaction for few nodes, FP64: the warps of a CTA share 32 nodes, warp g advancing state g of
-// each (Model::rates_group evaluates one state's rate from the lines it needs).  With one thread per node a
-// problem of a few ten thousand nodes leaves each SM a handful of warps whose Heun chains stall on FP64
-// latency; here every node gives nStates independent chains.  The states of the 32 nodes live in shared
-// memory; per substep each warp forms its y*, the CTA synchronizes, each warp forms its new state from both
-// rates, the CTA synchronizes.  Same expressions and operation order as heun_step (FP64), so the same values.
-template<class Model, class Math, int G>
-__device__ __forceinline__ double group_rate(int g, double t, const double* y, const double* P)
-{
-  if constexpr (G < Model::nGroups) {
-    if (g == G)
-      return Model::template rates_group<double, Math, G>(t, y, P);
-    return group_rate<Model, Math, G + 1>(g, t, y, P);
-  } else {
-    return 0.0;
-  }
-}
-
-template<class Model, class Math>
-__global__ void __launch_bounds__(32 * (Model::nGroups > 0 ? Model::nGroups : 1)) reaction_group_kernel(ReactionArgs a)
-{
-  constexpr int NS = Model::nStates;
-  constexpr int NP = Model::nParameters > 0 ? Model::nParameters : 1;
-  __shared__ double sy[NS][32], sys[NS][32];
-  const int lane = threadIdx.x, g = threadIdx.y;
-  const int64_t i = (int64_t)blockIdx.x * 32 + lane;
-  const bool ok = i < a.n_nodes;
-  const double* st = (const double*)a.states;
-  const double* pr = (const double*)a.params;
-  double own = 0.0;
-  if (ok)
-    own = g == 0 ? a.vm[i] : st[(g - 1) * a.stride + i];
-  sy[g][lane] = own;
-  double P[NP], Pstim[NP];
-#pragma unroll
-  for (int q = 0; q < Model::nParameters; q++) {
-    P[q] = ok ? pr[q * a.stride + i] : 0.0;
-    Pstim[q] = (a.stimulus_mode == 1 && q == a.stimulus_parameter) ? a.stimulus_value : P[q];
-  }
-  const int cf = ok ? a.clamp_fiber[i] : -1;
-  const int slot = (ok && g == 0 && a.trace_slot) ? a.trace_slot[i] : -1;
-  __syncthreads();
-#pragma unroll 1
-  for (int hh = 0; hh < a.n_halves; hh++) {
-    const int hs = a.step * 2 + a.half + hh; // half step of the window
-    const SplitStep s = a.steps[hs >> 1];
-    const double t0 = (hs & 1) ? s.mid : s.t;
-    const int base = hs * a.nsub_stride;
-#pragma unroll 1
-    for (int k = 0; k < s.n0; k++) {
-      const double t = xadd(t0, xmul((double)k, s.dt0));
-      const bool stim = cf >= 0 && stim_bit(a.flags, a.words_per_fiber, cf, base + k);
-      const bool vclamp = stim && a.stimulus_mode == 0;
-      double Pk[NP];
-#pragma unroll
-      for (int q = 0; q < NP; q++)
-        Pk[q] = (stim && a.stimulus_mode == 1) ? Pstim[q] : P[q];
-      double y[NS];
-#pragma unroll
-      for (int q = 0; q < NS; q++)
-        y[q] = sy[q][lane];
-      const double r = group_rate<Model, Math, 0>(g, t, y, Pk);
-      double ys = own + s.dt0 * r;
-      if (g == 0 && vclamp)
-        ys = a.vstim;
-      sys[g][lane] = ys;
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < NS; q++)
-        y[q] = sys[q][lane];
-      const double r2 = group_rate<Model, Math, 0>(g, t, y, Pk);
-      own += 0.5 * s.dt0 * (r + r2);
-      if (g == 0 && vclamp)
-        own = a.vstim;
-      sy[g][lane] = own;
-      __syncthreads();
-    }
-    if ((hs & 1) && slot >= 0)
-      record_trace(a.trace, a.n_trace, a.trace_capacity, a.act, slot, s.global_no, own);
-  }
-  if (!ok)
-    return;
-  if (g == 0)
-    a.vm[i] = own;
-  else
-    ((double*)a.states)[(g - 1) * a.stride + i] = own;
 }
 
 // affine map x -> F x + G; compose(first, second) = second o first

@@ -183,74 +183,6 @@ struct fdm_model_hodgkin_huxley_1952_anone_c2_3_4 {
 #undef FDM_ABS
 #undef FDM_SQRT
   }
-  // the right-hand side of one state at a time: rates_group<R, M, G> = RATES[G]
-  static constexpr int nGroups = 4;
-  template<class R, class M, int G>
-  __device__ __forceinline__ static R rates_group(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS)
-  {
-    (void)VOI; (void)PARAMS;
-    R ALGEBRAIC[9];
-    (void)ALGEBRAIC;
-#define FDM_EXP(...) M::fast_exp(__VA_ARGS__)
-#define FDM_EXPM1(...) M::fast_expm1(__VA_ARGS__)
-#define FDM_EXP_SAT(...) M::fast_exp_sat(__VA_ARGS__)
-#define FDM_EXPM1_SAT(...) M::fast_expm1_sat(__VA_ARGS__)
-#define FDM_EXP_OF(...) M::group_exp(__VA_ARGS__)
-#define FDM_EXPM1_OF(...) M::group_expm1(__VA_ARGS__)
-#define FDM_DIV(x, y) M::fast_div(x, y)
-#define FDM_DIV0(x, y) M::fast_div0(x, y)
-#define FDM_DIV_ANY(x, y) M::fast_div_any(x, y)
-#define FDM_LOG(x) M::log(x)
-#define FDM_POWF(x, y) M::pow(x, y)
-#define FDM_ABS(x) fabs(x)
-#define FDM_SQRT(x) sqrt(x)
-#define FDM_POW2(x) fdm_pow2(x)
-#define FDM_POW3(x) fdm_pow3(x)
-#define FDM_POW4(x) fdm_pow4(x)
-    if constexpr (G == 0) {
-      ALGEBRAIC[0] = (((PARAMS[1] * FDM_POW3(STATES[1])) * STATES[2]) * (STATES[0] - ((R)0x1.4000000000000p+5)));
-      ALGEBRAIC[4] = ((PARAMS[2] * FDM_POW4(STATES[3])) * (STATES[0] - ((R)-0x1.5c00000000000p+6)));
-      ALGEBRAIC[8] = (((R)0x1.3333333333333p-2) * (STATES[0] - ((R)-0x1.018c49ba5e354p+6)));
-      return (-((((-PARAMS[0]) + ALGEBRAIC[0]) + ALGEBRAIC[4]) + ALGEBRAIC[8]));
-    }
-    else if constexpr (G == 1) {
-      const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-      ALGEBRAIC[1] = FDM_DIV0((((R)-0x1.999999999999ap-4) * (STATES[0] + ((R)0x1.9000000000000p+5))), FDM_EXPM1_OF(fdm_g0, (STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
-      ALGEBRAIC[5] = (((R)0x1.0000000000000p+2) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{-0x1.c71c71c71c71cp-5, -0x1.c71c71c71c71cp-59, -0x1.484b13d7c02a9p-4, -0x1.8f40b5ed98000p+3, 0x1.0ba74058e83a2p-45}));
-      return ((ALGEBRAIC[1] * (((R)0x1.0000000000000p+0) - STATES[1])) - (ALGEBRAIC[5] * STATES[1]));
-    }
-    else if constexpr (G == 2) {
-      const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-      ALGEBRAIC[2] = (((R)0x1.1eb851eb851ecp-4) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-5, 0x1.999999999999ap-59, -0x1.2776c50ef9bfep-4, -0x1.bb9d3beb8c800p+3, 0x1.566f7e8b7365ap-47}));
-      ALGEBRAIC[6] = FDM_DIV(((R)0x1.0000000000000p+0), (FDM_EXP_OF(fdm_g0, fdm_exp_offset{0x1.a61298e1e069cp+0, -0x1.b4690082a4906p-55}, (STATES[0] + ((R)0x1.6800000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}) + ((R)0x1.0000000000000p+0)));
-      return ((ALGEBRAIC[2] * (((R)0x1.0000000000000p+0) - STATES[2])) - (ALGEBRAIC[6] * STATES[2]));
-    }
-    else if constexpr (G == 3) {
-      const typename M::exp_group fdm_g0((STATES[0] + ((R)0x1.9000000000000p+5)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47});
-      ALGEBRAIC[3] = FDM_DIV0((((R)-0x1.47ae147ae147bp-7) * (STATES[0] + ((R)0x1.0400000000000p+6))), FDM_EXPM1_OF(fdm_g0, fdm_exp_offset{0x1.c8f87724b5c1dp-3, 0x1.91afa497dc416p-57}, (STATES[0] + ((R)0x1.0400000000000p+6)), fdm_exp_scale{-0x1.999999999999ap-4, 0x1.999999999999ap-58, -0x1.2776c50ef9bfep-3, -0x1.bb9d3beb8c800p+2, 0x1.566f7e8b7365ap-47}));
-      ALGEBRAIC[7] = (((R)0x1.0000000000000p-3) * FDM_EXP((STATES[0] + ((R)0x1.2c00000000000p+6)), fdm_exp_scale{0x1.999999999999ap-7, -0x1.999999999999ap-61, 0x1.2776c50ef9bfep-6, 0x1.bb9d3beb8c800p+5, 0x1.566f7e8b7365ap-47}));
-      return ((ALGEBRAIC[3] * (((R)0x1.0000000000000p+0) - STATES[3])) - (ALGEBRAIC[7] * STATES[3]));
-    }
-    else {
-      return (R)0;
-    }
-#undef FDM_POW2
-#undef FDM_POW3
-#undef FDM_POW4
-#undef FDM_EXP
-#undef FDM_EXPM1
-#undef FDM_EXP_SAT
-#undef FDM_EXPM1_SAT
-#undef FDM_EXP_OF
-#undef FDM_EXPM1_OF
-#undef FDM_DIV
-#undef FDM_DIV0
-#undef FDM_DIV_ANY
-#undef FDM_LOG
-#undef FDM_POWF
-#undef FDM_ABS
-#undef FDM_SQRT
-  }
   // vector-Jacobian product: LAM_STATES += J^T LAM_RATES, LAM_PARAMS += (dRATES/dPARAMS)^T LAM_RATES
   template<class R, class M>
   __device__ __forceinline__ static void rates_vjp(const R VOI, const R* __restrict__ STATES, const R* __restrict__ PARAMS, const R* __restrict__ LAM_RATES, R* __restrict__ LAM_STATES, R* __restrict__ LAM_PARAMS)

@@ -27,7 +27,6 @@ __global__ void function_kernel(int f, int64_t n, const double* x, const double*
   }
 }
 
-// rates[form][state][i]: form 0 the one-thread form, form 1 a state at a time
 template<class Math>
 __global__ void rates_kernel(int64_t n, double t, const double* states, const double* params, double* rates)
 {
@@ -41,10 +40,8 @@ __global__ void rates_kernel(int64_t n, double t, const double* states, const do
   for (int q = 0; q < M::nParameters; q++)
     p[q] = params[q * n + i];
   fdm::model_rates<M, double, Math>(t, y, p, r, alg);
-  for (int s = 0; s < M::nStates; s++) {
+  for (int s = 0; s < M::nStates; s++)
     rates[s * n + i] = r[s];
-    rates[(M::nStates + s) * n + i] = fdm::group_rate<M, Math, 0>(s, t, y, p);
-  }
 }
 
 // device copy of a host array, freed at the end of the call
@@ -74,7 +71,7 @@ extern "C" int eval_function(int f, int64_t n, const double* x, const double* y,
 extern "C" int eval_rates(int approximate, int64_t n, double t, const double* states, const double* params, double* rates)
 {
   using M = TEST_MODEL;
-  Array S(states, n * M::nStates), P(params, n * M::nParameters), R(rates, 2 * n * M::nStates);
+  Array S(states, n * M::nStates), P(params, n * M::nParameters), R(rates, n * M::nStates);
   if (!S.d || !P.d || !R.d)
     return 1;
   const unsigned blocks = (unsigned)((n + 127) / 128);

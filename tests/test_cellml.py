@@ -180,14 +180,12 @@ def test_settings_with_mappings():
 def test_fp64_form_exponentials():
     # Hodgkin-Huxley in FP64: the three exponentials of slope 1/10 are in divisors and come from one reduction, at offsets 0
     # (alpha_m), -1.5 (alpha_n) and 0.5 (beta_h); exp(u) - 1 has a function of its own; the other three exponentials stand
-    # alone; in the one-thread form and in the one of a state at a time
+    # alone
     text = cellml.emit_cuda_model(cellml.builtin_model(H.HH), (), (2, 3, 4))
     f64 = text[text.index("static void rates_f64("):text.index("// FP32 form")]
-    group = text[text.index("static R rates_group("):text.index("// vector-Jacobian product")]
-    for body, reductions in ((f64, 1), (group, 3)):
-        body = "\n".join(x for x in body.split("\n") if not x.startswith("#"))
-        names = ("M::exp_group", "FDM_EXPM1_OF(", "FDM_EXP_OF(", "FDM_EXP(", "FDM_DIV(", "FDM_DIV0(")
-        assert [body.count(f) for f in names] == [reductions, 2, 1, 3, 1, 2]
+    body = "\n".join(x for x in f64.split("\n") if not x.startswith("#"))
+    names = ("M::exp_group", "FDM_EXPM1_OF(", "FDM_EXP_OF(", "FDM_EXP(", "FDM_DIV(", "FDM_DIV0(")
+    assert [body.count(f) for f in names] == [1, 2, 1, 3, 1, 2]
     for b in (Fraction(-3, 2), Fraction(1, 2)):
         e, lo = (float.fromhex(x) for x in re.search(r"\{(.*), (.*)\}", cellml._exp_offset_text(b)).groups())
         assert e == np.exp(float(b)) and cellml._exp_offset_text(b) in f64

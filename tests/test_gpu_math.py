@@ -65,7 +65,7 @@ def _function(lib, f, x, y=None):
 def _rates(lib, approximate, states, params=np.zeros((1, 1))):
     states, params = np.ascontiguousarray(states, np.float64), np.ascontiguousarray(params, np.float64)
     ns, n = states.shape
-    out = np.empty((2, ns, n))
+    out = np.empty((ns, n))
     assert lib.eval_rates(C.c_int(int(approximate)), C.c_int64(n), C.c_double(0.0), _pointer(states), _pointer(params),
                           _pointer(out)) == 0
     return out
@@ -166,9 +166,8 @@ def test_terms_with_vanishing_and_infinite_divisors(hill, approximate):
     with np.errstate(all="ignore"):
         e3, e7 = ((1 + v / 3 / 1024) ** 1024, (1 + v / 7 / 1024) ** 1024) if approximate else (np.exp(v / 3), np.exp(v / 7))
         want = np.stack([1 / (1 + 0.5 / c), 1 / (1 + e3), e7, d / c])
-    for got in _rates(hill, approximate, np.stack([v, c, d, c])):
-        # arguments of up to 857 lose 2^-53 of themselves; the approximate exponential's 1024th power 1e-13
-        np.testing.assert_allclose(got, want, rtol=4e-13, atol=1e-300)
+    # arguments of up to 857 lose 2^-53 of themselves; the approximate exponential's 1024th power 1e-13
+    np.testing.assert_allclose(_rates(hill, approximate, np.stack([v, c, d, c])), want, rtol=4e-13, atol=1e-300)
 
 
 # alpha_m = x / (exp(x) - 1) at V = -50 mV, alpha_n at -65 mV, around their removable singularities.  alpha_m is as exact
@@ -186,14 +185,12 @@ def test_rates_at_removable_singularities(hodgkin_huxley, singularity):
     tenth = np.longdouble(1) / 10
     # at the singularity itself the quotient is 0/0, as the equations are
     at = np.repeat([[singularity], [0.1], [0.5], [0.3]], 2, axis=1)
-    assert np.isnan(_rates(hodgkin_huxley, False, at, params[:, :2])[:, 1 if singularity == -50.0 else 3]).all()
-    both = _rates(hodgkin_huxley, False, states, params)
-    np.testing.assert_array_equal(both[0], both[1])
-    for got in both[:1]:
-        for k, y, top, scale, centre, beta in ((1, m, tenth, 10, 50, 4 * np.exp(-(V + 75) / 18)),
-                                               (3, g, tenth / 10, 10, 65, np.exp((V + 75) / 80) / 8)):
-            alpha = -(V + centre) * top / np.expm1(-(V + centre) / scale)
-            error = np.abs(got[k] - (alpha * (1 - y) - beta * y))
-            u = np.abs(V + centre) / 10
-            cancelled = 0.7 * (1 + 1 / u) * alpha * (1 - y) if k == 3 else 0
-            assert np.all(error < 2.0 ** -53 * (18 * (alpha * (1 - y) + beta * y) + cancelled))
+    assert np.isnan(_rates(hodgkin_huxley, False, at, params[:, :2])[1 if singularity == -50.0 else 3]).all()
+    got = _rates(hodgkin_huxley, False, states, params)
+    for k, y, top, scale, centre, beta in ((1, m, tenth, 10, 50, 4 * np.exp(-(V + 75) / 18)),
+                                           (3, g, tenth / 10, 10, 65, np.exp((V + 75) / 80) / 8)):
+        alpha = -(V + centre) * top / np.expm1(-(V + centre) / scale)
+        error = np.abs(got[k] - (alpha * (1 - y) - beta * y))
+        u = np.abs(V + centre) / 10
+        cancelled = 0.7 * (1 + 1 / u) * alpha * (1 - y) if k == 3 else 0
+        assert np.all(error < 2.0 ** -53 * (18 * (alpha * (1 - y) + beta * y) + cancelled))
