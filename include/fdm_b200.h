@@ -295,6 +295,10 @@ int fdm_adjoint_timing(const fdm_solver *s, double *backward_ms);
 int fdm_fused_shapes(int *threads, int *nodes_per_thread, int capacity);
 /* the same for the cluster mode of the fused kernel (a fiber spread over up to 8 CTAs of one cluster) */
 int fdm_fused_cluster_shapes(int *threads, int *nodes_per_thread, int capacity);
+/* how many thread-block clusters of that many CTAs (1 to 8) the CUDA device holds at once with an SM for every CTA (0: none,
+ * or no such device).  Few fibers, each over a cluster, are advanced that way (fused method, and whole windows of the FP64
+ * split method) as long as all their clusters fit; the grouping of the SMs, and so the number, differs between devices */
+int fdm_resident_clusters(int device, int cluster_size);
 /* the fused launch fdm_set_fibers chose: CTA size, nodes per thread, CTAs per fiber (1: bins of whole
  * fibers, > 1: cluster mode), number of CTAs */
 int fdm_fused_layout(const fdm_solver *s, int *threads, int *nodes_per_thread, int *cluster_size, int *n_blocks);

@@ -33,6 +33,7 @@ EXPORTED = [
     "fdm_adjoint_backward", "fdm_adjoint_release", "fdm_adjoint_timing", "fdm_rewind", "fdm_set_clamp_nodes",
     "fdm_select_clamp_nodes", "fdm_select_gate_codes", "fdm_set_gate_codes", "fdm_get_equilibrium_state",
     "fdm_cellml_rhs_device", "fdm_cellml_rhs_configure", "fdm_fused_cluster_shapes", "fdm_fused_layout",
+    "fdm_resident_clusters",
     "fdm_get_compute_state_information", "fdm_advance_async", "fdm_wait", "fdm_wait_for", "fdm_repeated_call_plan",
     "fdm_advance_pieces", "fdm_set_stimulation_log", "fdm_get_stimulation_log",
     "fdm_model_equilibrium", "fdm_emg_set_preconditioner", "fdm_emg_create", "fdm_emg_destroy", "fdm_emg_last_error",
@@ -131,6 +132,7 @@ def lib() -> C.CDLL:
         "fdm_checkpoint_restore": (C.c_int, [P]),
         "fdm_fused_shapes": (C.c_int, [i32, i32, C.c_int]),
         "fdm_fused_cluster_shapes": (C.c_int, [i32, i32, C.c_int]),
+        "fdm_resident_clusters": (C.c_int, [C.c_int, C.c_int]),
         "fdm_fused_layout": (C.c_int, [P, i32, i32, i32, i32]),
         "fdm_get_compute_state_information": (C.c_int, [P, d]),
         "fdm_emg_create": (C.c_int, [C.c_int, C.c_int, C.c_int, d, C.c_int, C.POINTER(P)]),

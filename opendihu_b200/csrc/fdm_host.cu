@@ -443,6 +443,18 @@ extern "C" int fdm_model_info(int model, int* n_states, int* n_algebraics, int* 
   return FDM_OK;
 }
 
+extern "C" int fdm_resident_clusters(int device, int cluster_size)
+{
+  int before = 0;
+  if (cudaGetDevice(&before) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const int n = clusters_with_own_sms(cluster_size);
+  cudaSetDevice(before);
+  return n;
+}
+
 extern "C" int fdm_fused_cluster_shapes(int* threads, int* nodes_per_thread, int capacity)
 {
   FusedShape sh[64];

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import helpers as H
+from opendihu_b200 import _native as N
 from opendihu_b200 import sharding as SH
 from opendihu_b200 import solver as S
 from opendihu_b200 import workloads as WL
@@ -45,6 +46,19 @@ def test_sharded_equals_unsharded(method, n_ranks):
     else:
         assert np.max(np.abs(st[0] - ref[0])) <= 1e-9   # the block scan's tree depends on the bin layout
     assert np.max(np.abs(st[0] - H.run_oracle(s.copy())[0][0])) <= 1e-6
+
+
+# the whole system takes a launch per half step and solve, its shards the windows in one launch
+def test_sharded_equals_unsharded_across_window_forms():
+    n = N.lib().fdm_resident_clusters(0, 1)
+    s = WL.batched_hh(n_fibers=n + 20, min_nodes=100, max_nodes=120, seed=5, end_time=0.5, clamp_rule="center")
+    s.call_enable_begin[:] = 0.0
+    H.complete(s)
+    ref = _unsharded(s, method="split")
+    with SH.ShardedSolver(s.copy(), devices=[0], n_shards=3, method="split") as sh:
+        assert max(len(f) for f in sh.fibers) <= n
+        sh.advanceTimeSpan()
+        np.testing.assert_array_equal(sh.states(), ref)
 
 
 def test_sharded_adjoint_equals_unsharded():
