@@ -446,7 +446,8 @@ extern "C" int fdm_model_info(int model, int* n_states, int* n_algebraics, int* 
 extern "C" int fdm_resident_clusters(int device, int cluster_size)
 {
   int before = 0;
-  if (cudaGetDevice(&before) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) {
+  if (cluster_size < 1 || cluster_size > FDM_MAX_CLUSTER || cudaGetDevice(&before) != cudaSuccess ||
+      cudaSetDevice(device) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
