@@ -239,16 +239,6 @@ __global__ void own_sm_probe_kernel()
 
 int clusters_with_own_sms(int csize)
 {
-  // the device's answer, asked once per device and size: 0 not asked yet, else 1 + the number (the driver's two calls take
-  // some 20 us, and fdm_set_fibers asks for up to eight sizes)
-  static std::atomic<int> known[64][FDM_MAX_CLUSTER + 1];
-  int dev = 0;
-  if (csize < 1 || csize > FDM_MAX_CLUSTER || cudaGetDevice(&dev) != cudaSuccess)
-    return 0;
-  std::atomic<int>* slot = dev < 64 ? &known[dev][csize] : nullptr;
-  if (slot)
-    if (const int k = slot->load(std::memory_order_relaxed))
-      return k - 1;
   constexpr int HALF_SM = 120 * 1024;
   int n = 0;
   cudaLaunchConfig_t cfg = {};
@@ -267,8 +257,6 @@ int clusters_with_own_sms(int csize)
     cudaGetLastError();
     return 0;
   }
-  if (slot)
-    slot->store(n + 1, std::memory_order_relaxed);
   return n;
 }
 
