@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(EMG_T, 4) cg_direction_kernel(Grid g, const do
 // 97 x 97 x 297 nodes a direction pass takes 115 us against 146 (0.56 of the measured copy rate), a V-cycle's passes over the two
 // finest levels, both marching, 457 against 593.
 constexpr int ST_T = 352;              // threads: (tx + 2) (ty + 2) <= ST_T
-constexpr int64_t ST_MIN_NODES = 600000;
+constexpr int64_t ST_MIN_NODES = 600000, ST_MIN_NODES_JACOBI = 1200000;   // see choose_tiles
 enum StencilOp { ST_RESIDUAL, ST_JACOBI, ST_DIRECTION };
 
 struct StencilTiles {
@@ -1297,7 +1297,6 @@ struct fdm_emg {
   int cgp_ctas = -1;                           // its CTAs that can be resident together (-1: not asked yet)
   cudaGraphExec_t graphs[1] = {nullptr};       // CG chunk of the bidomain solve
   int precond = FDM_EMG_PRECOND_MULTIGRID;     // of the bidomain solve
-  StencilTiles tiles{};                        // of the fine grid (chunks == 0: node-per-thread passes)
   std::vector<MgLevel*> mg;                    // multigrid hierarchy of K(sigma_i + sigma_e), built on first use
   bool have_dir = false, have_ops = false, have_map = false;
   int64_t n_tensor_i = 0, n_tensor_e = 0;
@@ -1404,14 +1403,15 @@ std::vector<int> coarse_indices(int n)
   return F;
 }
 
-// the tiles of a grid's stencil passes; grids below ST_MIN_NODES, which have too few planes and
-// columns for the chip, take the node-per-thread passes.  Per iteration, marching against a thread per node: Jacobi,
-// 114,345 nodes 21.5 us against 18.0, 384,160 36.4 / 34.6, 720,000 56.2 / 55.1, 1,408,000 94 / 99; multigrid 147 / 134,
-// 243 / 237, 333 / 341, 524 / 557.
-int choose_tiles(fdm_emg* m, const Grid& g, StencilTiles* tiles)
+// The tiles of a grid's stencil passes; grids of fewer than min_nodes, which have too few planes and columns for the chip,
+// take the node-per-thread passes.  Per iteration, marching against a thread per node: multigrid, whose V-cycle has five
+// such passes, 60 x 60 x 150 nodes 287 us / 290, 70 x 70 x 120 302 / 320, 60 x 60 x 170 309 / 308, 90 x 80 x 90 326 / 341;
+// Jacobi, with one pass, either way by shape up to a million nodes (80 x 80 x 100 52.2 / 50.6, 60 x 60 x 200 56.5 / 55.1,
+// 95^3 60.2 / 62.9, 100^3 74.1 / 72.6), then marching: 110 x 100 x 110 86.3 / 89.3, 80 x 80 x 220 94.8 / 100.0.
+int choose_tiles(fdm_emg* m, const Grid& g, int64_t min_nodes, StencilTiles* tiles)
 {
   *tiles = StencilTiles{};
-  if (g.n_nodes() < ST_MIN_NODES)
+  if (g.n_nodes() < min_nodes)
     return FDM_OK;
   int sms = 0;
   EMG_CUDA(m, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
@@ -1430,7 +1430,7 @@ int mg_build(fdm_emg* m)
   MgLevel* L0 = new MgLevel();
   L0->g = m->hm.g;
   m->mg.push_back(L0);
-  if (const int rc = choose_tiles(m, L0->g, &L0->tiles))
+  if (const int rc = choose_tiles(m, L0->g, ST_MIN_NODES, &L0->tiles))
     return rc;
   EMG_CUDA(m, L0->t.alloc(m->N));
   EMG_CUDA(m, L0->r.alloc(m->N));
@@ -1472,7 +1472,7 @@ int mg_build(fdm_emg* m)
     MgLevel* Cl = new MgLevel();
     m->mg.push_back(Cl);
     Cl->g = Grid{(int)Fi[0].size(), (int)Fi[1].size(), (int)Fi[2].size()};
-    if (const int rc = choose_tiles(m, Cl->g, &Cl->tiles))
+    if (const int rc = choose_tiles(m, Cl->g, ST_MIN_NODES, &Cl->tiles))
       return rc;
     const int64_t Nc = Cl->g.n_nodes();
     EMG_CUDA(m, F->lo.alloc(lo.size()));
@@ -1559,9 +1559,9 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
   const double bnorm = hs[CG_BB] > 0 ? std::sqrt(hs[CG_BB]) : std::sqrt(hs[CG_RR]);
   const double target = std::max(rtol * bnorm, atol);
   double rn = std::sqrt(hs[CG_RR]);
-  if (!m->tiles.chunks)
-    if (const int rc = choose_tiles(m, g, &m->tiles))
-      return rc;
+  StencilTiles tiles;
+  if (const int rc = choose_tiles(m, g, use_mg ? ST_MIN_NODES : ST_MIN_NODES_JACOBI, &tiles))
+    return rc;
   // small meshes, Jacobi: all iterations in one cooperative launch, as long as a CTA per CGP_T nodes is resident
   // (113,664 nodes on 148 SMs); beyond that a launch per pass
   if (!use_mg && m->cgp_ctas < 0) {
@@ -1604,9 +1604,9 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
   }
   // one iteration: direction and product, then the update
   auto iteration = [&]() {
-    if (!mask && m->tiles.chunks) {
-      StencilArgs a{g, m->tiles, U, m->z.p, nullptr, nullptr, nullptr, m->p0.p, m->q.p, S, P, C};
-      stencil_kernel<ST_DIRECTION><<<(unsigned)m->tiles.blocks(), ST_T, ST_SMEM, s>>>(a);
+    if (!mask && tiles.chunks) {
+      StencilArgs a{g, tiles, U, m->z.p, nullptr, nullptr, nullptr, m->p0.p, m->q.p, S, P, C};
+      stencil_kernel<ST_DIRECTION><<<(unsigned)tiles.blocks(), ST_T, ST_SMEM, s>>>(a);
     } else {
       cg_direction_kernel<<<nb, EMG_T, 0, s>>>(g, U, mask, m->z.p, m->p0.p, m->q.p, S, P, C);
     }

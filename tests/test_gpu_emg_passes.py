@@ -36,9 +36,9 @@ def _solver(shape, preconditioner, rtol):
 
 
 # 8 and 767 to 769 nodes: one block, full, one more; 3 x 256; the largest mesh of the persistent form and the first
-# beyond it are around 113,664 nodes on 148 SMs
+# beyond it are around 113,664 nodes on 148 SMs; the march along z from 1,200,000 nodes
 @pytest.mark.parametrize("shape", [(2, 2, 2), (13, 59, 2), (8, 8, 12), (769, 2, 2), (16, 16, 3), (37, 61, 50),
-                                   (37, 64, 48), (37, 64, 49)])
+                                   (37, 64, 48), (37, 64, 49), (110, 101, 109)])
 def test_jacobi_residual(shape):
     with _solver(shape, "jacobi", 1e-10) as s:
         vm = np.random.default_rng(1).uniform(-80.0, 40.0, s.n_nodes)
@@ -54,7 +54,7 @@ def test_jacobi_residual(shape):
 
 
 # tiles that do and do not divide the grid, a single tile, more tiles than planes, a thin grid
-# (the march along z takes grids from 600,000 nodes, the last six)
+# (here the march along z takes grids from 600,000 nodes, the last six)
 @pytest.mark.parametrize("shape", [(101, 37, 29), (16, 18, 360), (2, 300, 190), (101, 97, 65), (65, 97, 97),
                                    (16, 18, 2100), (550, 560, 2), (2, 500, 610), (1100, 3, 190)])
 def test_multigrid_residual(shape):
