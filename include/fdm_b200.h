@@ -81,7 +81,9 @@ typedef struct fdm_config {
   int threads_per_block;         /* fused kernel CTA size, 0 = choose */
   int nodes_per_thread;          /* fused kernel nodes per thread, 0 = choose */
   int check_nan;                 /* 1: fdm_advance fails with FDM_ERR_NAN if Vm is not finite */
-  int profile;                   /* 1: time the main kernel launches with CUDA events */
+  int profile;                   /* 1: time the main kernel launches with CUDA events: the fused kernel's, or the split
+                                    method's reaction launches, for which few fibers in FP64 then take a launch per half
+                                    step and solve instead of whole windows in one (the same values, a longer advance) */
   int device;                    /* CUDA device ordinal the solver lives on */
   int use_graph;                 /* 1: the split path replays each window's launch sequence as a CUDA graph */
   int only_compute_if_stimulated; /* "onlyComputeIfHasBeenStimulated" (compute.tpp:201-205): a node's Heun

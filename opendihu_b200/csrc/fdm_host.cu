@@ -747,8 +747,8 @@ static int choose_cluster(fdm_solver* s, int regular_bins, int* csize_out)
       continue;
     }
     // prefer: all CTAs resident at once with an SM each, fewer nodes per thread, then more CTAs.  (16 fibers of 1481
-    // nodes: clusters of 8, of which 15 fit, 5.71 us per step in FP32 and 18.1 in FP64; clusters of 6 with 256
-    // threads, of which 22 fit, 4.87 and 9.60.  24 fibers: those 9.28 and 18.7, 3 CTAs of 256 x 2 5.12 and 16.8.)
+    // nodes: clusters of 8, of which 15 fit, 5.67 us per step in FP32 and 21.8 in FP64; clusters of 6 with 256
+    // threads, of which 22 fit, 4.87 and 11.2.  24 fibers: those 9.30 and 22.0, 3 CTAs of 256 x 2 5.25 and 22.2.)
     const int64_t ctas = (int64_t)s->n_fibers * cs;
     const bool resident = s->n_fibers <= clusters_with_own_sms((int)cs);
     const int64_t key = (resident ? 0 : (int64_t)1 << 40) + ((int64_t)sh[i].nodes_per_thread << 20) - ctas;
@@ -2316,8 +2316,8 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
   }
   // Launches of the window: the first half step, the diffusion solve, then per following split step one launch of the
   // second half step and the next one's first (nothing lies between them: one launch and one pass over the states
-  // instead of two), the diffusion solve; the second half step of the last one.  (16 x 1481 fibers FP64, 400 steps:
-  // 8.26 -> 7.47 ms; 1024 uneven fibers, 50 steps: 19.3 -> 18.8.)
+  // instead of two), the diffusion solve; the second half step of the last one.  (A launch per half step took 11 % longer
+  // for 16 x 1481 fibers in FP64, 3 % for 1024 uneven ones.)
   auto launches = [&](auto&& reaction, auto&& diffusion) -> cudaError_t {
     cudaError_t e = cudaSuccess;
     for (int j = 0; j <= n_steps && e == cudaSuccess; j++) {
@@ -3537,7 +3537,8 @@ extern "C" int fdm_adjoint_backward(fdm_solver* s, const double* trace_grad, dou
     aa.n_trace = A.n_sensors;
     aa.use_tape = s->adjoint_tape;
     // Launches: the last second half step; then per split step the diffusion solve and one launch of its first half step
-    // and the second one of the step before (nothing lies between them): 2 x 26 -> 40 us per split step for 94,784 nodes.
+    // and the second one of the step before (nothing lies between them; a launch each took 1.3 times as long for 94,784
+    // nodes).
     aa.half_stride = (int64_t)hstride;
     for (int jj = len - 1; jj >= 0; jj--) {
       const size_t j = b + jj;

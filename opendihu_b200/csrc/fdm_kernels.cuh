@@ -1393,8 +1393,9 @@ __global__ void __launch_bounds__(T) adjoint_diffusion_block_kernel(
 // memory with one cluster barrier per Strang step, and within the CTA a warp needs the total of the warp before it
 // only.  Otherwise (large steps on fine meshes) the halos stay out of the scans, and the CTAs' scan totals
 // go through two more cluster barriers.  Every CTA of a cluster takes every barrier: no CTA returns early.
-// Bound by the latency of one node's Heun chain and of the exchange.  16 fibers of 1481 nodes, FP32, 8 CTAs of 192
-// nodes each: 6.93 us per Strang step with three cluster barriers and complete scans, 5.32 us so.
+// Bound by the latency of one node's Heun chain and of the exchange.  16 fibers of 1481 nodes, FP32, clusters of 8 CTAs of
+// 192 nodes: 6.93 us per Strang step with three cluster barriers and complete scans, 5.32 us so (now on clusters of 6, an
+// SM for every CTA: 4.87).
 constexpr double CHAIN_NEGLIGIBLE = 0x1p-70;   // times |Vm| <= 1e3 mV: below 1e-18 mV
 
 template<class Model, class RR, class Math, int T, int M, bool GATE, bool CLUSTER>

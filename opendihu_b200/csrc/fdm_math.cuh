@@ -168,7 +168,8 @@ __device__ __forceinline__ void fdm_rcp_batch(R d0, R d1, R d2, R& r0, R& r1, R&
 // FP64 exponential and division of the FP64 right-hand sides (rates_f64 and the fast adjoint forms).  A right-hand side
 // strings a few of them together, and one thread's chain of them is what bounds small problems: CUDA's exp takes 150
 // cycles here, its division 120, and their branches for special arguments keep the compiler from interleaving independent
-// ones.  These have no branches, only selects.
+// ones.  These have no branches, only selects: with CUDA's exp for its three single exponentials a Hodgkin-Huxley
+// right-hand side takes 304 ns instead of 189 with one warp per SM, 440 instead of 358 with 8, 1171 instead of 1131 with 24.
 // --------------------------------------------------------------------------------------------
 // The argument c x of an exponential with a constant c, reduced without being formed: c x = k ln 2 + c R with R = x - k
 // (ln 2/c), so that its rounding error is that of c R (at most 0.35), not that of c x.  hi: ln 2/c rounded to 42 bits (k hi
