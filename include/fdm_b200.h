@@ -347,6 +347,10 @@ int fdm_emg_map_values(fdm_emg *m, const double *fiber_values);
 int fdm_emg_set_vm(fdm_emg *m, const double *vm);
 int fdm_emg_solve(fdm_emg *m, double rtol, double atol, int max_iterations, int initial_guess_nonzero,
                   int *iterations, double *residual);
+/* 1: the solves run beside other work on the device (another stream's fibers): no launch that needs every SM at once.  A
+ * Jacobi solve of a small mesh is one cooperative launch otherwise, which waits until the other work leaves the SMs.  Default 0;
+ * the two forms round differently. */
+int fdm_emg_set_concurrent(fdm_emg *m, int concurrent);
 /* preconditioner of the bidomain solve ("preconditionerType"): Jacobi, or (default) a geometric multigrid
  * V-cycle (structured coarsening by 2, Galerkin coarse operators, two damped-Jacobi sweeps before and after);
  * levels: the number of grid levels (1 for Jacobi; the hierarchy is built once the operators exist) */

@@ -36,7 +36,7 @@ EXPORTED = [
     "fdm_resident_clusters",
     "fdm_get_compute_state_information", "fdm_advance_async", "fdm_wait", "fdm_wait_for", "fdm_repeated_call_plan",
     "fdm_advance_pieces", "fdm_set_stimulation_log", "fdm_get_stimulation_log",
-    "fdm_model_equilibrium", "fdm_emg_set_preconditioner", "fdm_emg_create", "fdm_emg_destroy", "fdm_emg_last_error",
+    "fdm_model_equilibrium", "fdm_emg_set_concurrent", "fdm_emg_set_preconditioner", "fdm_emg_create", "fdm_emg_destroy", "fdm_emg_last_error",
     "fdm_emg_potential_flow", "fdm_emg_set_direction", "fdm_emg_set_conductivity", "fdm_emg_set_fiber_mapping",
     "fdm_emg_map_fibers", "fdm_emg_map_values", "fdm_emg_set_vm", "fdm_emg_solve", "fdm_emg_get",
     "fdm_emg_get_stencil", "fdm_emg_timing", "fdm_debug_fail_allocation", "fdm_set_activation_recording",
@@ -149,6 +149,7 @@ def lib() -> C.CDLL:
         "fdm_emg_get": (C.c_int, [P, C.c_int, d]),
         "fdm_emg_get_stencil": (C.c_int, [P, C.c_int, d]),
         "fdm_emg_timing": (C.c_int, [P, d, i32, d]),
+        "fdm_emg_set_concurrent": (C.c_int, [P, C.c_int]),
         "fdm_emg_set_preconditioner": (C.c_int, [P, C.c_int, i32]),
         "fdm_diffusion_solve": (C.c_int, [C.c_int, C.c_int64, P, P, P, C.c_double, C.c_int, P, P]),
         "fdm_diffusion_solve_noalloc": (C.c_int, [C.c_int, C.c_int64, P, P, P, C.c_double, C.c_int, P, P]),

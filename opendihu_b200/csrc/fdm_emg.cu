@@ -1294,6 +1294,7 @@ struct fdm_emg {
   Buf<unsigned char> mask;
   Buf<unsigned> counter;                       // last-block counter of the grid reductions
   Buf<unsigned long long> cgp_slots;           // cg_persistent_kernel: slots of the grid-wide sums, result
+  bool concurrent = false;                     // solves run beside other work on the device
   int cgp_ctas = -1;                           // its CTAs that can be resident together (-1: not asked yet)
   cudaGraphExec_t graphs[1] = {nullptr};       // CG chunk of the bidomain solve
   int precond = FDM_EMG_PRECOND_MULTIGRID;     // of the bidomain solve
@@ -1563,7 +1564,9 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
   if (const int rc = choose_tiles(m, g, use_mg ? ST_MIN_NODES : ST_MIN_NODES_JACOBI, &tiles))
     return rc;
   // small meshes, Jacobi: all iterations in one cooperative launch, as long as a CTA per CGP_T nodes is resident
-  // (113,664 nodes on 148 SMs); beyond that a launch per pass
+  // (113,664 nodes on 148 SMs); beyond that a launch per pass.  Beside other work (concurrent) a launch per pass too: the
+  // cooperative launch waits for all SMs, so nothing overlaps (169 fibers of 1481 nodes and 25 x 25 x 149 mesh nodes: 19.8 ms
+  // per coupling step of 1 ms against 18.0; alone the solve takes 3.1 to 4.7 ms against 5.6)
   if (!use_mg && m->cgp_ctas < 0) {
     int coop = 0, sms = 0, per_sm = 0;
     EMG_CUDA(m, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device));
@@ -1573,7 +1576,7 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
     m->cgp_ctas = coop ? std::min(sms * per_sm, CGP_T / 2) : 0;
   }
   const int64_t ctas = (N + CGP_T - 1) / CGP_T;
-  if (!use_mg && ctas <= m->cgp_ctas && rn > target) {
+  if (!use_mg && !m->concurrent && ctas <= m->cgp_ctas && rn > target) {
     const size_t n_slots = 3 * CGP_SLOT * (size_t)ctas;
     EMG_CUDA(m, m->cgp_slots.alloc(n_slots + 1));
     EMG_CUDA(m, cudaMemsetAsync(m->cgp_slots.p, 0xff, sizeof(unsigned long long) * n_slots, s));
@@ -2094,6 +2097,14 @@ extern "C" int fdm_emg_solve(fdm_emg* m, double rtol, double atol, int max_itera
     *iterations = its;
   if (residual)
     *residual = res;
+  return FDM_OK;
+}
+
+extern "C" int fdm_emg_set_concurrent(fdm_emg* m, int concurrent)
+{
+  if (!m)
+    return FDM_ERR_ARG;
+  m->concurrent = concurrent != 0;
   return FDM_OK;
 }
 

@@ -241,6 +241,11 @@ class StaticBidomainSolver:
                    int(self.initial_guess_nonzero), C.byref(its), C.byref(res))
         return its.value
 
+    def set_concurrent(self, concurrent: bool):
+        """Whether the solves run beside other work on the device (fdm_emg_set_concurrent)."""
+        self.initialize()
+        self._call(N.lib().fdm_emg_set_concurrent, int(bool(concurrent)))
+
     def run(self):
         self.initialize()
         self.advanceTimeSpan()
@@ -453,6 +458,8 @@ class Coupling:
         if self.overlap and self._pool is None:
             from concurrent.futures import ThreadPoolExecutor
             self._pool = ThreadPoolExecutor(max_workers=1, thread_name_prefix="bidomain")
+        # (without overlap too: the solves take the same launches, so the results are the same)
+        self.term2.set_concurrent(True)
         try:
             for k in range(n):
                 self.term1.setTimeSpan(t, t + dt)
@@ -470,8 +477,12 @@ class Coupling:
                         self.callback(k, t + dt, self.term2)
                 t = self.start_time + (k + 1) / n * span
         finally:
-            if pending is not None:
-                finish(pending)
+            try:
+                if pending is not None:
+                    finish(pending)
+            finally:
+                if self.term2.initialized:
+                    self.term2.set_concurrent(False)
 
     def run(self):
         self.initialize()

@@ -39,8 +39,12 @@ def _solver(shape, preconditioner, rtol):
 # beyond it are around 113,664 nodes on 148 SMs; the march along z from 1,200,000 nodes
 @pytest.mark.parametrize("shape", [(2, 2, 2), (13, 59, 2), (8, 8, 12), (769, 2, 2), (16, 16, 3), (37, 61, 50),
                                    (37, 64, 48), (37, 64, 49), (110, 101, 109)])
-def test_jacobi_residual(shape):
+@pytest.mark.parametrize("concurrent", [False, True])
+def test_jacobi_residual(shape, concurrent):
+    if concurrent and np.prod(shape) > 113664:
+        pytest.skip("takes a launch per pass either way")
     with _solver(shape, "jacobi", 1e-10) as s:
+        s.set_concurrent(concurrent)     # beside other work: a launch per pass
         vm = np.random.default_rng(1).uniform(-80.0, 40.0, s.n_nodes)
         s.set_vm(vm)
         s.advanceTimeSpan()
