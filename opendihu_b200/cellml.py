@@ -1170,8 +1170,6 @@ class _Fast64Emitter(_Emitter):
             if af is not None and not af[0] and 1e-30 < abs(af[1]) < 1e30 and abs(_int_exponent(e[2][1])) <= 8:
                 c = Fraction(af[1]) ** _int_exponent(e[2][1])
                 return (1 / c if inverse else c), [], []
-        if inverse and e[0] == "call" and e[1] == "exp":
-            return Fraction(1), [("call", "exp", [("neg", e[2][0])])], []   # 1/exp(u) = exp(-u)
         if e[0] in ("neg", "pos"):
             c, n, d = self.factors(e[1], inverse)
             return (-c if e[0] == "neg" else c), n, d

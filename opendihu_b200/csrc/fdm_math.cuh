@@ -324,8 +324,8 @@ __device__ __forceinline__ double fdm_div64(double a, double b)
 __device__ __forceinline__ bool fdm_is_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
 // a/b as IEEE arithmetic has it for every a and b.  A divisor that is subnormal or at least 2^1021 is scaled together with
 // the dividend; the hardware's approximation of 1/b is infinite for b = 0 and 0 for infinite b and stays as it is then; what
-// the correction turns into NaN (such b, infinite a, a quotient that overflows) is a (1/b) itself.  Shorten's 26 of them
-// (36 x 1481 nodes, 4 steps): 5.74 ms, with CUDA's division 6.55, with fdm_div64, were it right for them, 5.4.
+// the correction turns into NaN (such b, infinite a, a quotient that overflows) is a (1/b) itself.  Shorten (36 x 1481
+// nodes, 4 steps) with 26 of them took 5.76 ms, with CUDA's division in their place 6.55.
 __device__ __forceinline__ double fdm_div64_any(double a, double b)
 {
   const int exponent = __double2hiint(b) & 0x7ff00000;

@@ -14,11 +14,11 @@ from opendihu_b200 import cellml as CM
 pytestmark = pytest.mark.gpu
 
 
-def _library(path, model, params_const=()):
+def _library(path, model, params_const=(), params_alg=()):
     """tests/cpp/math_functions.cu compiled with the model's right-hand side"""
     (path / "test_model.cuh").write_text(
-        CM.emit_cuda_model(model, (), params_const)
-        + f"\n#define TEST_MODEL fdm_model_{CM._ident(model)}_{CM.variant_tag((), params_const)}\n"
+        CM.emit_cuda_model(model, params_alg, params_const)
+        + f"\n#define TEST_MODEL fdm_model_{CM._ident(model)}_{CM.variant_tag(params_alg, params_const)}\n"
         + f"#define TEST_SCALE {CM._exp_scale_text(Fraction(-1, 10))}\n"
         + f"#define TEST_OFFSET {CM._exp_offset_text(Fraction(-3, 2))}\n")
     lib = str(path / "math_functions.so")
@@ -194,3 +194,15 @@ def test_rates_at_removable_singularities(hodgkin_huxley, singularity):
         u = np.abs(V + centre) / 10
         cancelled = 0.7 * (1 + 1 / u) * alpha * (1 - y) if k == 3 else 0
         assert np.all(error < 2.0 ** -53 * (18 * (alpha * (1 - y) + beta * y) + cancelled))
+
+
+# random states around the initial ones, against the equations in C; the tolerances are those of the plain form's test
+@pytest.mark.parametrize("model,approximate", [(H.HH, False), (H.HH, True), (H.SHORTEN, False), (H.SHORTEN, True)])
+def test_rates_match_equations(model, approximate, tmp_path):
+    import test_gpu_cellml_rhs as R
+    from opendihu_b200.solver import VARIANT_PARAMETERS
+    params_alg, params_const = VARIANT_PARAMETERS[model]
+    lib = _library(tmp_path, CM.builtin_model(model), params_const, params_alg)
+    states, params, ns, _ = R._inputs(model, 500, 4)
+    want, _ = R._oracle(model, states, params, 0.0, approximate)
+    np.testing.assert_allclose(_rates(lib, approximate, states, params), want, rtol=1e-11, atol=1e-12 * np.abs(want).max())
