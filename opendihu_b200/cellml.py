@@ -1010,8 +1010,8 @@ class _Fast64Emitter(_Emitter):
         for found in slopes.values():
             # the base: an exponential that 1 is subtracted from, if there is one (it is the most exact member)
             base, b0, _ = max(found.values(), key=lambda m: m[2])
-            # (exp(u + b) - 1 of another member is off by some 2^-53: too much where u + b = c (x + d) with a small c d comes
-            # closer to 0 than that)
+            # (exp(u + b) - 1 of another member is off by some 2^-53: too much where u + b = c (x + d) with a small c d
+            # comes closer to 0 than that)
             near = {r: b - b0 for r, (u, b, minus_one) in found.items()
                     if u is base or abs(b - b0) <= 2 and not (minus_one and abs(b) < 4)}
             if len(near) > 1:

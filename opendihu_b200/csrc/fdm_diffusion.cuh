@@ -335,10 +335,10 @@ __global__ void __launch_bounds__(DIFFUSION_T) diffusion_reg_kernel(const int64_
 // take about half of a step that has some hundred nodes per SM.  Here the states stay in registers for the window; the
 // CTAs send their Vm to the cluster's first one, which solves the fiber's diffusion as diffusion_reg_kernel does, with
 // the factors in registers, and the others fetch theirs back: two cluster barriers per step.  Same functions and
-// partition as the kernels it stands in for, and the same values, bit for bit, whichever form the number of fibers leads to.
-// Bound by the FP64 work of the Heun substeps at 8 warps per SM, 2.0 us of the 2.7 + 2.0 n0 us per step at n0 substeps a
-// half step.  Per step of 5 substeps a half step, with launches and so: 16 fibers of 1481 nodes (clusters of 6) 15.1 and
-// 12.6 us; one of 101 nodes 9.4 and 6.8; 74 of 500 14.1 and 10.6.
+// partition as the kernels it stands in for, and the same values, bit for bit, whichever form the number of fibers
+// leads to. Bound by the FP64 work of the Heun substeps at 8 warps per SM, 2.0 us of the 2.7 + 2.0 n0 us per step at n0
+// substeps a half step.  Per step of 5 substeps a half step, with launches and so: 16 fibers of 1481 nodes (clusters of
+// 6) 15.1 and 12.6 us; one of 101 nodes 9.4 and 6.8; 74 of 500 14.1 and 10.6.
 constexpr int WINDOW_T = DIFFUSION_T;
 
 template<class Model, class Math, int M>

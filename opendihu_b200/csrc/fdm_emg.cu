@@ -1404,11 +1404,12 @@ std::vector<int> coarse_indices(int n)
   return F;
 }
 
-// The tiles of a grid's stencil passes; grids of fewer than min_nodes, which have too few planes and columns for the chip,
-// take the node-per-thread passes.  Per iteration, marching against a thread per node: multigrid, whose V-cycle has five
-// such passes, 60 x 60 x 150 nodes 287 us / 290, 70 x 70 x 120 302 / 320, 60 x 60 x 170 309 / 308, 90 x 80 x 90 326 / 341;
-// Jacobi, with one pass, either way by shape up to a million nodes (80 x 80 x 100 52.2 / 50.6, 60 x 60 x 200 56.5 / 55.1,
-// 95^3 60.2 / 62.9, 100^3 74.1 / 72.6), then marching: 110 x 100 x 110 86.3 / 89.3, 80 x 80 x 220 94.8 / 100.0.
+// The tiles of a grid's stencil passes; grids of fewer than min_nodes, which have too few planes and columns for the
+// chip, take the node-per-thread passes.  Per iteration, marching against a thread per node: multigrid, whose V-cycle
+// has five such passes, 60 x 60 x 150 nodes 287 us / 290, 70 x 70 x 120 302 / 320, 60 x 60 x 170 309 / 308, 90 x 80 x
+// 90 326 / 341; Jacobi, with one pass, either way by shape up to a million nodes (80 x 80 x 100 52.2 / 50.6, 60 x 60 x
+// 200 56.5 / 55.1, 95^3 60.2 / 62.9, 100^3 74.1 / 72.6), then marching: 110 x 100 x 110 86.3 / 89.3, 80 x 80 x 220 94.8
+// / 100.0.
 int choose_tiles(fdm_emg* m, const Grid& g, int64_t min_nodes, StencilTiles* tiles)
 {
   *tiles = StencilTiles{};
@@ -1564,9 +1565,9 @@ int cg_solve(fdm_emg* m, const double* U, const unsigned char* mask, bool nullsp
   if (const int rc = choose_tiles(m, g, use_mg ? ST_MIN_NODES : ST_MIN_NODES_JACOBI, &tiles))
     return rc;
   // small meshes, Jacobi: all iterations in one cooperative launch, as long as a CTA per CGP_T nodes is resident
-  // (113,664 nodes on 148 SMs); beyond that a launch per pass.  Beside other work (concurrent) a launch per pass too: the
-  // cooperative launch waits for all SMs, so nothing overlaps (169 fibers of 1481 nodes and 25 x 25 x 149 mesh nodes: 19.8 ms
-  // per coupling step of 1 ms against 18.0; alone the solve takes 3.1 to 4.7 ms against 5.6)
+  // (113,664 nodes on 148 SMs); beyond that a launch per pass.  Beside other work (concurrent) a launch per pass too:
+  // the cooperative launch waits for all SMs, so nothing overlaps (169 fibers of 1481 nodes and 25 x 25 x 149 mesh
+  // nodes: 19.8 ms per coupling step of 1 ms against 18.0; alone the solve takes 3.1 to 4.7 ms against 5.6)
   if (!use_mg && m->cgp_ctas < 0) {
     int coop = 0, sms = 0, per_sm = 0;
     EMG_CUDA(m, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device));

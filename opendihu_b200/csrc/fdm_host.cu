@@ -2316,8 +2316,8 @@ static int run_window(fdm_solver* s, const SplitStep* host_steps, int n_steps, d
   }
   // Launches of the window: the first half step, the diffusion solve, then per following split step one launch of the
   // second half step and the next one's first (nothing lies between them: one launch and one pass over the states
-  // instead of two), the diffusion solve; the second half step of the last one.  (A launch per half step took 11 % longer
-  // for 16 x 1481 fibers in FP64, 3 % for 1024 uneven ones.)
+  // instead of two), the diffusion solve; the second half step of the last one.  (A launch per half step took 11 %
+  // longer for 16 x 1481 fibers in FP64, 3 % for 1024 uneven ones.)
   auto launches = [&](auto&& reaction, auto&& diffusion) -> cudaError_t {
     cudaError_t e = cudaSuccess;
     for (int j = 0; j <= n_steps && e == cudaSuccess; j++) {
@@ -3336,8 +3336,8 @@ extern "C" int fdm_adjoint_forward(fdm_solver* s, double t_start, double t_end, 
   }
   s->ev_used = 0;
   FDM_CUDA(cudaEventRecord(s->adv_start, s->stream));
-  // the replay in fdm_adjoint_backward issues the reaction and the solves launch by launch; the forward does so too, so that
-  // the replay reproduces it bit for bit
+  // the replay in fdm_adjoint_backward issues the reaction and the solves launch by launch; the forward does so too, so
+  // that the replay reproduces it bit for bit
   s->adj_forward = true;
   for (int c = 0; c < A.n_seg && !rc; c++) {
     rc = copy_state(s, A.ck_vm.p + (size_t)c * N, A.ck_states.p + (size_t)c * N * (NS - 1), A.ck_last.p + (size_t)c * nf,

@@ -292,11 +292,11 @@ __device__ __forceinline__ void accumulate(RR& s, RR& l, RR inc)
   }
 }
 
-// right-hand side: FP32 with the exact exponential takes the model's shared-exponential form (fewest SFU operations), with
-// the approximate one, which is not multiplicative, the plain form; FP64 the form without divisions by constants.
+// right-hand side: FP32 with the exact exponential takes the model's shared-exponential form (fewest SFU operations),
+// with the approximate one, which is not multiplicative, the plain form; FP64 the form without divisions by constants.
 // FP64 is bound by its pipe: one Hodgkin-Huxley right-hand side as the model writes it takes 6 exponentials and 10
-// divisions (7 of them by constants, which the compiler keeps as divisions), here the
-// work of 4 (three come from one reduction) and 3.
+// divisions (7 of them by constants, which the compiler keeps as divisions), here the work of 4 (three come from one
+// reduction) and 3.
 template<class Model, class RR, class Math>
 __device__ __forceinline__ void model_rates(const RR t, const RR* y, const RR* P, RR* r, RR* alg)
 {
@@ -621,13 +621,13 @@ struct ReactionArgs {
 };
 
 // CTAs of 128 threads per SM that the registers are held to.  A model of many states spills either way in FP64 (Shorten:
-// 110 registers for its states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 4 steps of
-// 53,316 nodes with their transfers 5.73 ms against 5.88 (four CTAs: 6.22).  In FP32 its 255 registers hold everything
-// (168: 481 -> 1173 us).
-// Hodgkin-Huxley in FP64 is bound by the FP64 pipe; four CTAs let the compiler interleave its exponentials: two half steps
-// of 5 substeps of 1,566,720 nodes 304 us against 318 with six and 319 with five (three: 310), of 94,784 nodes 30.3 against
-// 32.5.  So a thread per node is the fastest form for few nodes too: with a warp for each of a node's four states, 32 nodes
-// per CTA, a step took 11.0 us against 9.5 (101 nodes), 13.4 against 11.6 (6000) and 19.2 against 15.5 (23,696).
+// 110 registers for its states alone), and three CTAs of 168 registers hide more of its latency than two of 255: 4
+// steps of 53,316 nodes with their transfers 5.73 ms against 5.88 (four CTAs: 6.22).  In FP32 its 255 registers hold
+// everything (168: 481 -> 1173 us). Hodgkin-Huxley in FP64 is bound by the FP64 pipe; four CTAs let the compiler
+// interleave its exponentials: two half steps of 5 substeps of 1,566,720 nodes 304 us against 318 with six and 319 with
+// five (three: 310), of 94,784 nodes 30.3 against 32.5.  So a thread per node is the fastest form for few nodes too:
+// with a warp for each of a node's four states, 32 nodes per CTA, a step took 11.0 us against 9.5 (101 nodes), 13.4
+// against 11.6 (6000) and 19.2 against 15.5 (23,696).
 template<class Model, class RR>
 constexpr int reaction_min_ctas()
 {
@@ -1393,9 +1393,9 @@ __global__ void __launch_bounds__(T) adjoint_diffusion_block_kernel(
 // memory with one cluster barrier per Strang step, and within the CTA a warp needs the total of the warp before it
 // only.  Otherwise (large steps on fine meshes) the halos stay out of the scans, and the CTAs' scan totals
 // go through two more cluster barriers.  Every CTA of a cluster takes every barrier: no CTA returns early.
-// Bound by the latency of one node's Heun chain and of the exchange.  16 fibers of 1481 nodes, FP32, clusters of 8 CTAs of
-// 192 nodes: 6.93 us per Strang step with three cluster barriers and complete scans, 5.32 us so (now on clusters of 6, an
-// SM for every CTA: 4.87).
+// Bound by the latency of one node's Heun chain and of the exchange.  16 fibers of 1481 nodes, FP32, clusters of 8 CTAs
+// of 192 nodes: 6.93 us per Strang step with three cluster barriers and complete scans, 5.32 us so (now on clusters of
+// 6, an SM for every CTA: 4.87).
 constexpr double CHAIN_NEGLIGIBLE = 0x1p-70;   // times |Vm| <= 1e3 mV: below 1e-18 mV
 
 template<class Model, class RR, class Math, int T, int M, bool GATE, bool CLUSTER>

@@ -183,8 +183,8 @@ cudaError_t launch_pairs_to_states(const float* hi, const float* lo, double* x, 
   return cudaGetLastError();
 }
 
-// from this many fibers on a warp per fiber can fill the GPU (four warps on each of 148 SMs): launch_diffusion takes it for
-// short fibers and for fibers too long for registers, launch_adjoint_diffusion for all
+// from this many fibers on a warp per fiber can fill the GPU (four warps on each of 148 SMs): launch_diffusion takes it
+// for short fibers and for fibers too long for registers, launch_adjoint_diffusion for all
 constexpr int DIFFUSION_BLOCK_MAX_FIBERS = 4 * 148;
 
 template<int M>
@@ -263,7 +263,8 @@ int clusters_with_own_sms(int csize)
 // The few fibers a window kernel is for: a CTA for at most WINDOW_T nodes and an SM for every CTA; the most CTAs per
 // fiber (at most 8, down to 128 nodes each) with which that holds.  Where CTAs share an SM, the launches cost less than that:
 // per step of 5 substeps a half step 16 fibers of 1481 nodes take 12.6 us with clusters of 6, 24.3 with clusters of 8
-// (one more than fit) and 15.1 with a launch per half step and solve; 24 fibers 24.4 with clusters of 6 (22 fit) and 15.6.
+// (one more than fit) and 15.1 with a launch per half step and solve; 24 fibers 24.4 with clusters of 6 (22 fit) and
+// 15.6.
 int window_cluster_size(int model, int n_fibers, int64_t max_fiber_len)
 {
   const int least = (int)std::min<int64_t>((max_fiber_len + WINDOW_T - 1) / WINDOW_T, FDM_MAX_CLUSTER + 1);

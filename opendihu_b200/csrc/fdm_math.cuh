@@ -177,9 +177,9 @@ __device__ __forceinline__ void fdm_rcp_batch(R d0, R d1, R d2, R& r0, R& r1, R&
 struct fdm_exp_scale {
   double c, c_lo, l2e, hi, lo;
 };
-// exp(c x) = 2^k exp(r), |r| <= ln 2 / 2, with ln 2/c in two parts (Cody and Waite), k from the rounding of the sum with
-// 1.5 2^52; exp(r) = 1 + r + r^2 Q(r) with the degree-9 interpolation of Q at the Chebyshev nodes (relative error 3.4e-17),
-// evaluated by Estrin's scheme.
+// exp(c x) = 2^k exp(r), |r| <= ln 2 / 2, with ln 2/c in two parts (Cody and Waite), k from the rounding of the sum
+// with 1.5 2^52; exp(r) = 1 + r + r^2 Q(r) with the degree-9 interpolation of Q at the Chebyshev nodes (relative error
+// 3.4e-17), evaluated by Estrin's scheme.
 struct fdm_exp_reduced {
   double t, r;   // k as a double, r
   int k;
@@ -202,8 +202,8 @@ struct fdm_exp_reduced {
     return fma(r2, q, small);
   }
 };
-// The ends of the range: 0 below -708 (the result would be subnormal), infinite (SAT: 2^1020, for divisors) from where the
-// result would be within 3e-6 of the largest number; NaN for NaN.
+// The ends of the range: 0 below -708 (the result would be subnormal), infinite (SAT: 2^1020, for divisors) from where
+// the result would be within 3e-6 of the largest number; NaN for NaN.
 constexpr double FDM_EXP_MAX = 709.78271, FDM_EXP_MIN = -708.0;
 template<bool SAT>
 __device__ __forceinline__ double fdm_exp_ends(double e, bool over, bool under)
@@ -215,8 +215,8 @@ __device__ __forceinline__ double fdm_exp_times_2k(double e, int k)
 {
   return __hiloint2double(__double2hiint(e) + (k << 20), __double2loint(e));
 }
-// exp(x): 1 + r is rounded once and what that loses is added to the small terms.  At most 0.87 ulp and 0.253 on average of 4
-// million arguments (CUDA's exp: 0.88 and 0.258).
+// exp(x): 1 + r is rounded once and what that loses is added to the small terms.  At most 0.87 ulp and 0.253 on average
+// of 4 million arguments (CUDA's exp: 0.88 and 0.258).
 template<bool SAT = false>
 __device__ __forceinline__ double fdm_exp64(double x)
 {
@@ -240,8 +240,8 @@ __device__ __forceinline__ double fdm_exp64(double x, const fdm_exp_scale& f)
   return fdm_exp_ends<SAT>(fdm_exp_times_2k(e, z.k), f.c > 0.0 ? x > top : x < top, f.c > 0.0 ? x < bottom : x > bottom);
 }
 // exp(c x) - 1 without the cancellation: 2^k (exp(r) - 1) + (2^k - 1), halved on the way so that k = 1024 has a 2^k.
-// exp minus 1 loses 1/|exp(x) - 1| of exp's accuracy: 1.0 ulp on average for |x| <= 5 and 135 at 1e-2, this 0.27 and 0.25
-// (at most 2).
+// exp minus 1 loses 1/|exp(x) - 1| of exp's accuracy: 1.0 ulp on average for |x| <= 5 and 135 at 1e-2, this 0.27 and
+// 0.25 (at most 2).
 template<bool SAT = false>
 __device__ __forceinline__ double fdm_expm1_64(double x, const fdm_exp_scale& f)
 {
@@ -259,10 +259,11 @@ __device__ __forceinline__ double fdm_expm1_64(double x)
 {
   return fdm_expm1_64<SAT>(x, fdm_exp_scale{1.0, 0.0, 0x1.71547652b82fep+0, 0x1.62e42fefa3800p-1, 0x1.ef35793c76730p-45});
 }
-// exp(c x + b) and exp(c x + b) - 1 for several small b (|b| <= 2) from one reduction: exp(c x) = 2^k (s + p) with s = 1 + c R
-// rounded and p the rest, whose error is some 2^-56 of the sum, times e^b in two parts.  For divisors: the argument is held in
-// [-700, 700].  With exp(c x + b) - 1 near 0 the error is 0.3 of the 2^-53 that an exponential rounded first leaves there,
-// as long as x is exact (a sum V + d near -V is).  5 to 6 FP64 instructions each instead of about 20.
+// exp(c x + b) and exp(c x + b) - 1 for several small b (|b| <= 2) from one reduction: exp(c x) = 2^k (s + p) with s =
+// 1 + c R rounded and p the rest, whose error is some 2^-56 of the sum, times e^b in two parts.  For divisors: the
+// argument is held in [-700, 700].  With exp(c x + b) - 1 near 0 the error is 0.3 of the 2^-53 that an exponential
+// rounded first leaves there, as long as x is exact (a sum V + d near -V is).  5 to 6 FP64 instructions each instead of
+// about 20.
 struct fdm_exp_offset {
   double e, e_lo;   // e^b and what it leaves of e^b
 };
@@ -300,9 +301,9 @@ struct fdm_exp_group {
     return fma(p, o.e, fma(s, o.e_lo, fma(s, o.e, -h)));
   }
 };
-// 1/d by one Halley step (cubic) from the hardware's approximation: 0.507 ulp; a/b with one residual correction of a (1/b),
-// correctly rounded in 4 million quotients.  For b normal and finite (beyond 2^1022 in magnitude the quotient is 0), a and
-// the quotient finite; b = 0, subnormal or infinite, and a quotient that overflows, give NaN.
+// 1/d by one Halley step (cubic) from the hardware's approximation: 0.507 ulp; a/b with one residual correction of a
+// (1/b), correctly rounded in 4 million quotients.  For b normal and finite (beyond 2^1022 in magnitude the quotient is
+// 0), a and the quotient finite; b = 0, subnormal or infinite, and a quotient that overflows, give NaN.
 __device__ __forceinline__ double fdm_rcp_approx(double d)
 {
   double y;
@@ -322,10 +323,10 @@ __device__ __forceinline__ double fdm_div64(double a, double b)
   return fma(fma(-b, q, a), y, q);
 }
 __device__ __forceinline__ bool fdm_is_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
-// a/b as IEEE arithmetic has it for every a and b.  A divisor that is subnormal or at least 2^1021 is scaled together with
-// the dividend; the hardware's approximation of 1/b is infinite for b = 0 and 0 for infinite b and stays as it is then; what
-// the correction turns into NaN (such b, infinite a, a quotient that overflows) is a (1/b) itself.  Shorten (36 x 1481
-// nodes, 4 steps) with 26 of them took 5.76 ms, with CUDA's division in their place 6.55.
+// a/b as IEEE arithmetic has it for every a and b.  A divisor that is subnormal or at least 2^1021 is scaled together
+// with the dividend; the hardware's approximation of 1/b is infinite for b = 0 and 0 for infinite b and stays as it is
+// then; what the correction turns into NaN (such b, infinite a, a quotient that overflows) is a (1/b) itself.  Shorten
+// (36 x 1481 nodes, 4 steps) with 26 of them took 5.76 ms, with CUDA's division in their place 6.55.
 __device__ __forceinline__ double fdm_div64_any(double a, double b)
 {
   const int exponent = __double2hiint(b) & 0x7ff00000;
@@ -339,8 +340,8 @@ __device__ __forceinline__ double fdm_div64_any(double a, double b)
   const double c = fma(fma(-b, q, a), y, q);
   return fdm_is_nan(c) ? q : c;
 }
-// 1/d for every d: where the step would give NaN or the result is not normal, the hardware's approximation, infinite for
-// d = 0 and subnormal d, 0 for infinite d and from 2^1022 on.
+// 1/d for every d: where the step would give NaN or the result is not normal, the hardware's approximation, infinite
+// for d = 0 and subnormal d, 0 for infinite d and from 2^1022 on.
 __device__ __forceinline__ double fdm_rcp64_any(double d)
 {
   const double y = fdm_rcp_approx(d);

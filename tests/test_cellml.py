@@ -178,9 +178,9 @@ def test_settings_with_mappings():
 
 
 def test_fp64_form_exponentials():
-    # Hodgkin-Huxley in FP64: the three exponentials of slope 1/10 are in divisors and come from one reduction, at offsets 0
-    # (alpha_m), -1.5 (alpha_n) and 0.5 (beta_h); exp(u) - 1 has a function of its own; the other three exponentials stand
-    # alone
+    # Hodgkin-Huxley in FP64: the three exponentials of slope 1/10 are in divisors and come from one reduction, at
+    # offsets 0 (alpha_m), -1.5 (alpha_n) and 0.5 (beta_h); exp(u) - 1 has a function of its own; the other three
+    # exponentials stand alone
     text = cellml.emit_cuda_model(cellml.builtin_model(H.HH), (), (2, 3, 4))
     f64 = text[text.index("static void rates_f64("):text.index("// FP32 form")]
     body = "\n".join(x for x in f64.split("\n") if not x.startswith("#"))
@@ -202,8 +202,8 @@ def test_exponentials_far_apart_share_nothing():
 
 
 def test_divisions_that_need_no_special_values():
-    # FDM_DIV only where the divisor is known to be finite and away from 0 and the quotient finite; FDM_DIV0 only where dividend
-    # and divisor vanish together
+    # FDM_DIV only where the divisor is known to be finite and away from 0 and the quotient finite; FDM_DIV0 only where
+    # dividend and divisor vanish together
     model = lambda *texts: [("R", k, cellml.parse_expression(t)) for k, t in enumerate(texts)]
     lean = ("1.0/(1.0+exp(STATES[0]/10.0))", "STATES[1]/(2.0+exp(STATES[0]))",
             "3.0/(0.2+5.65*pow((STATES[0]+90.0)/100.0, 2.0))", "2.0/(-1.0-exp(STATES[0]))")

@@ -114,9 +114,9 @@ def test_exponential_minus_one(hodgkin_huxley):
     np.testing.assert_array_equal(_function(hodgkin_huxley, 5, -10.0 * x), [0, np.inf, -1, np.nan, np.inf, np.inf, -1, -1])
 
 
-# The members of a group, exp(-x/10 - b): the polynomial's 3.4e-17 relative to exp(r) >= 0.7, R as c R (2e-17) and the sum's
-# and the product's last roundings are below 1.2 ulp.  Minus 1: two roundings at the result's size, at most 1 ulp, and what
-# the exponential brings in before the subtraction, 0.6 of 2^-53 of it.
+# The members of a group, exp(-x/10 - b): the polynomial's 3.4e-17 relative to exp(r) >= 0.7, R as c R (2e-17) and the
+# sum's and the product's last roundings are below 1.2 ulp.  Minus 1: two roundings at the result's size, at most 1 ulp,
+# and what the exponential brings in before the subtraction, 0.6 of 2^-53 of it.
 def test_exponential_group(hodgkin_huxley):
     rng = np.random.default_rng(4)
     x = np.concatenate([10.0 * _exp_arguments(), *(-15.0 + s * 10.0 ** rng.uniform(-12, 1, 100000) for s in (1, -1))])
@@ -170,10 +170,10 @@ def test_terms_with_vanishing_and_infinite_divisors(hill, approximate):
     np.testing.assert_allclose(_rates(hill, approximate, np.stack([v, c, d, c])), want, rtol=4e-13, atol=1e-300)
 
 
-# alpha_m = x / (exp(x) - 1) at V = -50 mV, alpha_n at -65 mV, around their removable singularities.  alpha_m is as exact
-# there as elsewhere; 20 mV away, in halves of an ulp: the argument's 2.5 times u e^u / (e^u - 1) = 2.3, the numerator's 2.5,
-# the exponential's 4, quotient, difference, product and sum 4: 17.  alpha_n's exponential is alpha_m's times e^-1.5: before
-# 1 is subtracted it is off by 0.7 of 2^-53 at most (an exponential by itself: by 1).
+# alpha_m = x / (exp(x) - 1) at V = -50 mV, alpha_n at -65 mV, around their removable singularities.  alpha_m is as
+# exact there as elsewhere; 20 mV away, in halves of an ulp: the argument's 2.5 times u e^u / (e^u - 1) = 2.3, the
+# numerator's 2.5, the exponential's 4, quotient, difference, product and sum 4: 17.  alpha_n's exponential is alpha_m's
+# times e^-1.5: before 1 is subtracted it is off by 0.7 of 2^-53 at most (an exponential by itself: by 1).
 @pytest.mark.parametrize("singularity", [-50.0, -65.0])
 def test_rates_at_removable_singularities(hodgkin_huxley, singularity):
     rng = np.random.default_rng(3)

@@ -151,8 +151,9 @@ def test_cluster_halos(dt, threads, per_thread):
 
 # whole windows in one launch (few fibers: at most 2048 nodes, clusters of 1 to 8 CTAs with an SM each): one to eight
 # CTAs, nodes per CTA from 2 to 256, fibers shorter than the cluster's first CTA, the last number of fibers that still
-# fits 8 and 1 CTAs ("8" and "1") and the first that does not, 2049 nodes (a launch per half step and solve); windows of 1,
-# 7, 20 steps.  The forms give the same values, bit for bit, so that a fiber's do not depend on how many others there are.
+# fits 8 and 1 CTAs ("8" and "1") and the first that does not, 2049 nodes (a launch per half step and solve); windows of
+# 1, 7, 20 steps.  The forms give the same values, bit for bit, so that a fiber's do not depend on how many others there
+# are.
 @pytest.mark.parametrize("lengths", [[2], [3, 2], [128], [129], [256, 257], [1481], [2048, 2, 255, 1024, 1025],
                                      ("8", 0, 1024), ("8", 1, 1024), ("8", 1, 2041), ("1", 0, 100), ("1", 1, 100), [2049, 40]])
 @pytest.mark.parametrize("approximate", [False, True])
